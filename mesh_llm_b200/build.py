@@ -21,7 +21,7 @@ MAIN_SOURCES = ("kq_rpc_main.cu",)  # executables, not part of the library
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
-    "-Xcompiler", "-fPIC,-fvisibility=hidden,-O3", "--expt-relaxed-constexpr", *(["-DKQ_GEMM_PROF"] if os.environ.get("KQ_GEMM_PROF") else []),
+    "-Xcompiler", "-fPIC,-fvisibility=hidden,-O3", "--expt-relaxed-constexpr",
     "-ccbin", "/usr/bin/g++",
 ]
 

@@ -1,0 +1,114 @@
+"""The tensor-core product with K-quant weights at the edges of its tiles, shares and rings, against the oracle's integer block
+sums and a combination in 64 bits.
+
+Per block the kernel forms da (dw si - dmin sm) with three roundings and adds it to an f32 sum of at most K / 256 terms (a tile that
+was cut adds a few more), so |error| <= (K / 256 + 8) 2^-23 sum_b da (|dw si| + |dmin sm|)."""
+import numpy as np
+import pytest
+
+from oracle import binding as orc
+
+pytestmark = pytest.mark.gpu
+
+# rows: part of a tile, several; K: one block, odd counts, Q6_K groups with an odd tail
+SHAPES = [(1, 256), (100, 512), (129, 2816), (264, 768)]
+TOKENS = [9, 16, 17, 64, 65, 128, 129, 193, 256, 257]
+
+
+def blocks_of(ty, N, K, seed):
+    rng = np.random.default_rng(seed)
+    blk = rng.integers(0, 256, size=(N * K // 256, 144 if ty == orc.TYPE_Q4_K else 210), dtype=np.uint8)
+    half = lambda lo, hi: rng.uniform(lo, hi, len(blk)).astype(np.float16)[:, None].view(np.uint8)
+    if ty == orc.TYPE_Q4_K:
+        blk[:, 0:2], blk[:, 2:4] = half(1e-4, 1e-3), half(1e-4, 1e-3)
+    else:
+        blk[:, 208:210] = half(1e-5, 1e-4)
+    return blk.reshape(N, -1)
+
+
+def exact(ty, W, x, N, K):
+    """-> y and the sum of the magnitudes of its terms, both in 64 bits"""
+    q, d, bs = orc.quantize_act(x)
+    si, sm = orc.block_sums(ty, W, q, bs, N, K)
+    b = np.ascontiguousarray(W).reshape(N, K // 256, -1)
+    f16 = lambda at: np.ascontiguousarray(b[:, :, at:at + 2]).view(np.float16)[..., 0].astype(np.float64)
+    main = si.reshape(-1, N, K // 256) * (f16(0) if ty == orc.TYPE_Q4_K else f16(208))
+    low = sm.reshape(-1, N, K // 256) * f16(2) if ty == orc.TYPE_Q4_K else np.zeros_like(main)
+    d = d.reshape(-1, 1, K // 256).astype(np.float64)
+    return ((main - low) * d).sum(-1), ((np.abs(main) + np.abs(low)) * d).sum(-1)
+
+
+def check(got, want, size, K):
+    bound = (K // 256 + 8) * 2.0 ** -23 * size + 1e-30
+    assert np.all(np.abs(got.astype(np.float64) - want) <= bound)
+
+
+@pytest.mark.parametrize("ty", [orc.TYPE_Q4_K, orc.TYPE_Q6_K], ids=["q4_k", "q6_k"])
+@pytest.mark.parametrize("N,K", SHAPES)
+def test_dense(ty, N, K):
+    import torch
+
+    from mesh_llm_b200 import capi, ops
+
+    W = blocks_of(ty, N, K, N + K)
+    dev = ops.upload_weights(ty, W, N, K)
+    for M in TOKENS:
+        x = np.random.default_rng(M).standard_normal((M, K)).astype(np.float32)
+        want, size = exact(ty, W, x, N, K)
+        got = ops.mul_mat(ty, dev, torch.from_numpy(x).cuda(), N, K).cpu().numpy()
+        assert capi.lib().b200_check_device_waits() == 0
+        check(got, want, size, K)
+
+
+@pytest.mark.parametrize("ty,N,K,M", [(orc.TYPE_Q4_K, 20000, 4096, 16), (orc.TYPE_Q6_K, 20000, 4096, 16), (orc.TYPE_Q6_K, 6000, 2816, 200)])
+def test_long_shares_and_cut_tiles(ty, N, K, M):
+    """a CTA walks through more blocks than any ring has stages, and through parts of tiles"""
+    import torch
+
+    from mesh_llm_b200 import capi, ops
+
+    W = blocks_of(ty, N, K, 5)
+    dev = ops.upload_weights(ty, W, N, K)
+    x = np.random.default_rng(6).standard_normal((M, K)).astype(np.float32)
+    want, size = exact(ty, W, x, N, K)
+    xd = torch.from_numpy(x).cuda()
+    got = [ops.mul_mat(ty, dev, xd, N, K) for _ in range(3)]
+    assert capi.lib().b200_check_device_waits() == 0
+    assert torch.equal(got[0], got[1]) and torch.equal(got[0], got[2]) # the order of additions does not depend on the timing
+    check(got[0].cpu().numpy(), want, size, K)
+
+
+def test_more_tokens_than_a_slab():
+    import torch
+
+    from mesh_llm_b200 import ops
+
+    N, K, M = 130, 256, 4100
+    W = blocks_of(orc.TYPE_Q4_K, N, K, 7)
+    x = np.random.default_rng(8).standard_normal((M, K)).astype(np.float32)
+    want, size = exact(orc.TYPE_Q4_K, W, x, N, K)
+    got = ops.mul_mat(orc.TYPE_Q4_K, ops.upload_weights(orc.TYPE_Q4_K, W, N, K), torch.from_numpy(x).cuda(), N, K).cpu().numpy()
+    check(got, want, size, K)
+
+
+@pytest.mark.parametrize("ty", [orc.TYPE_Q4_K, orc.TYPE_Q6_K], ids=["q4_k", "q6_k"])
+@pytest.mark.parametrize("rows,ku,E,N,K", [(5, 2, 3, 100, 768), (300, 2, 4, 192, 512), (16, 8, 128, 64, 256)])
+def test_experts(ty, rows, ku, E, N, K):
+    """experts without pairs, with one, and with more than a tile; rows of an expert that end inside a tile"""
+    import torch
+
+    from mesh_llm_b200 import capi, ops
+
+    rng = np.random.default_rng(rows)
+    W = blocks_of(ty, E * N, K, 9)
+    x = rng.standard_normal((rows, K)).astype(np.float32)
+    ids = rng.integers(0, E, rows * ku).astype(np.int32)
+    ids[ids == 1] = 0
+    ids[-1] = 1
+    got = ops.mul_mat_id(ty, ops.upload_weights(ty, W, E * N, K), E, torch.from_numpy(x).cuda(), torch.from_numpy(ids).cuda(), N, K).cpu().numpy()
+    assert capi.lib().b200_check_device_waits() == 0
+    for e in range(E):
+        at = np.nonzero(ids == e)[0]
+        if len(at):
+            want, size = exact(ty, W[e * N:(e + 1) * N], x[at // ku], N, K)
+            check(got[at], want, size, K)
