@@ -156,11 +156,9 @@ b200_status b200_mul_mat_q8(uint32_t type, const void *W, const int8_t *q, const
                (long long)M, (long long)N, (long long)K);
     KQ_REQUIRE(type == B200_TYPE_Q4_K || type == B200_TYPE_Q6_K, "mul_mat: weight type %u", type);
     cudaStream_t st = (cudaStream_t)stream;
-    if (M <= 8) {
-        KqGemvSeg sg = {(const uint8_t *)W, type, (int32_t)N, y, bias, (int32_t)N, 0};
-        return kq_launch_gemv(&sg, 1, q, d, bsum16, (int)M, K, residual, 0, nullptr, st);
-    }
-    return kq_launch_gemm(type, (const uint8_t *)W, q, d, bsum16, M, N, K, y, bias, residual, st);
+    KqGemvSeg sg = {(const uint8_t *)W, type, (int32_t)N, y, bias, (int32_t)N, 0};
+    if (M <= 8) return kq_launch_gemv(&sg, 1, q, d, bsum16, (int)M, K, residual, 0, nullptr, st);
+    return kq_launch_gemm(&sg, 1, q, d, bsum16, M, K, residual, st);
 }
 
 size_t b200_mul_mat_bf16_scratch_bytes(int64_t M, int64_t K) { return M <= 8 ? 256 : (size_t)(M * kq_bf16_ld(K) * 2 + 256); }
@@ -222,13 +220,12 @@ b200_status b200_mul_mat_id(uint32_t type, const void *W, int64_t E, const float
     if (rc != B200_OK) return rc;
     const int act_div = (int)(n_pairs / n_x_rows);
     const int64_t estride = kq_device_row_bytes(type, K) * N;
+    KqGemvSeg sg = {(const uint8_t *)W, type, (int32_t)N, y, nullptr, (int32_t)N, estride};
     if (n_pairs > 8) { // many pairs: gathered per expert, one grouped launch of the tensor-core kernel
         rc = kq_moe_sort(ids, n_pairs, E, sorted, kq_moe_sort_scratch_bytes(n_pairs, E), st);
         if (rc != B200_OK) return rc;
-        rc = kq_launch_gemm_grouped(type, (const uint8_t *)W, estride, q, d, bs, act_div, n_pairs, E, N, K, y, sorted, st);
-        if (rc != B200_ERR_UNSUPPORTED) return rc;
+        return kq_launch_gemm_grouped(&sg, 1, q, d, bs, act_div, n_pairs, E, K, sorted, st);
     }
-    KqGemvSeg sg = {(const uint8_t *)W, type, (int32_t)N, y, nullptr, (int32_t)N, estride};
     KqGemvIndirect ind = {ids, (int32_t)n_pairs, (int32_t)act_div};
     return kq_launch_gemv(&sg, 1, q, d, bs, 1, K, nullptr, 0, &ind, st);
 }

@@ -310,9 +310,8 @@ b200_status kq_rms_norm(const float *x, const float *w, int64_t T, int64_t h, fl
 // launch of the tensor-core GEMM per expert-packed matrix (y[pair][N] = W[expert(pair)] . x[pair / act_div])
 size_t kq_moe_sort_scratch_bytes(int64_t n_pairs, int64_t E);
 b200_status kq_moe_sort(const int32_t *ids, int64_t n_pairs, int64_t E, int32_t *scratch, size_t scratch_bytes, cudaStream_t st);
-b200_status kq_launch_gemm_grouped(uint32_t type, const uint8_t *W, int64_t expert_stride, const int8_t *q, const float *d,
-                                   const int16_t *bs, int act_div, int64_t n_pairs, int64_t E, int64_t N, int64_t K, float *y,
-                                   const int32_t *sorted, cudaStream_t st);
+b200_status kq_launch_gemm_grouped(const KqGemvSeg *segs, int nseg, const int8_t *q, const float *d, const int16_t *bs, int act_div,
+                                   int64_t n_pairs, int64_t E, int64_t K, const int32_t *sorted, cudaStream_t st);
 int kq_stream_error_fetch(); // 0 ok; nonzero = a bounded device-side wait gave up since the last call
 int kq_gemm_error_fetch();
 int kq_attn_tc_error_fetch();
@@ -321,6 +320,6 @@ int kq_prompt_attn_error_fetch();
 int kq_state_error_fetch();
 int kq_state_chunk_error_fetch();
 int kq_device_wait_errors(); // all of the above in one code
-b200_status kq_launch_gemm(uint32_t type, const uint8_t *W, const int8_t *q, const float *d,
-                           const int16_t *bs, int64_t M, int64_t N, int64_t K, float *y,
-                           const float *bias, const float *residual, cudaStream_t st);
+// more than 8 tokens, up to three matrices of rows of K (any mix of types) on the same tokens; a residual with one matrix only
+b200_status kq_launch_gemm(const KqGemvSeg *segs, int nseg, const int8_t *q, const float *d, const int16_t *bs, int64_t M, int64_t K,
+                           const float *residual, cudaStream_t st);

@@ -14,6 +14,8 @@
 // two warpgroups drain the accumulators into the running f32 result, which stays in registers for the whole tile.  Lanes of a
 // warp hold neighbouring rows of W, so results leave in full lines.
 //
+// Up to three matrices that read the same tokens (q / k / v, gate / up) share the image and, type by type, the launch: the small ones would
+// leave most of the GPU idle (256 x 2048 at 77 tokens: 19 us alone, two of them in the launch of q: none).
 // The (tile, block) pairs are dealt out to the CTAs in equal contiguous shares, so that any number of tiles fills the GPU.  A tile
 // that was cut is added up, in the order of its parts, by the CTA that arrives last; nobody waits.
 //
@@ -54,14 +56,21 @@ struct Cfg {
 __device__ int g_gemm_error;
 __device__ int g_parts_done[MAX_CTAS]; // parts of a cut tile that have been written, by the CTA that holds its first block; back to zero after use
 
+constexpr int MAX_SEGS = 3;
+struct Seg { // one of the matrices that share the tokens
+    float *y;
+    const float *bias;
+    const uint8_t *W;
+    int32_t N, tile_end; // rows; row tiles up to this matrix's last
+};
 struct Params {
-    CUtensorMap w, w_tail; // packed blocks; Q6_K: rows' full groups of eight blocks, and their last, smaller group
+    CUtensorMap w[2 * MAX_SEGS]; // packed blocks; Q6_K: rows' full groups of eight blocks, then their last, smaller group
+    Seg seg[MAX_SEGS];
     const uint8_t *img;    // token images [block][8 tokens][GROUP_BYTES]
     const float *da;       // activation scales [block][m_pad]
-    const uint8_t *W;
-    float *y, *part;
-    const float *bias, *residual;
-    int32_t M, N, nb, m_pad, row_tiles, tok_tiles, tile_tok, min_share;
+    float *part;
+    const float *residual; // with one matrix only
+    int32_t M, nb, m_pad, row_tiles, tok_tiles, tile_tok, min_share;
     int64_t w_row;
     // products with experts: token tile t belongs to expert tile_expert[t] and holds the tile_count[t] pairs row_src[128 t ..]
     const int32_t *row_src, *tile_expert, *tile_count, *n_tiles;
@@ -73,12 +82,15 @@ __host__ __device__ __forceinline__ void chunks_of(int n, int &c, int &cw) { // 
 }
 
 struct TilePos {
-    int n0, t0, n, c, cw, expert;
+    int n0, t0, n, c, cw, expert, seg;
 };
+// selects, not indexing: parameters indexed by a variable are read through generic loads
+__device__ __forceinline__ int seg_rows(const Params &p, int s) { return s == 0 ? p.seg[0].N : s == 1 ? p.seg[1].N : p.seg[2].N; }
 __device__ __forceinline__ TilePos tile_at(const Params &p, int tile) {
     TilePos t;
-    const int tt = tile / p.row_tiles;
-    t.n0 = (tile - tt * p.row_tiles) * ROWS;
+    const int tt = tile / p.row_tiles, rt = tile - tt * p.row_tiles;
+    t.seg = (rt >= p.seg[0].tile_end) + (rt >= p.seg[1].tile_end);
+    t.n0 = (rt - (t.seg == 0 ? 0 : t.seg == 1 ? p.seg[0].tile_end : p.seg[1].tile_end)) * ROWS;
     if (p.row_src) {
         t.t0 = tt * 128, t.n = p.tile_count[tt], t.expert = p.tile_expert[tt];
     } else {
@@ -191,16 +203,16 @@ __global__ void __launch_bounds__(NTHREADS, 1) gemm_kq_kernel(const __grid_const
                     if (lead) {
                         bar_expect(&raw_full[s], C::RAW_BYTES);
                         const uint32_t dst = smem_u32(smem + C::SM_RAW + s * C::RAW_BYTES), bar = smem_u32(&raw_full[s]);
-                        const int row = t.expert * p.N + t.n0;
+                        const int row = t.expert * seg_rows(p, t.seg) + t.n0;
                         if (Q6) {
                             const int grp = b / KQ_Q6_GROUP, full = nb / KQ_Q6_GROUP, x = (b % KQ_Q6_GROUP) / 2 * 32;
-                            const CUtensorMap *m = grp < full ? &p.w : &p.w_tail;
+                            const CUtensorMap *m = p.w + 2 * t.seg + (grp < full ? 0 : 1);
                             asm volatile("cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], [%6];" ::"r"(dst),
                                          "l"(m), "r"(x), "r"(row), "r"(0), "r"(grp < full ? grp : 0), "r"(bar)
                                          : "memory");
                         } else {
                             asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(dst),
-                                         "l"(&p.w), "r"(b * KQ_Q4K_BYTES), "r"(row), "r"(bar)
+                                         "l"(p.w + 2 * t.seg), "r"(b * KQ_Q4K_BYTES), "r"(row), "r"(bar)
                                          : "memory");
                         }
                     }
@@ -360,7 +372,8 @@ __global__ void __launch_bounds__(NTHREADS, 1) gemm_kq_kernel(const __grid_const
             for (int u = 0; u < total && ok; u++) {
                 if (u == 0 || b == 0) {
                     const TilePos t = tile_at(p, tile);
-                    wr = p.W + ((int64_t)t.expert * p.N + min(t.n0 + row, p.N - 1)) * p.w_row;
+                    const int n = seg_rows(p, t.seg);
+                    wr = (t.seg == 0 ? p.seg[0].W : t.seg == 1 ? p.seg[1].W : p.seg[2].W) + ((int64_t)t.expert * n + min(t.n0 + row, n - 1)) * p.w_row;
                 }
                 if (u == 0 || b % KQ_Q6_GROUP == 0)
                     dv = __ldg(reinterpret_cast<const uint4 *>(wr + kq_q6_addr(nb, b / KQ_Q6_GROUP * KQ_Q6_GROUP).d));
@@ -474,31 +487,35 @@ __global__ void __launch_bounds__(NTHREADS, 1) gemm_kq_kernel(const __grid_const
                 auto cta_of = [&](uint32_t v) { return v < big ? v / (per + 1) : rem + (v - big) / per; };
                 const uint32_t c0 = cta_of(first), c1 = cta_of(first + nb - 1);
                 // 16 tokens of this thread's row, from token col0 of the tile on
+                const Seg &sg = t.seg == 0 ? p.seg[0] : t.seg == 1 ? p.seg[1] : p.seg[2];
+                const int N = sg.N;
+                float *const y_out = sg.y;
+                const float *const bias_in = sg.bias;
                 auto put = [&](float (&v)[16], int col0) {
                     const int n = t.n0 + row, live = t.n - col0;
-                    if (n >= p.N) return;
+                    if (n >= N) return;
                     if (p.row_src) {
                         const int32_t *src = p.row_src + t.t0 + col0;
 #pragma unroll
                         for (int j = 0; j < 16; j++)
-                            if (j < live) p.y[(int64_t)src[j] * p.N + n] = v[j];
+                            if (j < live) y_out[(int64_t)src[j] * N + n] = v[j];
                         return;
                     }
-                    const int64_t o = (int64_t)(t.t0 + col0) * p.N + n;
-                    if (p.bias) {
-                        const float bias = p.bias[n];
+                    const int64_t o = (int64_t)(t.t0 + col0) * N + n;
+                    if (bias_in) {
+                        const float bias = bias_in[n];
 #pragma unroll
                         for (int j = 0; j < 16; j++) v[j] += bias;
                     }
                     if (p.residual) {
                         const float *src = p.residual + o;
 #pragma unroll
-                        for (int j = 0; j < 16; j++, src += p.N)
+                        for (int j = 0; j < 16; j++, src += N)
                             if (j < live) v[j] += *src;
                     }
-                    float *dst = p.y + o;
+                    float *dst = y_out + o;
 #pragma unroll
-                    for (int j = 0; j < 16; j++, dst += p.N)
+                    for (int j = 0; j < 16; j++, dst += N)
                         if (j < live) *dst = v[j];
                 };
 #pragma unroll 1
@@ -778,39 +795,67 @@ b200_status scratch(int dev, size_t img_bytes, size_t da_bytes, Scratch *out) {
     return B200_OK;
 }
 
-b200_status weight_maps(Params &p, uint32_t type, const uint8_t *W, int64_t rows, int64_t K) {
-    const uint64_t row = (uint64_t)kq_device_row_bytes(type, K);
-    p.W = W;
+b200_status add_seg(Params &p, int i, const KqGemvSeg &g, int64_t experts, int64_t K) {
+    CUtensorMap *w = p.w + 2 * i;
+    const int64_t rows = g.n_rows * experts;
+    const uint64_t row = (uint64_t)kq_device_row_bytes(g.type, K);
     p.w_row = (int64_t)row;
-    if (type == B200_TYPE_Q4_K) {
+    if (g.type == B200_TYPE_Q4_K) {
         const uint64_t dims[2] = {row, (uint64_t)rows}, str[1] = {row};
         const uint32_t box[2] = {KQ_Q4K_BYTES, ROWS};
-        KQ_TRY(kq_tmap_encode(&p.w, 1, 2, W, dims, str, box, 0));
-        p.w_tail = p.w;
-        return B200_OK;
+        KQ_TRY(kq_tmap_encode(w, 1, 2, g.W, dims, str, box, 0));
+    } else {
+        const int full = (int)(K / 256 / KQ_Q6_GROUP), tail = (int)(K / 256 % KQ_Q6_GROUP);
+        const uint32_t box[4] = {32, ROWS, 13, 1}; // two blocks' 16-byte chunks: 8 of low nibbles, 4 of high bits, the scales
+        if (full) {
+            const uint64_t dims[4] = {KQ_Q6_GROUP * 16, (uint64_t)rows, 13, (uint64_t)full}, str[3] = {row, KQ_Q6_GROUP * 16, KQ_Q6_GROUP_BYTES};
+            KQ_TRY(kq_tmap_encode(w, 1, 4, g.W, dims, str, box, 0));
+        }
+        if (tail) {
+            const uint64_t dims[4] = {(uint64_t)tail * 16, (uint64_t)rows, 13, 1}, str[3] = {row, (uint64_t)tail * 16, row};
+            KQ_TRY(kq_tmap_encode(w + 1, 1, 4, g.W + (int64_t)full * KQ_Q6_GROUP_BYTES, dims, str, box, 0));
+        }
     }
-    const int full = (int)(K / 256 / KQ_Q6_GROUP), tail = (int)(K / 256 % KQ_Q6_GROUP);
-    const uint32_t box[4] = {32, ROWS, 13, 1}; // two blocks' 16-byte chunks: 8 of low nibbles, 4 of high bits, the scales
-    if (full) {
-        const uint64_t dims[4] = {KQ_Q6_GROUP * 16, (uint64_t)rows, 13, (uint64_t)full}, str[3] = {row, KQ_Q6_GROUP * 16, KQ_Q6_GROUP_BYTES};
-        KQ_TRY(kq_tmap_encode(&p.w, 1, 4, W, dims, str, box, 0));
-    }
-    if (tail) {
-        const uint64_t dims[4] = {(uint64_t)tail * 16, (uint64_t)rows, 13, 1}, str[3] = {row, (uint64_t)tail * 16, row};
-        KQ_TRY(kq_tmap_encode(&p.w_tail, 1, 4, W + (int64_t)full * KQ_Q6_GROUP_BYTES, dims, str, box, 0));
-    }
-    if (!full) p.w = p.w_tail;
-    if (!tail) p.w_tail = p.w;
+    p.row_tiles += (int)kq_div_up(g.n_rows, ROWS);
+    p.seg[i] = {g.y, g.bias, g.W, g.n_rows, p.row_tiles};
+    for (int k = i + 1; k < MAX_SEGS; k++) p.seg[k].tile_end = 0x7fffffff;
     return B200_OK;
 }
 
-constexpr int MIN_SHARE = 4; // blocks of a CTA at least
+// Blocks of a CTA at least: shorter shares are shorter chains, but more parts to add up.  77 tokens through nine layers of the 3B shape take
+// 1457 / 1468 / 1633 us at 2 / 4 / 8, 16 users of the experts' model 1073 / 1089 / 1132; large products do not depend on it.
+constexpr int MIN_SHARE = 2;
 
-b200_status launch(const Params &p, uint32_t type, int grid, cudaStream_t st) {
-    if (type == B200_TYPE_Q4_K) KQ_CUDA(kq_launch(gemm_kq_kernel<false>, dim3(grid), dim3(NTHREADS), Cfg<false>::SMEM, st, p));
-    else KQ_CUDA(kq_launch(gemm_kq_kernel<true>, dim3(grid), dim3(NTHREADS), Cfg<true>::SMEM, st, p));
-    KQ_COUNT_LAUNCH();
-    KQ_LAUNCH_CHECK();
+// one launch per weight type for the matrices that read the image in p
+b200_status launch_segs(Params p, const KqGemvSeg *segs, int nseg, int64_t experts, int64_t K, cudaStream_t st) {
+    for (const uint32_t type : {(uint32_t)B200_TYPE_Q4_K, (uint32_t)B200_TYPE_Q6_K}) {
+        int n = 0;
+        p.row_tiles = 0;
+        for (int i = 0; i < nseg; i++)
+            if (segs[i].type == type) KQ_TRY(add_seg(p, n++, segs[i], experts, K));
+        if (!n) continue;
+        p.min_share = MIN_SHARE;
+        const int64_t units = (int64_t)p.tok_tiles * p.row_tiles * p.nb;
+        KQ_REQUIRE(units < (int64_t)1 << 31, "gemm: bad shape");
+        // with experts the number of tiles is known on the device only
+        const int grid = p.row_src ? kq_sm_count() : (int)std::min<int64_t>(kq_sm_count(), std::max<int64_t>(1, units / p.min_share));
+        if (type == B200_TYPE_Q4_K) KQ_CUDA(kq_launch(gemm_kq_kernel<false>, dim3(grid), dim3(NTHREADS), Cfg<false>::SMEM, st, p));
+        else KQ_CUDA(kq_launch(gemm_kq_kernel<true>, dim3(grid), dim3(NTHREADS), Cfg<true>::SMEM, st, p));
+        KQ_COUNT_LAUNCH();
+        KQ_LAUNCH_CHECK();
+    }
+    return B200_OK;
+}
+
+b200_status check_segs(const KqGemvSeg *segs, int nseg, const int8_t *q, int64_t K, int *dev) {
+    KQ_REQUIRE(nseg >= 1 && nseg <= MAX_SEGS && K > 0 && K % 256 == 0 && ((uintptr_t)q & 15) == 0, "gemm: bad shape");
+    for (int i = 0; i < nseg; i++) {
+        KQ_REQUIRE(segs[i].type == B200_TYPE_Q4_K || segs[i].type == B200_TYPE_Q6_K, "gemm: weight type %u", segs[i].type);
+        KQ_REQUIRE(segs[i].n_rows > 0, "gemm: bad shape");
+        KQ_REQUIRE(((uintptr_t)segs[i].W & 15) == 0, "gemm: operands must be 16-byte aligned");
+    }
+    KQ_CUDA(cudaGetDevice(dev));
+    KQ_REQUIRE(*dev >= 0 && *dev < MAX_DEVICES, "gemm: device %d out of range", *dev);
     return B200_OK;
 }
 
@@ -829,38 +874,35 @@ int kq_gemm_error_fetch() {
 
 constexpr int64_t SLAB = 4096; // tokens whose images are held at a time
 
-b200_status kq_launch_gemm_tc(uint32_t type, const uint8_t *W, const int8_t *q, const float *d, const int16_t *bs, int64_t M, int64_t N,
-                              int64_t K, float *y, const float *bias, const float *residual, cudaStream_t st) {
-    KQ_REQUIRE(type == B200_TYPE_Q4_K || type == B200_TYPE_Q6_K, "gemm: weight type %u", type);
-    KQ_REQUIRE(K % 256 == 0 && M > 0 && N > 0, "gemm: bad shape");
-    KQ_REQUIRE(((uintptr_t)W & 15) == 0 && ((uintptr_t)q & 15) == 0, "gemm: operands must be 16-byte aligned");
+b200_status kq_launch_gemm_tc(const KqGemvSeg *segs, int nseg, const int8_t *q, const float *d, const int16_t *bs, int64_t M, int64_t K,
+                              const float *residual, cudaStream_t st) {
     int dev = 0;
-    KQ_CUDA(cudaGetDevice(&dev));
-    KQ_REQUIRE(dev >= 0 && dev < MAX_DEVICES, "gemm: device %d out of range", dev);
+    KQ_TRY(check_segs(segs, nseg, q, K, &dev));
+    KQ_REQUIRE(M > 0 && (!residual || nseg == 1), "gemm: bad shape");
     const int64_t nb = K / 256;
-    Params p = {};
-    KQ_TRY(weight_maps(p, type, W, N, K));
     for (int64_t m0 = 0; m0 < M; m0 += SLAB) {
         const int64_t mc = std::min(SLAB, M - m0);
+        Params p = {};
         int c, cw;
         p.tok_tiles = (int)kq_div_up(mc, MAX_CHUNKS * CHUNK);
         chunks_of((int)kq_div_up(mc, p.tok_tiles), c, cw);
         p.tile_tok = c * cw;
         p.tok_tiles = (int)kq_div_up(mc, p.tile_tok);
         p.m_pad = p.tok_tiles * p.tile_tok;
+        p.M = (int32_t)mc, p.nb = (int32_t)nb;
         Scratch sc;
         KQ_TRY(scratch(dev, (size_t)p.m_pad * TOK_BYTES * nb, (size_t)p.m_pad * 4 * nb, &sc));
         const ImageParams ip = {q + m0 * K, d + m0 * nb, bs + m0 * nb * 16, sc.img, sc.da, (int32_t)mc, (int32_t)nb, p.m_pad, 1, nullptr, nullptr, nullptr};
         KQ_CUDA(kq_launch(act_image_kernel, dim3((unsigned)nb, (unsigned)(p.m_pad / 16)), dim3(288), 0, st, ip));
         KQ_COUNT_LAUNCH();
         p.img = sc.img, p.da = sc.da, p.part = sc.part;
-        p.y = y + m0 * N, p.bias = bias, p.residual = residual ? residual + m0 * N : nullptr;
-        p.M = (int32_t)mc, p.N = (int32_t)N, p.nb = (int32_t)nb;
-        p.row_tiles = (int)kq_div_up(N, ROWS);
-        p.min_share = MIN_SHARE;
-        const int64_t units = (int64_t)p.tok_tiles * p.row_tiles * nb;
-        KQ_REQUIRE(units < (int64_t)1 << 31, "gemm: bad shape");
-        KQ_TRY(launch(p, type, (int)std::min<int64_t>(kq_sm_count(), std::max<int64_t>(1, units / p.min_share)), st));
+        KqGemvSeg sg[MAX_SEGS];
+        for (int i = 0; i < nseg; i++) {
+            sg[i] = segs[i];
+            sg[i].y += m0 * sg[i].n_rows;
+        }
+        p.residual = residual ? residual + m0 * segs[0].n_rows : nullptr;
+        KQ_TRY(launch_segs(p, sg, nseg, 1, K, st));
     }
     return B200_OK;
 }
@@ -887,22 +929,19 @@ b200_status kq_moe_sort(const int32_t *ids, int64_t n_pairs, int64_t E, int32_t 
     return B200_OK;
 }
 
-// y[pair][N] = W[expert of the pair] . x[pair / act_div]: q / d / bs are the quantised activations of the
-// n_pairs / act_div source rows, sorted = the scratch kq_moe_sort left for these pairs.
-b200_status kq_launch_gemm_grouped(uint32_t type, const uint8_t *W, int64_t expert_stride, const int8_t *q, const float *d,
-                                   const int16_t *bs, int act_div, int64_t n_pairs, int64_t E, int64_t N, int64_t K, float *y,
-                                   const int32_t *sorted, cudaStream_t st) {
-    KQ_REQUIRE(type == B200_TYPE_Q4_K || type == B200_TYPE_Q6_K, "grouped gemm: weight type %u", type);
-    KQ_REQUIRE(K % 256 == 0 && n_pairs > 0 && N > 0 && act_div >= 1, "grouped gemm: bad shape");
-    KQ_REQUIRE(((uintptr_t)W & 15) == 0 && ((uintptr_t)q & 15) == 0 && expert_stride % 16 == 0, "grouped gemm: operands must be 16-byte aligned");
-    KQ_REQUIRE(expert_stride == kq_device_row_bytes(type, K) * N, "grouped gemm: expert matrices must be contiguous");
+// y[pair][N] = W[expert of the pair] . x[pair / act_div] for up to three expert-packed matrices: q / d / bs are the quantised
+// activations of the n_pairs / act_div source rows, sorted = the scratch kq_moe_sort left for these pairs.
+b200_status kq_launch_gemm_grouped(const KqGemvSeg *segs, int nseg, const int8_t *q, const float *d, const int16_t *bs, int act_div,
+                                   int64_t n_pairs, int64_t E, int64_t K, const int32_t *sorted, cudaStream_t st) {
     int dev = 0;
-    KQ_CUDA(cudaGetDevice(&dev));
-    KQ_REQUIRE(dev >= 0 && dev < MAX_DEVICES, "gemm: device %d out of range", dev);
+    KQ_TRY(check_segs(segs, nseg, q, K, &dev));
+    KQ_REQUIRE(n_pairs > 0 && act_div >= 1, "grouped gemm: bad shape");
+    for (int i = 0; i < nseg; i++)
+        KQ_REQUIRE(segs[i].expert_stride == kq_device_row_bytes(segs[i].type, K) * segs[i].n_rows && segs[i].expert_stride % 16 == 0,
+                   "grouped gemm: expert matrices must be contiguous and 16-byte aligned");
     const int64_t nb = K / 256, mt = moe_max_tiles(n_pairs, E);
     Params p = {};
-    KQ_TRY(weight_maps(p, type, W, N * E, K));
-    p.m_pad = (int32_t)(mt * TM);
+    p.M = p.m_pad = (int32_t)(mt * TM), p.nb = (int32_t)nb, p.tok_tiles = (int)mt;
     Scratch sc;
     KQ_TRY(scratch(dev, (size_t)p.m_pad * TOK_BYTES * nb, (size_t)p.m_pad * 4 * nb, &sc));
     p.n_tiles = sorted, p.tile_expert = sorted + 1, p.row_src = sorted + 1 + mt, p.tile_count = sorted + 1 + mt + mt * TM;
@@ -910,11 +949,5 @@ b200_status kq_launch_gemm_grouped(uint32_t type, const uint8_t *W, int64_t expe
     KQ_CUDA(kq_launch(act_image_kernel, dim3((unsigned)nb, (unsigned)(p.m_pad / 16)), dim3(288), 0, st, ip));
     KQ_COUNT_LAUNCH();
     p.img = sc.img, p.da = sc.da, p.part = sc.part;
-    p.y = y;
-    p.M = p.m_pad, p.N = (int32_t)N, p.nb = (int32_t)nb;
-    p.row_tiles = (int)kq_div_up(N, ROWS);
-    p.tok_tiles = (int)mt;
-    p.min_share = MIN_SHARE;
-    KQ_REQUIRE(mt * p.row_tiles * nb < (int64_t)1 << 31, "grouped gemm: bad shape");
-    return launch(p, type, kq_sm_count(), st);
+    return launch_segs(p, segs, nseg, E, K, st);
 }

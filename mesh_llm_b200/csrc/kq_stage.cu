@@ -181,19 +181,17 @@ b200_status forward_body(b200_stage *st, const int32_t *tokens, const float *hid
         // ---- attention block
         const bool fuse = rows <= 2; // the streaming GEMV normalises and quantises its own input
         if (!fuse) OTHER_(kq_rms_norm(xin, L.attn_norm, rows, h, c.rms_eps, nullptr, st->aq, st->ad, st->abs16, s));
+        KqGemvSeg segs[3] = {
+            {(const uint8_t *)L.wq->dev, L.wq->type, nq, st->q, L.bq, nq, 0},
+            {(const uint8_t *)L.wk->dev, L.wk->type, nkv, st->k, L.bk, nkv, 0},
+            {(const uint8_t *)L.wv->dev, L.wv->type, nkv, st->v, L.bv, nkv, 0},
+        };
         if (rows <= 8) {
-            KqGemvSeg segs[3] = {
-                {(const uint8_t *)L.wq->dev, L.wq->type, nq, st->q, L.bq, nq, 0},
-                {(const uint8_t *)L.wk->dev, L.wk->type, nkv, st->k, L.bk, nkv, 0},
-                {(const uint8_t *)L.wv->dev, L.wv->type, nkv, st->v, L.bv, nkv, 0},
-            };
             KqActPrep pr = {xin, L.attn_norm, c.rms_eps, 1};
             GEMV_(kq_launch_gemv(segs, 3, st->aq, st->ad, st->abs16, rows, h, nullptr, 0, nullptr, s,
                                  fuse ? &pr : nullptr));
         } else {
-            GEMV_(mm(st, L.wq, rows, st->q, L.bq, nullptr, s));
-            GEMV_(mm(st, L.wk, rows, st->k, L.bk, nullptr, s));
-            GEMV_(mm(st, L.wv, rows, st->v, L.bv, nullptr, s));
+            GEMV_(kq_launch_gemm(segs, 3, st->aq, st->ad, st->abs16, rows, h, nullptr, s));
         }
         if (c.qk_norm) {
             OTHER_(kq_rms_norm(st->q, L.q_norm, (int64_t)rows * c.n_head, hd, c.rms_eps, st->q, nullptr,
@@ -309,13 +307,11 @@ b200_status forward_body(b200_stage *st, const int32_t *tokens, const float *hid
             bool grouped = grouped_on && rows > 8 && fe % 64 == 0 && h % 64 == 0 && classes == CLS_ALL;
             if (grouped) {
                 KQ_TRY(kq_moe_sort(st->rid, pairs, E, st->moe_sorted, st->moe_sorted_bytes, s));
-                KQ_TRY(kq_launch_gemm_grouped(L.gate_e->type, (const uint8_t *)L.gate_e->dev, gstride, st->aq, st->ad, st->abs16, ku,
-                                              pairs, E, fe, h, st->hp, st->moe_sorted, s));
-                KQ_TRY(kq_launch_gemm_grouped(L.up_e->type, (const uint8_t *)L.up_e->dev, gstride, st->aq, st->ad, st->abs16, ku,
-                                              pairs, E, fe, h, st->hp2, st->moe_sorted, s));
+                const KqGemvSeg both[2] = {gu[0], {gu[1].W, gu[1].type, fe, st->hp2, nullptr, fe, kq_device_row_bytes(gu[1].type, h) * fe}};
+                KQ_TRY(kq_launch_gemm_grouped(both, 2, st->aq, st->ad, st->abs16, ku, pairs, E, h, st->moe_sorted, s));
                 KQ_TRY(kq_swiglu_quantize(st->hp, st->hp2, pairs, fe, st->hp, st->aq, st->ad, st->abs16, s));
-                KQ_TRY(kq_launch_gemm_grouped(L.down_e->type, (const uint8_t *)L.down_e->dev, dstride, st->aq, st->ad, st->abs16, 1,
-                                              pairs, E, h, fe, st->yp, st->moe_sorted, s));
+                const KqGemvSeg down = {(const uint8_t *)L.down_e->dev, L.down_e->type, h, st->yp, nullptr, h, dstride};
+                KQ_TRY(kq_launch_gemm_grouped(&down, 1, st->aq, st->ad, st->abs16, 1, pairs, E, fe, st->moe_sorted, s));
             } else {
             KqGemvIndirect ind = {st->rid, pairs, ku};
             b200_status rg = B200_ERR_UNSUPPORTED;
@@ -346,11 +342,11 @@ b200_status forward_body(b200_stage *st, const int32_t *tokens, const float *hid
         } else {
             if (!fuse) OTHER_(kq_rms_norm(st->x, L.ffn_norm, rows, h, c.rms_eps, nullptr, st->aq, st->ad, st->abs16, s));
             KqEmitQ8 emit = {st->aq, st->ad, st->abs16, st->emit_counters, 0};
+            KqGemvSeg gu[2] = {
+                {(const uint8_t *)L.gate->dev, L.gate->type, c.n_ff, st->g, nullptr, c.n_ff, 0},
+                {(const uint8_t *)L.up->dev, L.up->type, c.n_ff, rows <= 8 ? st->g : st->u, nullptr, c.n_ff, 0},
+            };
             if (rows <= 8) {
-                KqGemvSeg gu[2] = {
-                    {(const uint8_t *)L.gate->dev, L.gate->type, c.n_ff, st->g, nullptr, c.n_ff, 0},
-                    {(const uint8_t *)L.up->dev, L.up->type, c.n_ff, st->g, nullptr, c.n_ff, 0},
-                };
                 KqActPrep pr = {st->x, L.ffn_norm, c.rms_eps, 1};
                 // the launch also leaves the Q8 form of its output for the down projection (B200_GEMV_EMIT_Q8=0: off)
                 const char *ev = getenv("B200_GEMV_EMIT_Q8"); // read when a step is captured
@@ -358,8 +354,7 @@ b200_status forward_body(b200_stage *st, const int32_t *tokens, const float *hid
                 GEMV_(kq_launch_gemv(gu, 2, st->aq, st->ad, st->abs16, rows, h, nullptr, 1, nullptr, s,
                                      fuse ? &pr : nullptr, want ? &emit : nullptr));
             } else {
-                GEMV_(mm(st, L.gate, rows, st->g, nullptr, nullptr, s));
-                GEMV_(mm(st, L.up, rows, st->u, nullptr, nullptr, s));
+                GEMV_(kq_launch_gemm(gu, 2, st->aq, st->ad, st->abs16, rows, h, nullptr, s));
                 // SwiGLU and the Q8 form the down projection reads, in one pass
                 OTHER_(kq_swiglu_quantize(st->g, st->u, rows, c.n_ff, st->g, st->aq, st->ad, st->abs16, s));
             }
