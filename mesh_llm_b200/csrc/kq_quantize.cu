@@ -92,6 +92,29 @@ __global__ void __launch_bounds__(256) rms_norm_kernel(const float *x,
     }
 }
 
+// Rows of up to 128 values (one head), f32 output only: a warp per row, with the sums in the order of the kernel above, which gives such a row
+// 256 threads and two barriers.  32768 rows of 128: 52 -> 9 us.
+__global__ void __launch_bounds__(256) rms_norm_head_kernel(const float *x, const float *w, int64_t rows, int h, float eps, float *y, int64_t x_row_stride) {
+    KQ_PDL_ENTER();
+    const int lane = threadIdx.x & 31;
+    const int64_t row = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
+    if (row >= rows) return;
+    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (lane * 4 < h) v = *reinterpret_cast<const float4 *>(x + row * x_row_stride + lane * 4);
+    double ss = (double)v.x * v.x + (double)v.y * v.y + (double)v.z * v.z + (double)v.w * v.w;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+    const float scale = 1.0f / sqrtf((float)(ss / (double)h) + eps);
+    if (lane * 4 < h) {
+        float f[4] = {1.f, 1.f, 1.f, 1.f};
+        if (w) {
+#pragma unroll
+            for (int i = 0; i < 4; i++) f[i] = w[lane * 4 + i];
+        }
+        *reinterpret_cast<float4 *>(y + row * h + lane * 4) = make_float4(v.x * scale * f[0], v.y * scale * f[1], v.z * scale * f[2], v.w * scale * f[3]);
+    }
+}
+
 // ---- Q6_K repack: GGUF block-interleaved rows <-> device rows [ql | qh | scales | d | pad] ------
 __global__ void repack_q6k_kernel(const uint16_t *src, uint16_t *dst,
                                   int64_t n_rows, int nb, int64_t dst_row_u16, int inverse) {
@@ -275,6 +298,13 @@ b200_status kq_rms_norm(const float *x, const float *w, int64_t T, int64_t h, fl
     KQ_REQUIRE(T > 0 && h > 0 && h % 4 == 0, "rms_norm: bad shape");
     KQ_REQUIRE(!q || h % 256 == 0, "rms_norm: Q8 output needs h %% 256 == 0");
     KQ_REQUIRE(y || q, "rms_norm: no output");
+    const int64_t ldx = x_row_stride ? x_row_stride : h;
+    if (!q && h <= 128 && ldx % 4 == 0 && (((uintptr_t)x | (uintptr_t)y) & 15) == 0) {
+        kq_launch(rms_norm_head_kernel, (unsigned)kq_div_up(T, 8), 256, 0, st, x, w, T, (int)h, eps, y, ldx);
+        KQ_COUNT_LAUNCH();
+        KQ_LAUNCH_CHECK();
+        return B200_OK;
+    }
     kq_launch(rms_norm_kernel, (unsigned)T, 256, 0, st, x, w, (int)h, eps, y, q, d, bs, x_row_stride ? x_row_stride : h);
     KQ_COUNT_LAUNCH();
     KQ_LAUNCH_CHECK();

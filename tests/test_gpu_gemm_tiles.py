@@ -112,3 +112,17 @@ def test_experts(ty, rows, ku, E, N, K):
         if len(at):
             want, size = exact(ty, W[e * N:(e + 1) * N], x[at // ku], N, K)
             check(got[at], want, size, K)
+
+
+@pytest.mark.parametrize("h", [4, 64, 128, 132, 256])
+def test_norm_of_short_rows(h):
+    """a warp per row up to 128 values, a CTA above; the sum of squares is taken in double, then three f32 roundings"""
+    import torch
+
+    from mesh_llm_b200 import ops
+
+    x = np.random.default_rng(h).standard_normal((37, h)).astype(np.float32)
+    w = np.random.default_rng(h + 1).standard_normal(h).astype(np.float32)
+    got = ops.rms_norm(torch.from_numpy(x).cuda(), torch.from_numpy(w).cuda(), 1e-6).cpu().numpy()
+    want = x.astype(np.float64) / np.sqrt((x.astype(np.float64) ** 2).mean(-1, keepdims=True) + 1e-6) * w
+    assert np.all(np.abs(got - want) <= 2.0 ** -21 * np.abs(want))
