@@ -646,17 +646,18 @@ __global__ void __launch_bounds__(288) act_image_kernel(const __grid_constant__ 
 // ---- expert-major order of the (token, slot) pairs of a routed batch (MUL_MAT_ID with many tokens) ----
 // A stable counting sort by expert: the pairs of expert e, in pair order, become the rows of that
 // expert's token tiles; every expert starts on a tile boundary, the rows behind its last pair are
-// padding (-1).  One CTA of 8 warps; warp w walks a contiguous range of the pairs 32 at a time, so the
-// order inside an expert is the pair order whatever the timing.  Output: n_tiles, the expert of each
+// padding (-1).  One CTA of 16 warps; warp w walks a contiguous range of the pairs 32 at a time, so the
+// order inside an expert is the pair order whatever the timing (with 8 warps and a serial table of tiles 55 us
+// for 8192 pairs and 128 experts, now 27).  Output: n_tiles, the expert of each
 // tile, and for each tile row the pair it holds.
-constexpr int TM = 128, SORT_WARPS = 8, SORT_MAX_E = 256;
+constexpr int TM = 128, SORT_WARPS = 16, SORT_MAX_E = 256;
 __global__ void __launch_bounds__(SORT_WARPS * 32) moe_sort_kernel(const int32_t *ids, int n_pairs, int E,
                                                                    int32_t *n_tiles_out, int32_t *tile_expert, int32_t *row_src,
                                                                    int32_t *tile_count) {
     KQ_PDL_ENTER();
     __shared__ int cnt[SORT_WARPS][SORT_MAX_E]; // pass 1: pairs of expert e in warp w's range; then the range's offset inside the expert
     __shared__ int tile_start[SORT_MAX_E];
-    __shared__ int s_tiles;
+    __shared__ int s_tiles, s_warp[8];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     for (int i = threadIdx.x; i < SORT_WARPS * SORT_MAX_E; i += blockDim.x) (&cnt[0][0])[i] = 0;
     __syncthreads();
@@ -681,16 +682,26 @@ __global__ void __launch_bounds__(SORT_WARPS * 32) moe_sort_kernel(const int32_t
         tile_start[threadIdx.x] = run; // the expert's pair count, for the moment
     }
     __syncthreads();
-    if (threadIdx.x == 0) {
-        int t = 0;
-        for (int e = 0; e < E; e++) {
-            const int n = tile_start[e], nt = (n + TM - 1) / TM;
+    if (warp < 8) { // tiles in front of every expert's first: a scan over the warp, then over the warps
+        const int e = threadIdx.x, n = e < E ? tile_start[e] : 0, nt = (n + TM - 1) / TM;
+        int incl = nt;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int v = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += v;
+        }
+        if (lane == 31) s_warp[warp] = incl;
+        asm volatile("bar.sync 1, 256;" ::: "memory");
+        int t = incl - nt;
+        for (int w = 0; w < warp; w++) t += s_warp[w];
+        if (e < E) {
             tile_start[e] = t;
             for (int k = 0; k < nt; k++) tile_expert[t + k] = e, tile_count[t + k] = min(TM, n - k * TM);
-            t += nt;
+            if (e == E - 1) {
+                s_tiles = t + nt;
+                *n_tiles_out = t + nt;
+            }
         }
-        s_tiles = t;
-        *n_tiles_out = t;
     }
     __syncthreads();
     const int live = s_tiles * TM;
