@@ -256,7 +256,11 @@ b200_status launch_gemv(const GemvParams &p, size_t smem, cudaStream_t st) {
     }
     const int64_t units = p.V / (p.c.glu ? 2 : 1);
     const int64_t want = std::max<int64_t>(1, kq_div_up(units * (p.c.glu ? 2 : 1), 4));
-    const unsigned grid = (unsigned)std::min<int64_t>(want, (int64_t)kq_sm_count() * mul);
+    // no more CTAs than run at the same time: every one prepares the activations for itself, and 8 rows of 3072 leave room for one per SM
+    // (8 rows, 2 x 9216 rows of weights of 3072: 153 us in four waves, 92 in one)
+    int fit = 1;
+    KQ_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit, gemv_bf16_kernel<M>, NT, smem));
+    const unsigned grid = (unsigned)std::min<int64_t>(want, (int64_t)kq_sm_count() * std::max(1, std::min(mul, fit)));
     kq_launch(gemv_bf16_kernel<M>, grid, NT, smem, st, p);
     KQ_COUNT_LAUNCH();
     KQ_LAUNCH_CHECK();
