@@ -242,7 +242,11 @@ __device__ __forceinline__ void rec_coeff(float r, float i, float u, float decay
 // Prefill in two passes over chunks of `chunk` positions, a thread per channel.  First: coefficients (over the gates, in
 // place) and each chunk's map of the state, s -> A s + B.  Second: the state in front of a chunk from the maps of the
 // chunks before it, then the recurrence inside the chunk.
-constexpr int RC = 128, RCHUNK = 64; // channels per CTA, positions per chunk
+constexpr int RC = 128, RCHUNK = 16, RCHUNKS = 64; // channels per CTA, positions per chunk at least, chunks at most
+// Positions per chunk.  A thread's walk through its chunk is a chain of dependent steps, and many short chunks hide it; the second pass reads the
+// maps of all chunks in front of its own, so there are not more than 64 of them (a call of 1000 x 3072: 16 chunks of 64 positions
+// take 49 + 42 us, 63 of 16 take 19 + 20).
+__host__ inline int rec_chunk(int T) { return std::max(RCHUNK, (int)kq_div_up(kq_div_up(T, RCHUNKS), RCHUNK) * RCHUNK); }
 __global__ void __launch_bounds__(RC) recurrence_chunks_kernel(const __grid_constant__ KqRecW w, KqRecState st, float *r, float *ig, int64_t ldr, const float *u,
                                                                int64_t ldu, int T, const int32_t *pos0_dev, int pos0_val, int chunk, float *maps) {
     KQ_PDL_ENTER();
@@ -445,15 +449,16 @@ b200_status kq_linear_recurrence(const KqRecW &w, const KqRecState &s, float *r,
                                  float *scratch, size_t scratch_bytes, cudaStream_t st) {
     const b200_status rc = check_rec(w, n_seq, T);
     if (rc != B200_OK) return rc;
-    const unsigned chunks = (unsigned)kq_div_up(T, RCHUNK);
+    const int chunk = rec_chunk(T);
+    const unsigned chunks = (unsigned)kq_div_up(T, chunk);
     KQ_REQUIRE(scratch && scratch_bytes >= (size_t)n_seq * (chunks + 1) * 2 * w.width * 4, "recurrence: scratch");
     const int64_t cols = z16 ? std::max<int64_t>(w.width, ld16) : w.width;
     kq_launch(recurrence_chunks_kernel, dim3((unsigned)kq_div_up(w.width, RC), chunks, (unsigned)n_seq), RC, 0, st, w, s, r, i, ldr, u, ldu, T, pos0_dev,
-              pos0, RCHUNK, scratch);
+              pos0, chunk, scratch);
     KQ_COUNT_LAUNCH();
     KQ_LAUNCH_CHECK();
     kq_launch(recurrence_scan_kernel, dim3((unsigned)kq_div_up(cols, RC), chunks, (unsigned)n_seq), RC, 0, st, w, s, r, i, ldr, x, ldx, y, ldy, T,
-              pos0_dev, pos0, RCHUNK, scratch, z32, ld32, z16, ld16);
+              pos0_dev, pos0, chunk, scratch, z32, ld32, z16, ld16);
     KQ_COUNT_LAUNCH();
     KQ_LAUNCH_CHECK();
     return B200_OK;
