@@ -1,7 +1,7 @@
 // Prefill products with bf16 weights, y[m][n] = sum_k W[n][k] x[m][k]: the tensor-core form (tcgen05.mma
 // kind::f16 on bf16 operands, f32 accumulators in TMEM) and the f32 form on CUDA cores of the 32-bit mode.
 //
-// Tensor cores: a persistent CTA per SM walks tiles of 128 tokens (TMEM lanes) x 256, 128 or 64 weight rows (columns), token
+// Tensor cores: a persistent CTA per SM walks tiles of 128 tokens (TMEM lanes) x 256, 192, 128 or 64 weight rows (columns), token
 // tiles innermost, so that the CTAs at work share the weight rows they read.  K runs in slices of 64 (one
 // 128-byte-swizzled row per operand row); a producer thread brings the slices in by tiled TMA copies through a ring
 // of stages, one thread issues the MMAs into one of two accumulators in TMEM, four warps drain the other one meanwhile,
@@ -27,7 +27,7 @@ template <int TN>
 struct Tile {
     static constexpr int B_BYTES = TN * BK * 2, STAGE_BYTES = A_BYTES + B_BYTES, STAGES = 192 * 1024 / STAGE_BYTES;
     static constexpr int SMEM_TOTAL = STAGES * STAGE_BYTES + EPI_BYTES + 1024;
-    static constexpr uint32_t TMEM_COLS = 2 * TN; // two accumulators
+    static constexpr uint32_t TMEM_COLS = TN == 192 ? 512 : 2 * TN; // two accumulators, in a power of two of columns
 };
 constexpr int NTHREADS = 192, NEPI = 128; // producer warp, MMA warp, four epilogue warps
 constexpr uint64_t LIMIT = 5 * KQ_WAIT_LIMIT_NS;
@@ -390,7 +390,9 @@ b200_status kq_gemm_bf16(const KqDense &c, const uint16_t *a, int64_t lda, int p
     const int64_t sms = kq_sm_count();
     const int64_t w256 = kq_div_up((int64_t)p.mt * n_tiles(256) * c.groups, sms) * 20, w128 = kq_div_up((int64_t)p.mt * n_tiles(128) * c.groups, sms) * 13,
                   w64 = kq_div_up((int64_t)p.mt * n_tiles(64) * c.groups, sms) * 9;
-    const int tn = w256 <= w128 && w256 <= w64 ? 256 : w128 <= w64 ? 128 : 64;
+    // 192 rows fill waves that 256 leave part empty (1000 tokens x 3072 rows: 128 tiles instead of 96 on 148 SMs; with K = 9216 74 -> 67 us, with K = 3072 36 -> 32; 6144 rows 61 -> 51)
+    const int64_t w192 = kq_div_up((int64_t)p.mt * n_tiles(192) * c.groups, sms) * 16;
+    const int tn = w256 <= w192 && w256 <= w128 && w256 <= w64 ? 256 : w192 <= w128 && w192 <= w64 ? 192 : w128 <= w64 ? 128 : 64;
     p.nt = n_tiles(tn);
     {
         const uint64_t dims[3] = {(uint64_t)lda, (uint64_t)c.M, (uint64_t)parts};
@@ -415,11 +417,13 @@ b200_status kq_gemm_bf16(const KqDense &c, const uint16_t *a, int64_t lda, int p
     KQ_CUDA(cudaGetDevice(&dev));
     if (dev < 0 || dev >= 16 || !attr[dev]) {
         KQ_CUDA(cudaFuncSetAttribute(gemm_bf16_kernel<256>, cudaFuncAttributeMaxDynamicSharedMemorySize, Tile<256>::SMEM_TOTAL));
+        KQ_CUDA(cudaFuncSetAttribute(gemm_bf16_kernel<192>, cudaFuncAttributeMaxDynamicSharedMemorySize, Tile<192>::SMEM_TOTAL));
         KQ_CUDA(cudaFuncSetAttribute(gemm_bf16_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, Tile<128>::SMEM_TOTAL));
         KQ_CUDA(cudaFuncSetAttribute(gemm_bf16_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, Tile<64>::SMEM_TOTAL));
         if (dev >= 0 && dev < 16) attr[dev] = true;
     }
     if (tn == 256) kq_launch(gemm_bf16_kernel<256>, grid, NTHREADS, Tile<256>::SMEM_TOTAL, st, p);
+    else if (tn == 192) kq_launch(gemm_bf16_kernel<192>, grid, NTHREADS, Tile<192>::SMEM_TOTAL, st, p);
     else if (tn == 64) kq_launch(gemm_bf16_kernel<64>, grid, NTHREADS, Tile<64>::SMEM_TOTAL, st, p);
     else kq_launch(gemm_bf16_kernel<128>, grid, NTHREADS, Tile<128>::SMEM_TOTAL, st, p);
     KQ_COUNT_LAUNCH();

@@ -126,3 +126,20 @@ def test_norm_of_short_rows(h):
     got = ops.rms_norm(torch.from_numpy(x).cuda(), torch.from_numpy(w).cuda(), 1e-6).cpu().numpy()
     want = x.astype(np.float64) / np.sqrt((x.astype(np.float64) ** 2).mean(-1, keepdims=True) + 1e-6) * w
     assert np.all(np.abs(got - want) <= 2.0 ** -21 * np.abs(want))
+
+
+@pytest.mark.parametrize("M", [300, 900, 1000])
+@pytest.mark.parametrize("N,K", [(3072, 128), (3000, 200), (6200, 64)])
+def test_bf16_tiles(M, N, K):
+    """sizes that choose every tile width, the one of 192 rows among them; bf16 operands, f32 sums of at most 200 terms (truncating: 2^-22 each)"""
+    import torch
+
+    from mesh_llm_b200 import ops
+
+    g = torch.Generator(device="cuda").manual_seed(M + N)
+    w = torch.randn((N, K), generator=g, device="cuda").to(torch.bfloat16)
+    x = torch.randn((M, K), generator=g, device="cuda").to(torch.bfloat16).float()
+    got = ops.mul_mat_bf16(ops.upload_bf16(w.view(torch.int16).cpu().numpy()), x, N, K).double()
+    want = x.double() @ w.double().T
+    size = x.double().abs() @ w.double().abs().T
+    assert ((got - want).abs() <= K * 2.0 ** -22 * size).all()
