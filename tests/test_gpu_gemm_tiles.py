@@ -139,7 +139,30 @@ def test_bf16_tiles(M, N, K):
     g = torch.Generator(device="cuda").manual_seed(M + N)
     w = torch.randn((N, K), generator=g, device="cuda").to(torch.bfloat16)
     x = torch.randn((M, K), generator=g, device="cuda").to(torch.bfloat16).float()
-    got = ops.mul_mat_bf16(ops.upload_bf16(w.view(torch.int16).cpu().numpy()), x, N, K).double()
+    got = ops.mul_mat_bf16(ops.upload_bf16(w), x, N, K).double()
     want = x.double() @ w.double().T
     size = x.double().abs() @ w.double().abs().T
     assert ((got - want).abs() <= K * 2.0 ** -22 * size).all()
+
+
+@pytest.mark.parametrize("n", [1, 3, 4, 255, 2048, 2052, 32001, 151936, 152064])
+def test_greedy_token(n):
+    """the first of the largest values, at the edges of the slices, with infinities and NaN; the same as the statistics' most likely token"""
+    import torch
+
+    from mesh_llm_b200 import capi
+
+    rng = np.random.default_rng(n)
+    x = rng.standard_normal((5, n)).astype(np.float32)
+    x[1, rng.integers(0, n)] = x[1, n - 1] = 9.0
+    x[2] = -np.inf
+    x[3, :] = np.float32(-3.4028235e38)
+    x[4, rng.integers(0, n)] = np.inf
+    if n > 4:
+        x[0, 2] = np.nan
+    L, xd, out = capi.lib(), torch.from_numpy(x).cuda(), torch.empty(5, dtype=torch.int32, device="cuda")
+    scratch = torch.zeros(L.b200_logit_signals_scratch_bytes(5), dtype=torch.uint8, device="cuda")
+    for _ in range(2): # the counters are left as they were found
+        capi.check(L.b200_logit_signals(capi.ptr(xd), 5, n, None, None, capi.ptr(out), capi.ptr(scratch), scratch.numel(), capi.cur_stream()))
+    got = out.cpu().numpy()
+    assert np.array_equal(got, [int(np.argmax(np.where(np.isnan(r), -np.inf, r))) for r in x])
