@@ -21,7 +21,8 @@
 //
 // What bounds it, in clocks per block of 128 rows x 256 tokens: the MMAs 2900 (42 each at N = 64, where 32 would be the tensor
 // rate), the drains 1000 of every scheduler, the decoding of Q4_K 870 (alone; of Q6_K twice as much).  Measured about 5500: what is left are
-// the hand-overs between the roles, of which each accumulator has two per chunk.  Two int8 planes per weight instead (the form
+// the hand-overs between the roles, of which each accumulator has two per chunk, and instruction fetch: four roles run four loops, and
+// the same decoding unrolled four times made the whole kernel 10 % slower.  Two int8 planes per weight instead (the form
 // before this one) had to turn three accumulators per output from integers into floats: 1659 us against 1200 for 2048 tokens x 28672 x 8192
 // in Q4_K (580 -> 800 TFLOP/s), 547 against 312 at 512 tokens, 169 against 68 at 16; Q6_K at 64 tokens 254 against 151 us.
 // Every wait is bounded; on a time-out the kernel records an error, lets its copies and MMAs end, frees its TMEM and returns.
@@ -41,7 +42,7 @@ constexpr int B_BYTES = CHUNK * TOK_BYTES, DA_RING = 8, SC_RING = 8;
 constexpr int TILE_OUT = MAX_CHUNKS * CHUNK * ROWS; // outputs of a tile
 constexpr int MAX_CTAS = 256, MAX_DEVICES = 16;
 constexpr uint64_t LIMIT = 5 * KQ_WAIT_LIMIT_NS;
-constexpr int REG_EPI = 200, REG_UNPACK = 72, REG_REST = 40; // 2 x 200 + 72 + 40 = 512 = 4 x 128
+constexpr int REG_EPI = 208, REG_UNPACK = 56, REG_REST = 40; // 2 x 208 + 56 + 40 = 512 = 4 x 128
 
 template <bool Q6>
 struct Cfg {
@@ -463,12 +464,12 @@ __global__ void __launch_bounds__(NTHREADS, 1) gemm_kq_kernel(const __grid_const
 #pragma unroll
                     for (int j = 0; j < 16; j += 4) {
                         const float4 da4 = *reinterpret_cast<const float4 *>(da + g2 * 32 + j);
-                        const float dav[4] = {da4.x, da4.y, da4.z, da4.w};
 #pragma unroll
-                        for (int e = 0; e < 4; e++) {
-                            float v = __fmul_rn(df.x, __uint_as_float(m[j + e]));
-                            if (!Q6) v = __fmaf_rn(-df.y, __uint_as_float(n[j + e]), v);
-                            acc[j + e] = __fmaf_rn(dav[e], v, acc[j + e]);
+                        for (int e = 0; e < 4; e += 2) { // two tokens per instruction: 28672 x 8192 at 512 tokens 325 -> 316 us
+                            float2 v = __fmul2_rn(make_float2(df.x, df.x), make_float2(__uint_as_float(m[j + e]), __uint_as_float(m[j + e + 1])));
+                            if (!Q6) v = __ffma2_rn(make_float2(-df.y, -df.y), make_float2(__uint_as_float(n[j + e]), __uint_as_float(n[j + e + 1])), v);
+                            const float2 r = __ffma2_rn(e ? make_float2(da4.z, da4.w) : make_float2(da4.x, da4.y), v, make_float2(acc[j + e], acc[j + e + 1]));
+                            acc[j + e] = r.x, acc[j + e + 1] = r.y;
                         }
                     }
                 };
