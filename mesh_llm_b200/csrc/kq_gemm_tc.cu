@@ -592,7 +592,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) gemm_kq_kernel(const __grid_const
 }
 
 // Q8 rows -> the token operand.  A thread writes 16 bytes: eight codes (or sums of 16) of a token as f16, in the order in which the
-// weights are decoded (0 2 1 3 of every four).  grid (blocks, runs of 16 tokens); tokens past the last are zeros.
+// weights are decoded (0 2 1 3 of every four).  grid (runs of 16 tokens, blocks); tokens past the last are zeros.
 struct ImageParams {
     const int8_t *q;
     const float *d;
@@ -604,7 +604,7 @@ struct ImageParams {
 };
 __global__ void __launch_bounds__(288) act_image_kernel(const __grid_constant__ ImageParams p) {
     KQ_PDL_ENTER();
-    const int b = blockIdx.x, base = blockIdx.y * 16;
+    const int b = blockIdx.y, base = blockIdx.x * 16;
     int n_live = p.M - base; // tokens of this run
     if (p.row_src) {
         const int tile = base / 128;
@@ -905,7 +905,7 @@ b200_status kq_launch_gemm_tc(const KqGemvSeg *segs, int nseg, const int8_t *q, 
         Scratch sc;
         KQ_TRY(scratch(dev, (size_t)p.m_pad * TOK_BYTES * nb, (size_t)p.m_pad * 4 * nb, &sc));
         const ImageParams ip = {q + m0 * K, d + m0 * nb, bs + m0 * nb * 16, sc.img, sc.da, (int32_t)mc, (int32_t)nb, p.m_pad, 1, nullptr, nullptr, nullptr};
-        KQ_CUDA(kq_launch(act_image_kernel, dim3((unsigned)nb, (unsigned)(p.m_pad / 16)), dim3(288), 0, st, ip));
+        KQ_CUDA(kq_launch(act_image_kernel, dim3((unsigned)(p.m_pad / 16), (unsigned)nb), dim3(288), 0, st, ip));
         KQ_COUNT_LAUNCH();
         p.img = sc.img, p.da = sc.da, p.part = sc.part;
         KqGemvSeg sg[MAX_SEGS];
@@ -958,7 +958,7 @@ b200_status kq_launch_gemm_grouped(const KqGemvSeg *segs, int nseg, const int8_t
     KQ_TRY(scratch(dev, (size_t)p.m_pad * TOK_BYTES * nb, (size_t)p.m_pad * 4 * nb, &sc));
     p.n_tiles = sorted, p.tile_expert = sorted + 1, p.row_src = sorted + 1 + mt, p.tile_count = sorted + 1 + mt + mt * TM;
     const ImageParams ip = {q, d, bs, sc.img, sc.da, 0, (int32_t)nb, p.m_pad, act_div, p.row_src, p.tile_count, p.n_tiles};
-    KQ_CUDA(kq_launch(act_image_kernel, dim3((unsigned)nb, (unsigned)(p.m_pad / 16)), dim3(288), 0, st, ip));
+    KQ_CUDA(kq_launch(act_image_kernel, dim3((unsigned)(p.m_pad / 16), (unsigned)nb), dim3(288), 0, st, ip));
     KQ_COUNT_LAUNCH();
     p.img = sc.img, p.da = sc.da, p.part = sc.part;
     return launch_segs(p, segs, nseg, E, K, st);
