@@ -17,7 +17,8 @@
 // Up to three matrices that read the same tokens (q / k / v, gate / up) share the image and, type by type, the launch: the small ones would
 // leave most of the GPU idle (256 x 2048 at 77 tokens: 19 us alone, two of them in the launch of q: none).
 // The (tile, block) pairs are dealt out to the CTAs in equal contiguous shares, so that any number of tiles fills the GPU.  A tile
-// that was cut is added up, in the order of its parts, by the CTA that arrives last; nobody waits.
+// that was cut is added up, in the order of its parts, by the CTA that arrives last, each draining warp its own rows and tokens of the
+// tile; nobody waits, and no barrier stands between a wait that can give up and the end of the kernel.
 //
 // What bounds it, in clocks per block of 128 rows x 256 tokens: the MMAs 2900 (42 each at N = 64, where 32 would be the tensor
 // rate), the drains 1000 of every scheduler, the decoding of Q4_K 870 (alone; of Q6_K twice as much).  Measured about 5500: what is left are
@@ -40,7 +41,7 @@ constexpr int NTHREADS = 512, CHUNK = 64, MAX_CHUNKS = 4, ROWS = 128, TOK_BYTES 
 constexpr int GROUP_BYTES = 8 * TOK_BYTES; // eight tokens: [34 chunks of 16 bytes][8 tokens]
 constexpr int B_BYTES = CHUNK * TOK_BYTES, DA_RING = 8, SC_RING = 8;
 constexpr int TILE_OUT = MAX_CHUNKS * CHUNK * ROWS; // outputs of a tile
-constexpr int MAX_CTAS = 256, MAX_DEVICES = 16;
+constexpr int MAX_CTAS = 256, MAX_DEVICES = 16, DRAIN_WARPS = 8;
 constexpr uint64_t LIMIT = 5 * KQ_WAIT_LIMIT_NS;
 constexpr int REG_EPI = 208, REG_UNPACK = 56, REG_REST = 40; // 2 x 208 + 56 + 40 = 512 = 4 x 128
 
@@ -55,7 +56,9 @@ struct Cfg {
 };
 
 __device__ int g_gemm_error;
-__device__ int g_parts_done[MAX_CTAS]; // parts of a cut tile that have been written, by the CTA that holds its first block; back to zero after use
+// Parts of a cut tile that have been written, by the CTA that holds its first block and the draining warp; one set for each of the two launches
+// (Q4_K, Q6_K) that may read an image, cleared by the launch that writes the image, so that a call which gave up leaves nothing behind.
+__device__ int4 g_parts_done[2 * MAX_CTAS * DRAIN_WARPS / 4];
 
 constexpr int MAX_SEGS = 3;
 struct Seg { // one of the matrices that share the tokens
@@ -159,7 +162,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) gemm_kq_kernel(const __grid_const
     __shared__ uint64_t raw_full[C::RAW_STAGES], raw_empty[C::RAW_STAGES], b_full[C::B_STAGES], b_empty[C::B_STAGES];
     __shared__ uint64_t da_full[DA_RING], sc_full[SC_RING], a_full[2], a_empty[2], acc_full[2], acc_empty[2], s_end[2];
     __shared__ uint32_t s_tmem;
-    __shared__ int s_abort, s_last;
+    __shared__ int s_abort;
     KQ_PDL_TRIGGER();
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     if (tid == 0) {
@@ -548,15 +551,11 @@ __global__ void __launch_bounds__(NTHREADS, 1) gemm_kq_kernel(const __grid_const
                 }
                 if (!whole) {
                     __threadfence();
-                    asm volatile("bar.sync 1, 256;" ::: "memory");
-                    if (tid == 0) {
-                        const int before = atomicAdd(&g_parts_done[c0], 1);
-                        s_last = before == (int)(c1 - c0);
-                        if (before == (int)(c1 - c0)) g_parts_done[c0] = 0;
-                        __threadfence();
-                    }
-                    asm volatile("bar.sync 1, 256;" ::: "memory");
-                    if (s_last) {
+                    __syncwarp();
+                    int before = 0;
+                    if (lane == 0) before = atomicAdd(reinterpret_cast<int *>(g_parts_done) + ((Q6 ? MAX_CTAS : 0) + c0) * DRAIN_WARPS + warp, 1);
+                    before = __shfl_sync(0xffffffffu, before, 0);
+                    if (before == (int)(c1 - c0)) { // this warp's part of the tile is complete
                         __threadfence();
 #pragma unroll 1
                         for (int i = 0; i < 8; i++) {
@@ -592,7 +591,8 @@ __global__ void __launch_bounds__(NTHREADS, 1) gemm_kq_kernel(const __grid_const
 }
 
 // Q8 rows -> the token operand.  A thread writes 16 bytes: eight codes (or sums of 16) of a token as f16, in the order in which the
-// weights are decoded (0 2 1 3 of every four).  grid (runs of 16 tokens, blocks); tokens past the last are zeros.
+// weights are decoded (0 2 1 3 of every four).  grid (runs of 16 tokens, blocks); tokens past the last are zeros.  The first CTA clears the
+// counters of cut tiles for the products that read this image.
 struct ImageParams {
     const int8_t *q;
     const float *d;
@@ -604,6 +604,8 @@ struct ImageParams {
 };
 __global__ void __launch_bounds__(288) act_image_kernel(const __grid_constant__ ImageParams p) {
     KQ_PDL_ENTER();
+    if (blockIdx.x == 0 && blockIdx.y == 0)
+        for (int i = threadIdx.x; i < 2 * MAX_CTAS * DRAIN_WARPS / 4; i += blockDim.x) g_parts_done[i] = make_int4(0, 0, 0, 0);
     const int b = blockIdx.y, base = blockIdx.x * 16;
     int n_live = p.M - base; // tokens of this run
     if (p.row_src) {
@@ -876,11 +878,7 @@ b200_status check_segs(const KqGemvSeg *segs, int nseg, const int8_t *q, int64_t
 int kq_gemm_error_fetch() {
     int v = 0, zero = 0;
     if (cudaMemcpyFromSymbol(&v, g_gemm_error, sizeof(int)) != cudaSuccess) return -1;
-    if (v) {
-        static const int none[MAX_CTAS] = {};
-        cudaMemcpyToSymbol(g_gemm_error, &zero, sizeof(int));
-        cudaMemcpyToSymbol(g_parts_done, none, sizeof(none));
-    }
+    if (v) cudaMemcpyToSymbol(g_gemm_error, &zero, sizeof(int));
     return v;
 }
 
