@@ -53,6 +53,9 @@ struct Cfg {
                          SM_DA = SM_AMIN + (Q6 ? 0 : 2 * 4096), SM_SC = SM_DA + DA_RING * CHUNK * 4, SMEM = SM_SC + SC_RING * ROWS * 4;
     static_assert(SM_RAW % 128 == 0 && RAW_BYTES % 128 == 0 && SM_AMIN % 16 == 0, "TMA destinations are 128-byte aligned");
     static_assert(SMEM <= 226 * 1024, "shared memory of a CTA");
+    // chunk q - 2 has been drained when chunk q is issued, and a stage is filled again when its chunk's MMAs are over: what the rings without
+    // barriers of their own rely on
+    static_assert(B_STAGES >= 3 && DA_RING >= B_STAGES + 2 && SC_RING >= 4, "rings");
 };
 
 __device__ int g_gemm_error;
@@ -264,6 +267,9 @@ __global__ void __launch_bounds__(NTHREADS, 1) gemm_kq_kernel(const __grid_const
                     // decoded weights, tokens, the accumulator (free from the start)
                     const uint32_t bar = smem_u32(lane == 0 ? &a_full[sa] : lane == 1 ? &b_full[s] : &acc_empty[w]);
                     const uint32_t par = lane == 0 ? pa : lane == 1 ? (q / C::B_STAGES) & 1 : (q / 2 - 1) & 1;
+                    // With an odd number of token stages a warp waits for every second phase of b_full[s] only, all of one parity, and would take
+                    // the one before last for its own.  The phase between is over once chunk q - 2 has been drained: wait for that first.
+                    if (C::B_STAGES % 2 && q >= 2 && !(ok = wait(&acc_empty[w], (q / 2 - 1) & 1, 3))) break;
                     if (!(ok = wait_on(bar, par, lane, q < 2 ? 2 : 3, &s_abort, 3))) break;
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                     const uint64_t bd = nosw_desc(smem_u32(smem + C::SM_B + s * B_BYTES), 128, GROUP_BYTES);

@@ -2,6 +2,8 @@
 import os
 import re
 
+import pytest
+
 SRC = os.path.join(os.path.dirname(__file__), "..", "mesh_llm_b200", "csrc", "kq_gemm_tc.cu")
 
 
@@ -25,3 +27,51 @@ def test_no_barrier_that_a_warp_can_miss_by_giving_up():
     assert not re.search(r"\bbar\.sync\b|barrier\.sync|__syncthreads_|named_barrier", roles)
     drain = roles[roles.index("setmaxnreg.inc"):roles.index("__syncthreads")]
     assert drain.index("if (!ok) break;") < drain.index("atomicAdd")
+
+
+def constants(q6):
+    """the sizes of the rings of one instance"""
+    s = source()
+    v = dict(re.findall(r"\b(DA_RING|SC_RING) = (\d+)", s))
+    for name in ("RAW_STAGES", "B_STAGES"):
+        a, b = re.search(name + r" = Q6 \? (\d+) : (\d+)", s).groups()
+        v[name] = a if q6 else b
+    return {k: int(n) for k, n in v.items()}
+
+
+def drained_when_issued(q):
+    """the last chunk that is known to be drained when the MMAs of chunk q are issued (they wait for its accumulator)"""
+    return q - 2
+
+
+@pytest.mark.parametrize("q6", [False, True], ids=["q4_k", "q6_k"])
+@pytest.mark.parametrize("chunks", [1, 2, 3, 4])
+def test_waits_by_parity_are_unambiguous(q6, chunks):
+    """a wait by parity for phase n of a barrier is right only if phase n - 1 is known to be over: the waiting warp has waited for it, or for
+    something that comes behind it, before it tries.  Walks the waits of the two issuing warps on the token stages"""
+    c, body = constants(q6), kernel_body()
+    acc_first = c["B_STAGES"] % 2 == 0 or "C::B_STAGES % 2 && q >= 2 && !(ok = wait(&acc_empty[w]" in body
+    for w in (0, 1):
+        seen = {}
+        for q in range(w, 64 * chunks, 2):  # a warp issues every second chunk of the whole walk, whatever the blocks
+            s, phase = q % c["B_STAGES"], q // c["B_STAGES"]
+            known = seen.get(s, -1)
+            if acc_first and q >= 2:  # every chunk up to q - 2 has been drained, so it had been loaded
+                d = drained_when_issued(q)
+                known = max(known, max((p // c["B_STAGES"] for p in range(d + 1) if p % c["B_STAGES"] == s), default=-1))
+            assert known >= phase - 1
+            seen[s] = phase
+
+
+@pytest.mark.parametrize("q6", [False, True], ids=["q4_k", "q6_k"])
+@pytest.mark.parametrize("chunks", [1, 2, 3, 4])
+def test_rings_without_an_empty_barrier(q6, chunks):
+    """the scales of tokens and of weight blocks are overwritten only when their last reader is known to be through"""
+    c = constants(q6)
+    for q in range(200):
+        # token scales of chunk q are requested when the MMAs of chunk q - B_STAGES are over: then their place's former chunk is drained
+        assert q - c["DA_RING"] <= drained_when_issued(q - c["B_STAGES"])
+        # scales of block u are written when the MMAs of block u - 2 are over
+        u = q
+        last = (u - 2) * chunks + chunks - 1  # its last chunk
+        assert (u - c["SC_RING"]) * chunks + chunks - 1 <= drained_when_issued(last)
