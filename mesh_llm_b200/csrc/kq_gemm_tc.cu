@@ -1,16 +1,17 @@
 // Products of more than a few tokens with K-quant weights on the 5th-generation tensor cores:
 // y[m][n] = sum_k W[n][k] x[m][k], W in Q4_K / Q6_K blocks, x in Q8 blocks of 256.
 //
-// The integer scale of a sub-block is folded into the weight: w' = sc_j q is at most 945 (Q4_K), exact in f16, and so is a
-// Q8 code, so one tcgen05.mma of kind::f16 per 16 elements adds up  sum_j sc_j sum_i q_ij a_ij  of a 256-element block in f32,
-// exactly while it stays below 2^24.  Q6_K's w' = sc (q - 32) has 13 bits: it goes in as two addends, (sc & ~7)(q - 32) and
-// (sc & 7)(q - 32), both exact in f16, into the same accumulator.  The Q4_K min term sum_j m_j bsum_j is one more MMA (K = 16)
-// into an accumulator of its own.  Per block an output then takes y += d_a (d_w main - d_min min) in f32.
+// The integer scale of a sub-block is folded into the weight, and the products of a 256-element block are added up as integers.
+// Q4_K: w' = sc_j q is at most 945, exact in f16, and so is a Q8 code, so one tcgen05.mma of kind::f16 per 16 elements adds up
+// sum_j sc_j sum_i q_ij a_ij  in f32, exactly while it stays below 2^24.  The min term sum_j m_j bsum_j is one more MMA (K = 16) into an
+// accumulator of its own.  Per block an output then takes y += d_a (d_w main - d_min min) in f32.
+// Q6_K: w' = sc (q - 32) has 14 bits with its sign, w' = 64 hi + lo with |hi| <= 64 and 0 <= lo < 64.  Both are bytes, and two tcgen05.mma of
+// kind::i8 per 32 elements, each into an int32 accumulator of its own, give the sum of the block whatever its size; it is rounded once, to f32.
 //
 // A tile is 128 weight rows x up to 256 tokens.  Weight rows are the M of the MMA (TMEM lanes), tokens its N in chunks of
-// up to 64.  Packed blocks arrive by TMA; a warpgroup (a thread per row) decodes them into TMEM, from where the MMAs take
-// them as their A operand, so that decoded weights never pass through shared memory.  The token operand is an image that
-// act_image_kernel writes: one bulk copy per chunk and block.  Two warps issue MMAs in turn, each with an accumulator of its own;
+// up to 64.  Packed blocks arrive by TMA; a warpgroup (a thread per row) decodes them into TMEM, two bytes per weight in both types, from where
+// the MMAs take them as their A operand, so that decoded weights never pass through shared memory.  The token operand is an image that
+// act_image_kernel writes (f16 codes and sums of 16 for Q4_K, the codes themselves for Q6_K): one bulk copy per chunk and block.  Two warps issue MMAs in turn, each with an accumulator of its own;
 // two warpgroups drain the accumulators into the running f32 result, which stays in registers for the whole tile.  Lanes of a
 // warp hold neighbouring rows of W, so results leave in full lines.
 //
@@ -20,12 +21,13 @@
 // that was cut is added up, in the order of its parts, by the CTA that arrives last, each draining warp its own rows and tokens of the
 // tile; nobody waits, and no barrier stands between a wait that can give up and the end of the kernel.
 //
-// What bounds it, in clocks per block of 128 rows x 256 tokens: the MMAs 2900 (42 each at N = 64, where 32 would be the tensor
-// rate), the drains 1000 of every scheduler, the decoding of Q4_K 870 (alone; of Q6_K twice as much).  Measured about 5500: what is left are
-// the hand-overs between the roles, of which each accumulator has two per chunk, and instruction fetch: four roles run four loops, and
-// the same decoding unrolled four times made the whole kernel 10 % slower.  Two int8 planes per weight instead (the form
-// before this one) had to turn three accumulators per output from integers into floats: 1659 us against 1200 for 2048 tokens x 28672 x 8192
-// in Q4_K (580 -> 800 TFLOP/s), 547 against 312 at 512 tokens, 169 against 68 at 16; Q6_K at 64 tokens 254 against 151 us.
+// What bounds it, in clocks per block of 128 rows x 256 tokens: the MMAs 2900 in either type (42 each at N = 64, where 32 would be the tensor
+// rate), the drains about 1000 of every scheduler.  Measured about 5500 for 256 tokens and 2600 (Q4_K) or 4000 (Q6_K) for 16, where the decoding is
+// what is left: one warp of each scheduler walks through it.  The same decoding unrolled four times made the whole kernel 10 % slower.
+// Q4_K: two int8 planes per weight out of shared memory (the form before this one) took 1659 us where this takes 1240, for 2048 tokens x 28672 x
+// 8192, 547 against 315 at 512 tokens, 169 against 66 at 16.  Q6_K, whose two planes came from shared memory as well: 1637 against 1324,
+// 624 against 351, 248 against 110; as two f16 addends into one f32 accumulator, with the decoded operand in a single buffer, it
+// took 2125, 512 and 155, and was exact only below 2^24.
 // Every wait is bounded; on a time-out the kernel records an error, lets its copies and MMAs end, frees its TMEM and returns.
 #include "kq_tc.cuh"
 
@@ -37,9 +39,9 @@
 
 namespace {
 
-constexpr int NTHREADS = 512, CHUNK = 64, MAX_CHUNKS = 4, ROWS = 128, TOK_BYTES = 544; // bytes of a token in an image: 256 f16 codes, 16 f16 sums
-constexpr int GROUP_BYTES = 8 * TOK_BYTES; // eight tokens: [34 chunks of 16 bytes][8 tokens]
-constexpr int B_BYTES = CHUNK * TOK_BYTES, DA_RING = 8, SC_RING = 8;
+constexpr int NTHREADS = 512, CHUNK = 64, MAX_CHUNKS = 4, ROWS = 128, DA_RING = 8, SC_RING = 8;
+// bytes of a token and block in an image: 256 f16 codes and 16 f16 sums (Q4_K), or 256 codes (Q6_K); eight tokens are [chunks of 16 bytes][8 tokens]
+constexpr int TOK16 = 544, TOK8 = 256;
 constexpr int TILE_OUT = MAX_CHUNKS * CHUNK * ROWS; // outputs of a tile
 constexpr int MAX_CTAS = 256, MAX_DEVICES = 16, DRAIN_WARPS = 8;
 constexpr uint64_t LIMIT = 5 * KQ_WAIT_LIMIT_NS;
@@ -48,14 +50,17 @@ constexpr int REG_EPI = 208, REG_UNPACK = 56, REG_REST = 40; // 2 x 208 + 56 + 4
 template <bool Q6>
 struct Cfg {
     static constexpr int RAW_BYTES = Q6 ? 13 * ROWS * 32 : ROWS * KQ_Q4K_BYTES; // Q6_K: two blocks of each row
-    static constexpr int RAW_STAGES = Q6 ? 2 : 4, B_STAGES = Q6 ? 3 : 4;
+    static constexpr int TOK_BYTES = Q6 ? TOK8 : TOK16, B_BYTES = CHUNK * TOK_BYTES;
+    static constexpr int RAW_STAGES = Q6 ? 2 : 4, B_STAGES = Q6 ? 6 : 4;
     static constexpr int SM_B = 0, SM_RAW = B_STAGES * B_BYTES, SM_AMIN = SM_RAW + RAW_STAGES * RAW_BYTES,
                          SM_DA = SM_AMIN + (Q6 ? 0 : 2 * 4096), SM_SC = SM_DA + DA_RING * CHUNK * 4, SMEM = SM_SC + SC_RING * ROWS * 4;
     static_assert(SM_RAW % 128 == 0 && RAW_BYTES % 128 == 0 && SM_AMIN % 16 == 0, "TMA destinations are 128-byte aligned");
     static_assert(SMEM <= 226 * 1024, "shared memory of a CTA");
+    // the two issuing warps take alternate chunks: with an even number a stage is always the same warp's, which then waits for every phase of it
+    static_assert(B_STAGES % 2 == 0, "a wait by parity must not miss a phase");
     // chunk q - 2 has been drained when chunk q is issued, and a stage is filled again when its chunk's MMAs are over: what the rings without
     // barriers of their own rely on
-    static_assert(B_STAGES >= 3 && DA_RING >= B_STAGES + 2 && SC_RING >= 4, "rings");
+    static_assert(DA_RING >= B_STAGES + 2 && SC_RING >= 4, "rings");
 };
 
 __device__ int g_gemm_error;
@@ -73,7 +78,7 @@ struct Seg { // one of the matrices that share the tokens
 struct Params {
     CUtensorMap w[2 * MAX_SEGS]; // packed blocks; Q6_K: rows' full groups of eight blocks, then their last, smaller group
     Seg seg[MAX_SEGS];
-    const uint8_t *img;    // token images [block][8 tokens][GROUP_BYTES]
+    const uint8_t *img;    // token images [block][groups of 8 tokens]
     const float *da;       // activation scales [block][m_pad]
     float *part;
     const float *residual; // with one matrix only
@@ -115,11 +120,20 @@ __device__ __forceinline__ uint32_t u2(__half2 v) { return *reinterpret_cast<uin
 // byte b of v as an f16 pair, 1024 + byte in both halves
 __device__ __forceinline__ __half2 byte_pair(uint32_t v, int b) { return h2(__byte_perm(v, 0x64646464u, 0x4040u | (b << 8) | b)); }
 
-#define TMEM_ST8(taddr, r)                                                                              \
-    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};"                \
-                 :                                                                                      \
-                 : "r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]) \
-                 : "memory")
+#define TMEM_ST4(taddr, r) \
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x4.b32 [%0], {%1,%2,%3,%4};" ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]) : "memory")
+
+// kind::i8, A in TMEM (four elements to a column), s32 accumulators, B signed
+__device__ __forceinline__ constexpr uint32_t idesc_i8(int m, int n, bool a_signed) {
+    return (2u << 4) | ((a_signed ? 1u : 0u) << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24);
+}
+__device__ __forceinline__ void mma_i8_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b, uint32_t id, uint32_t acc) {
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+                 "tcgen05.mma.cta_group::1.kind::i8 [%0], [%1], %2, %3, p;\n\t}"
+                 :
+                 : "r"(d_tmem), "r"(a_tmem), "l"(b), "r"(id), "r"(acc)
+                 : "memory");
+}
 
 __device__ __forceinline__ void bar_init(uint64_t *b, int count) { asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(b)), "r"(count)); }
 __device__ __forceinline__ void bar_arrive(uint64_t *b) { asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(b)) : "memory"); }
@@ -234,15 +248,15 @@ __global__ void __launch_bounds__(NTHREADS, 1) gemm_kq_kernel(const __grid_const
             if (!ok && lead) // copies that were posted must land before the CTA goes away
                 for (int i = max(0, k - C::RAW_STAGES); i < k; i++) kq_mbar_wait(smem_u32(&raw_full[i % C::RAW_STAGES]), (i / C::RAW_STAGES) & 1, KQ_WAIT_LIMIT_NS);
         } else if (warp == 13) { // token images and scales
-            const int64_t block_bytes = (int64_t)p.m_pad * TOK_BYTES;
+            const int64_t block_bytes = (int64_t)p.m_pad * C::TOK_BYTES;
             for (int u = 0; u < total && ok; u++) {
                 for (int c = 0; c < t.c; c++, k++) {
                     const int s = k % C::B_STAGES, round = k / C::B_STAGES;
                     if (round > 0 && !(ok = wait(&b_empty[s], (round - 1) & 1, 2))) break;
                     if (lead) {
                         const int tok = t.t0 + c * t.cw, d = k % DA_RING;
-                        bar_expect(&b_full[s], t.cw * TOK_BYTES);
-                        bulk_in(smem_u32(smem + C::SM_B + s * B_BYTES), p.img + b * block_bytes + (int64_t)tok * TOK_BYTES, t.cw * TOK_BYTES, &b_full[s]);
+                        bar_expect(&b_full[s], t.cw * C::TOK_BYTES);
+                        bulk_in(smem_u32(smem + C::SM_B + s * C::B_BYTES), p.img + b * block_bytes + (int64_t)tok * C::TOK_BYTES, t.cw * C::TOK_BYTES, &b_full[s]);
                         bar_expect(&da_full[d], t.cw * 4);
                         bulk_in(smem_u32(smem + C::SM_DA + d * CHUNK * 4), p.da + (int64_t)b * p.m_pad + tok, t.cw * 4, &da_full[d]);
                     }
@@ -261,39 +275,29 @@ __global__ void __launch_bounds__(NTHREADS, 1) gemm_kq_kernel(const __grid_const
         } else { // MMAs: one warp waits while the other one issues
             const int w = warp & 1;
             for (int u = 0; u < total && ok; u++) {
-                const uint32_t id = tc_idesc(128, t.cw, false, false), sa = Q6 ? 0 : u & 1, pa = Q6 ? u & 1 : (u >> 1) & 1;
+                const uint32_t id = Q6 ? idesc_i8(128, t.cw, true) : tc_idesc(128, t.cw, false, false), sa = u & 1, pa = (u >> 1) & 1;
                 for (int c = (k & 1) ^ w; c < t.c; c += 2) {
                     const int q = k + c, s = q % C::B_STAGES;
                     // decoded weights, tokens, the accumulator (free from the start)
                     const uint32_t bar = smem_u32(lane == 0 ? &a_full[sa] : lane == 1 ? &b_full[s] : &acc_empty[w]);
                     const uint32_t par = lane == 0 ? pa : lane == 1 ? (q / C::B_STAGES) & 1 : (q / 2 - 1) & 1;
-                    // With an odd number of token stages a warp waits for every second phase of b_full[s] only, all of one parity, and would take
-                    // the one before last for its own.  The phase between is over once chunk q - 2 has been drained: wait for that first.
-                    if (C::B_STAGES % 2 && q >= 2 && !(ok = wait(&acc_empty[w], (q / 2 - 1) & 1, 3))) break;
                     if (!(ok = wait_on(bar, par, lane, q < 2 ? 2 : 3, &s_abort, 3))) break;
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                    const uint64_t bd = nosw_desc(smem_u32(smem + C::SM_B + s * B_BYTES), 128, GROUP_BYTES);
+                    const uint64_t bd = nosw_desc(smem_u32(smem + C::SM_B + s * C::B_BYTES), 128, 8 * C::TOK_BYTES);
                     const uint32_t acc = tmem + 256 + w * 2 * CHUNK, a = tmem + sa * 128;
                     const bool last = c + 2 >= t.c; // this warp's last use of the decoded weights
-                    if (Q6) { // by halves of the block, each with its two addends
-#pragma unroll
-                        for (int h = 0; h < 2; h++) {
-                            if (h && !(ok = wait(&a_full[1], pa, 3))) break;
-                            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                            if (lead) {
+                    if (lead) {
+                        if (Q6) {
 #pragma unroll 4
-                                for (int i = 0; i < 8; i++) tc_mma_ts(acc, a + h * 128 + i * 8, bd + h * 128 + i * 16, id, h + i > 0);
+                            for (int i = 0; i < 8; i++) mma_i8_ts(acc, a + i * 8, bd + i * 16, id, i > 0);
+                            const uint32_t id_lo = idesc_i8(128, t.cw, false);
 #pragma unroll 4
-                                for (int i = 0; i < 8; i++) tc_mma_ts(acc, a + h * 128 + 64 + i * 8, bd + h * 128 + i * 16, id, 1);
-                                if (last) tc_commit(smem_u32(&a_empty[h]));
-                            }
-                            __syncwarp();
+                            for (int i = 0; i < 8; i++) mma_i8_ts(acc + CHUNK, a + 64 + i * 8, bd + i * 16, id_lo, i > 0);
+                        } else {
+#pragma unroll 4
+                            for (int i = 0; i < 16; i++) tc_mma_ts(acc, a + i * 8, bd + i * 16, id, i > 0);
+                            tc_mma_ss(acc + CHUNK, nosw_desc(smem_u32(smem + C::SM_AMIN + sa * 4096), 2048, 128), bd + 256, id, 0);
                         }
-                        if (!ok) break;
-                    } else if (lead) {
-#pragma unroll 4
-                        for (int i = 0; i < 16; i++) tc_mma_ts(acc, a + i * 8, bd + i * 16, id, i > 0);
-                        tc_mma_ss(acc + CHUNK, nosw_desc(smem_u32(smem + C::SM_AMIN + sa * 4096), 2048, 128), bd + 256, id, 0);
                         if (last) tc_commit(smem_u32(&a_empty[sa]));
                     }
                     if (lead) {
@@ -303,11 +307,8 @@ __global__ void __launch_bounds__(NTHREADS, 1) gemm_kq_kernel(const __grid_const
                     __syncwarp();
                 }
                 if (ok && ((k & 1) ^ w) >= t.c) { // no chunk of this block for this warp; it still sees every phase of a_full, and arrives once per phase of a_empty
-                    ok = wait(&a_full[sa], pa, 3) && (!Q6 || wait(&a_full[1], pa, 3));
-                    if (ok && lead) {
-                        bar_arrive(&a_empty[sa]);
-                        if (Q6) bar_arrive(&a_empty[1]);
-                    }
+                    ok = wait(&a_full[sa], pa, 3);
+                    if (ok && lead) bar_arrive(&a_empty[sa]);
                 }
                 __syncwarp();
                 k += t.c;
@@ -378,8 +379,8 @@ __global__ void __launch_bounds__(NTHREADS, 1) gemm_kq_kernel(const __grid_const
             int tile = tile0, b = b0, k = -1;
             uint4 dv = make_uint4(0, 0, 0, 0); // block scales of the row's group of eight blocks
             const uint8_t *wr = nullptr;
-            bool ok = true;
-            for (int u = 0; u < total && ok; u++) {
+            for (int u = 0; u < total; u++) {
+                const int sa = u & 1;
                 if (u == 0 || b == 0) {
                     const TilePos t = tile_at(p, tile);
                     const int n = seg_rows(p, t.seg);
@@ -389,8 +390,10 @@ __global__ void __launch_bounds__(NTHREADS, 1) gemm_kq_kernel(const __grid_const
                     dv = __ldg(reinterpret_cast<const uint4 *>(wr + kq_q6_addr(nb, b / KQ_Q6_GROUP * KQ_Q6_GROUP).d));
                 if (u == 0 || b % 2 == 0) {
                     k++;
-                    if (!(ok = wait(&raw_full[k % C::RAW_STAGES], (k / C::RAW_STAGES) & 1, 6))) break;
+                    if (!wait(&raw_full[k % C::RAW_STAGES], (k / C::RAW_STAGES) & 1, 6)) break;
                 }
+                if (u >= 2 && !wait(&a_empty[sa], ((u >> 1) - 1) & 1, 7)) break;
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const int s = k % C::RAW_STAGES;
                 const uint8_t *blk = smem + C::SM_RAW + s * C::RAW_BYTES + row * 32 + (b & 1) * 16; // chunk i of the block 4096 i further
                 const uint4 sc4 = *reinterpret_cast<const uint4 *>(blk + 12 * 4096);
@@ -398,9 +401,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) gemm_kq_kernel(const __grid_const
                 const uint32_t dw = b8 < 2 ? dv.x : b8 < 4 ? dv.y : b8 < 6 ? dv.z : dv.w;
                 *reinterpret_cast<uint32_t *>(smem + C::SM_SC + ((u % SC_RING) * ROWS + row) * 4) = (b8 & 1 ? dw >> 16 : dw) & 0xFFFFu;
 #pragma unroll 1
-                for (int hh = 0; hh < 2; hh++) { // 128 elements: 64 columns with the multiples of eight of the scales, 64 with the rest
-                    if (u > 0 && !(ok = wait(&a_empty[hh], (u - 1) & 1, 7))) break;
-                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                for (int hh = 0; hh < 2; hh++) { // 128 elements
                     const uint32_t sc_a = hh ? sc4.z : sc4.x, sc_b = hh ? sc4.w : sc4.y;
 #pragma unroll 1
                     for (int h = 0; h < 2; h++) { // elements 128 hh + 32 q + 16 h + ..
@@ -409,33 +410,31 @@ __global__ void __launch_bounds__(NTHREADS, 1) gemm_kq_kernel(const __grid_const
                         const uint32_t a[4] = {a4.x, a4.y, a4.z, a4.w}, c[4] = {c4.x, c4.y, c4.z, c4.w}, qh[4] = {q4.x, q4.y, q4.z, q4.w};
 #pragma unroll
                         for (int q = 0; q < 4; q++) { // 16 elements: scale group 8 hh + 2 q + h
-                            const uint32_t sw = (q < 2 ? sc_a : sc_b) >> (8 * h);
-                            const __half2 hi = __hsub2(byte_pair((sw ^ 0x80808080u) & 0xF8F8F8F8u, (2 * q) & 3), __float2half2_rn(1152.f)),
-                                          lo = __hsub2(byte_pair(sw & 0x07070707u, (2 * q) & 3), __float2half2_rn(1024.f));
-                            const __half2 hi96 = __hmul2(hi, __float2half2_rn(-96.f)), lo96 = __hmul2(lo, __float2half2_rn(-96.f));
-                            uint32_t o[8], r[8];
+                            // Two codes to a register, 16 bits each: 4 (sc (q - 32) + 8192) is between 16384 and 49152, so neither half reaches into the
+                            // other.  Its upper byte is hi + 128, its lower one 4 lo.
+                            const int sc = (int)((q < 2 ? sc_a : sc_b) << (24 - 8 * ((2 * q) & 3) - 8 * h)) >> 24;
+                            const uint32_t k4 = 4u * (uint32_t)sc, base = 0x80008000u - 0x00800080u * (uint32_t)sc;
+                            uint32_t hi[4], lo[4];
 #pragma unroll
                             for (int i = 0; i < 4; i++) {
-                                // the code in bits 4..9 of an f16 in [64, 128): 64 + code; (64 + code) sc - 96 sc rounds an exact result
-                                const uint32_t n = q & 1 ? c[i] : a[i], ne = q & 2 ? n : n << 4, no = q & 2 ? n >> 8 : n >> 4;
-                                const uint32_t he = q == 0 ? qh[i] << 8 : q == 1 ? qh[i] << 6 : q == 2 ? qh[i] << 4 : qh[i] << 2;
-                                const uint32_t ho = q == 0 ? qh[i] : q == 1 ? qh[i] >> 2 : q == 2 ? qh[i] >> 4 : qh[i] >> 6;
-                                const __half2 ve = h2(((ne & 0x00F000F0u) | 0x54005400u) | (he & 0x03000300u)), vo = h2(((no & 0x00F000F0u) | 0x54005400u) | (ho & 0x03000300u));
-                                o[2 * i] = u2(__hfma2(ve, hi, hi96)), o[2 * i + 1] = u2(__hfma2(vo, hi, hi96));
-                                r[2 * i] = u2(__hfma2(ve, lo, lo96)), r[2 * i + 1] = u2(__hfma2(vo, lo, lo96));
+                                const uint32_t n = q & 1 ? c[i] : a[i], top = q == 0 ? qh[i] << 4 : q == 1 ? qh[i] << 2 : q == 2 ? qh[i] : qh[i] >> 2;
+                                const uint32_t code = ((q & 2 ? n >> 4 : n) & 0x0F0F0F0Fu) | (top & 0x30303030u);
+                                const uint32_t even = (code & 0x00FF00FFu) * k4 + base, odd = ((code >> 8) & 0x00FF00FFu) * k4 + base;
+                                hi[i] = __byte_perm(even, odd, 0x7351) ^ 0x80808080u;
+                                lo[i] = __byte_perm(even, odd, 0x6240);
                             }
-                            TMEM_ST8(tl + hh * 128 + (2 * q + h) * 8, o);
-                            TMEM_ST8(tl + hh * 128 + 64 + (2 * q + h) * 8, r);
+                            const uint32_t at = tl + sa * 128 + 32 * hh + 8 * q + 4 * h;
+                            TMEM_ST4(at, hi);
+                            TMEM_ST4(at + 64, lo);
                         }
                     }
-                    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-                    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-                    __syncwarp();
-                    if (lane == 0) {
-                        bar_arrive(&a_full[hh]);
-                        if (hh) bar_arrive(&sc_full[u % SC_RING]);
-                        if (hh && (b % 2 == 1 || b == nb - 1)) bar_arrive(&raw_empty[s]);
-                    }
+                }
+                asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+                asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                __syncwarp();
+                if (lane == 0) {
+                    bar_arrive(&a_full[sa]), bar_arrive(&sc_full[u % SC_RING]);
+                    if (b % 2 == 1 || b == nb - 1) bar_arrive(&raw_empty[s]);
                 }
                 if (++b == nb) b = 0, tile++;
             }
@@ -461,21 +460,24 @@ __global__ void __launch_bounds__(NTHREADS, 1) gemm_kq_kernel(const __grid_const
                 if (!(ok = wait_on(bar, lane == 0 ? (q >> 1) & 1 : lane == 1 ? (q / DA_RING) & 1 : (u / SC_RING) & 1, lane, 3, &s_abort, 9))) continue;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const uint32_t dd = *reinterpret_cast<const uint32_t *>(smem + C::SM_SC + (ks * ROWS + row) * 4);
-                const float2 df = __half22float2(h2(dd)); // d_w, d_min
+                float2 df = __half22float2(h2(dd)); // d_w, d_min
+                if (Q6) df.x *= 0.25f; // the sums come four times
                 const float *da = reinterpret_cast<const float *>(smem + C::SM_DA + kd * CHUNK * 4) + wg * 16;
                 const uint32_t ta = tl + slot * 2 * CHUNK + wg * 16;
-                auto add16 = [&](float (&acc)[16], int g2) { // acc += d_a (d_w main - d_min min)
+                auto add16 = [&](float (&acc)[16], int g2) { // acc += d_a (d_w main - d_min min), or d_a d_w (64 hi + lo)
                     if ((2 * g2 + wg) * 16 >= t.cw) return;
                     uint32_t m[16], n[16];
                     TMEM_LD16(ta + g2 * 32, m);
-                    if (!Q6) TMEM_LD16(ta + g2 * 32 + CHUNK, n);
+                    TMEM_LD16(ta + g2 * 32 + CHUNK, n);
                     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
                     for (int j = 0; j < 16; j += 4) {
                         const float4 da4 = *reinterpret_cast<const float4 *>(da + g2 * 32 + j);
 #pragma unroll
                         for (int e = 0; e < 4; e += 2) { // two tokens per instruction: 28672 x 8192 at 512 tokens 325 -> 316 us
-                            float2 v = __fmul2_rn(make_float2(df.x, df.x), make_float2(__uint_as_float(m[j + e]), __uint_as_float(m[j + e + 1])));
+                            const float2 main = Q6 ? make_float2(__int2float_rn((int)(m[j + e] * 256u + n[j + e])), __int2float_rn((int)(m[j + e + 1] * 256u + n[j + e + 1])))
+                                                   : make_float2(__uint_as_float(m[j + e]), __uint_as_float(m[j + e + 1]));
+                            float2 v = __fmul2_rn(make_float2(df.x, df.x), main);
                             if (!Q6) v = __ffma2_rn(make_float2(-df.y, -df.y), make_float2(__uint_as_float(n[j + e]), __uint_as_float(n[j + e + 1])), v);
                             const float2 r = __ffma2_rn(e ? make_float2(da4.z, da4.w) : make_float2(da4.x, da4.y), v, make_float2(acc[j + e], acc[j + e + 1]));
                             acc[j + e] = r.x, acc[j + e + 1] = r.y;
@@ -596,14 +598,14 @@ __global__ void __launch_bounds__(NTHREADS, 1) gemm_kq_kernel(const __grid_const
     if (warp == 15) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512) : "memory");
 }
 
-// Q8 rows -> the token operand.  A thread writes 16 bytes: eight codes (or sums of 16) of a token as f16, in the order in which the
-// weights are decoded (0 2 1 3 of every four).  grid (runs of 16 tokens, blocks); tokens past the last are zeros.  The first CTA clears the
-// counters of cut tiles for the products that read this image.
+// Q8 rows -> the token operand, in the forms that the call's matrices read.  A thread writes 16 bytes of a token: eight codes (or sums of 16) as
+// f16, in the order in which Q4_K weights are decoded (0 2 1 3 of every four), or 16 codes.  grid (runs of 16 tokens, blocks); tokens past
+// the last are zeros.  The first CTA clears the counters of cut tiles for the products that read this image.
 struct ImageParams {
     const int8_t *q;
     const float *d;
     const int16_t *bs;
-    uint8_t *img;
+    uint8_t *img16, *img8; // null: not wanted
     float *da;
     int32_t M, nb, m_pad, act_div;
     const int32_t *row_src, *tile_count, *n_tiles; // products with experts
@@ -624,31 +626,40 @@ __global__ void __launch_bounds__(288) act_image_kernel(const __grid_constant__ 
         n_live = n - (base - tile * 128);
     }
     const __half2 k1152 = __float2half2_rn(1152.f);
-    for (int i = threadIdx.x; i < 2 * 34 * 8; i += blockDim.x) {
-        const int r = i & 7, kc = (i >> 3) % 34, g = i / 272, at = g * 8 + r; // token at of the run
-        const bool in = at < n_live;
-        int m = 0;
-        if (in) m = p.row_src ? p.row_src[base + at] / p.act_div : base + at;
-        uint4 o = make_uint4(0, 0, 0, 0);
-        if (kc < 32) {
-            if (in) {
-                const uint2 v = *reinterpret_cast<const uint2 *>(p.q + ((int64_t)m * p.nb + b) * 256 + kc * 8);
-                const uint32_t x = v.x ^ 0x80808080u, y = v.y ^ 0x80808080u;
-                o.x = u2(__hsub2(h2((x & 0x00FF00FFu) | 0x64006400u), k1152));
-                o.y = u2(__hsub2(h2(((x >> 8) & 0x00FF00FFu) | 0x64006400u), k1152));
-                o.z = u2(__hsub2(h2((y & 0x00FF00FFu) | 0x64006400u), k1152));
-                o.w = u2(__hsub2(h2(((y >> 8) & 0x00FF00FFu) | 0x64006400u), k1152));
-            }
-            if (kc == 0) p.da[(int64_t)b * p.m_pad + base + at] = in ? p.d[(int64_t)m * p.nb + b] : 0.f;
-        } else if (in) { // |sum of 16| <= 2032: exact
-            const int4 s8 = *reinterpret_cast<const int4 *>(p.bs + ((int64_t)m * p.nb + b) * 16 + 8 * (kc - 32));
-            const int16_t *s = reinterpret_cast<const int16_t *>(&s8);
-            __half h[8];
+    auto source_row = [&](int at) { return (int64_t)(p.row_src ? p.row_src[base + at] / p.act_div : base + at) * p.nb + b; };
+    if (threadIdx.x < 16) p.da[(int64_t)b * p.m_pad + base + threadIdx.x] = (int)threadIdx.x < n_live ? p.d[source_row(threadIdx.x)] : 0.f;
+    if (p.img16) {
+        for (int i = threadIdx.x; i < 2 * 34 * 8; i += blockDim.x) {
+            const int r = i & 7, kc = (i >> 3) % 34, g = i / 272, at = g * 8 + r; // token at of the run
+            uint4 o = make_uint4(0, 0, 0, 0);
+            if (at < n_live) {
+                const int64_t m = source_row(at);
+                if (kc < 32) {
+                    const uint2 v = *reinterpret_cast<const uint2 *>(p.q + m * 256 + kc * 8);
+                    const uint32_t x = v.x ^ 0x80808080u, y = v.y ^ 0x80808080u;
+                    o.x = u2(__hsub2(h2((x & 0x00FF00FFu) | 0x64006400u), k1152));
+                    o.y = u2(__hsub2(h2(((x >> 8) & 0x00FF00FFu) | 0x64006400u), k1152));
+                    o.z = u2(__hsub2(h2((y & 0x00FF00FFu) | 0x64006400u), k1152));
+                    o.w = u2(__hsub2(h2(((y >> 8) & 0x00FF00FFu) | 0x64006400u), k1152));
+                } else { // |sum of 16| <= 2048: exact
+                    const int4 s8 = *reinterpret_cast<const int4 *>(p.bs + m * 16 + 8 * (kc - 32));
+                    const int16_t *s = reinterpret_cast<const int16_t *>(&s8);
+                    __half h[8];
 #pragma unroll
-            for (int j = 0; j < 8; j++) h[j] = __int2half_rn((int)s[j]);
-            o = *reinterpret_cast<uint4 *>(&h[0]);
+                    for (int j = 0; j < 8; j++) h[j] = __int2half_rn((int)s[j]);
+                    o = *reinterpret_cast<uint4 *>(&h[0]);
+                }
+            }
+            *reinterpret_cast<uint4 *>(p.img16 + ((int64_t)b * p.m_pad + base) * TOK16 + g * 8 * TOK16 + kc * 128 + r * 16) = o;
         }
-        *reinterpret_cast<uint4 *>(p.img + ((int64_t)b * p.m_pad + base) * TOK_BYTES + g * GROUP_BYTES + kc * 128 + r * 16) = o;
+    }
+    if (p.img8) {
+        for (int i = threadIdx.x; i < 2 * 16 * 8; i += blockDim.x) {
+            const int r = i & 7, kc = (i >> 3) & 15, g = i >> 7, at = g * 8 + r;
+            uint4 o = make_uint4(0, 0, 0, 0);
+            if (at < n_live) o = *reinterpret_cast<const uint4 *>(p.q + source_row(at) * 256 + kc * 16);
+            *reinterpret_cast<uint4 *>(p.img8 + ((int64_t)b * p.m_pad + base) * TOK8 + g * 8 * TOK8 + kc * 128 + r * 16) = o;
+        }
     }
 }
 
@@ -770,17 +781,17 @@ namespace {
 // at a time).  A buffer that has become too small is kept: a captured graph may hold its address; the next one is at
 // least twice as large, so all of them together stay below twice the largest.
 struct Scratch {
-    uint8_t *img;
+    uint8_t *img16, *img8;
     float *da, *part;
 };
-b200_status scratch(int dev, size_t img_bytes, size_t da_bytes, Scratch *out) {
+b200_status scratch(int dev, size_t img16_bytes, size_t img8_bytes, size_t da_bytes, Scratch *out) {
     static std::mutex mu;
-    static void *buf[MAX_DEVICES][3];
-    static size_t cap[MAX_DEVICES][3];
+    static void *buf[MAX_DEVICES][4];
+    static size_t cap[MAX_DEVICES][4];
     static bool attr[MAX_DEVICES];
     std::lock_guard<std::mutex> lock(mu);
-    const size_t need[3] = {img_bytes, da_bytes, (size_t)kq_sm_count() * 2 * TILE_OUT * 4};
-    for (int i = 0; i < 3; i++) {
+    const size_t need[4] = {img16_bytes, img8_bytes, da_bytes, (size_t)kq_sm_count() * 2 * TILE_OUT * 4};
+    for (int i = 0; i < 4; i++) {
         if (need[i] <= cap[dev][i]) continue;
         size_t bytes = std::max(need[i], cap[dev][i] * 2);
         void *b = nullptr;
@@ -811,8 +822,15 @@ b200_status scratch(int dev, size_t img_bytes, size_t da_bytes, Scratch *out) {
         KQ_REQUIRE(4 * std::min(a4.numRegs, a6.numRegs) >= 2 * REG_EPI + REG_UNPACK + REG_REST, "gemm: built with %d / %d registers", a4.numRegs, a6.numRegs);
         attr[dev] = true;
     }
-    *out = {(uint8_t *)buf[dev][0], (float *)buf[dev][1], (float *)buf[dev][2]};
+    *out = {img16_bytes ? (uint8_t *)buf[dev][0] : nullptr, img8_bytes ? (uint8_t *)buf[dev][1] : nullptr, (float *)buf[dev][2], (float *)buf[dev][3]};
     return B200_OK;
+}
+
+// images of m_pad tokens in the forms that the matrices read
+b200_status scratch_for(int dev, const KqGemvSeg *segs, int nseg, int64_t m_pad, int64_t nb, Scratch *out) {
+    bool q4 = false, q6 = false;
+    for (int i = 0; i < nseg; i++) (segs[i].type == B200_TYPE_Q4_K ? q4 : q6) = true;
+    return scratch(dev, q4 ? (size_t)(m_pad * nb * TOK16) : 0, q6 ? (size_t)(m_pad * nb * TOK8) : 0, (size_t)(m_pad * nb * 4), out);
 }
 
 b200_status add_seg(Params &p, int i, const KqGemvSeg &g, int64_t experts, int64_t K) {
@@ -846,11 +864,12 @@ b200_status add_seg(Params &p, int i, const KqGemvSeg &g, int64_t experts, int64
 // 1457 / 1468 / 1633 us at 2 / 4 / 8, 16 users of the experts' model 1073 / 1089 / 1132; large products do not depend on it.
 constexpr int MIN_SHARE = 2;
 
-// one launch per weight type for the matrices that read the image in p
-b200_status launch_segs(Params p, const KqGemvSeg *segs, int nseg, int64_t experts, int64_t K, cudaStream_t st) {
+// one launch per weight type for the matrices that read the images in sc
+b200_status launch_segs(Params p, const Scratch &sc, const KqGemvSeg *segs, int nseg, int64_t experts, int64_t K, cudaStream_t st) {
     for (const uint32_t type : {(uint32_t)B200_TYPE_Q4_K, (uint32_t)B200_TYPE_Q6_K}) {
         int n = 0;
         p.row_tiles = 0;
+        p.img = type == B200_TYPE_Q4_K ? sc.img16 : sc.img8, p.da = sc.da, p.part = sc.part;
         for (int i = 0; i < nseg; i++)
             if (segs[i].type == type) KQ_TRY(add_seg(p, n++, segs[i], experts, K));
         if (!n) continue;
@@ -907,18 +926,17 @@ b200_status kq_launch_gemm_tc(const KqGemvSeg *segs, int nseg, const int8_t *q, 
         p.m_pad = p.tok_tiles * p.tile_tok;
         p.M = (int32_t)mc, p.nb = (int32_t)nb;
         Scratch sc;
-        KQ_TRY(scratch(dev, (size_t)p.m_pad * TOK_BYTES * nb, (size_t)p.m_pad * 4 * nb, &sc));
-        const ImageParams ip = {q + m0 * K, d + m0 * nb, bs + m0 * nb * 16, sc.img, sc.da, (int32_t)mc, (int32_t)nb, p.m_pad, 1, nullptr, nullptr, nullptr};
+        KQ_TRY(scratch_for(dev, segs, nseg, p.m_pad, nb, &sc));
+        const ImageParams ip = {q + m0 * K, d + m0 * nb, bs + m0 * nb * 16, sc.img16, sc.img8, sc.da, (int32_t)mc, (int32_t)nb, p.m_pad, 1, nullptr, nullptr, nullptr};
         KQ_CUDA(kq_launch(act_image_kernel, dim3((unsigned)(p.m_pad / 16), (unsigned)nb), dim3(288), 0, st, ip));
         KQ_COUNT_LAUNCH();
-        p.img = sc.img, p.da = sc.da, p.part = sc.part;
         KqGemvSeg sg[MAX_SEGS];
         for (int i = 0; i < nseg; i++) {
             sg[i] = segs[i];
             sg[i].y += m0 * sg[i].n_rows;
         }
         p.residual = residual ? residual + m0 * segs[0].n_rows : nullptr;
-        KQ_TRY(launch_segs(p, sg, nseg, 1, K, st));
+        KQ_TRY(launch_segs(p, sc, sg, nseg, 1, K, st));
     }
     return B200_OK;
 }
@@ -959,11 +977,10 @@ b200_status kq_launch_gemm_grouped(const KqGemvSeg *segs, int nseg, const int8_t
     Params p = {};
     p.M = p.m_pad = (int32_t)(mt * TM), p.nb = (int32_t)nb, p.tok_tiles = (int)mt;
     Scratch sc;
-    KQ_TRY(scratch(dev, (size_t)p.m_pad * TOK_BYTES * nb, (size_t)p.m_pad * 4 * nb, &sc));
+    KQ_TRY(scratch_for(dev, segs, nseg, p.m_pad, nb, &sc));
     p.n_tiles = sorted, p.tile_expert = sorted + 1, p.row_src = sorted + 1 + mt, p.tile_count = sorted + 1 + mt + mt * TM;
-    const ImageParams ip = {q, d, bs, sc.img, sc.da, 0, (int32_t)nb, p.m_pad, act_div, p.row_src, p.tile_count, p.n_tiles};
+    const ImageParams ip = {q, d, bs, sc.img16, sc.img8, sc.da, 0, (int32_t)nb, p.m_pad, act_div, p.row_src, p.tile_count, p.n_tiles};
     KQ_CUDA(kq_launch(act_image_kernel, dim3((unsigned)(p.m_pad / 16), (unsigned)nb), dim3(288), 0, st, ip));
     KQ_COUNT_LAUNCH();
-    p.img = sc.img, p.da = sc.da, p.part = sc.part;
-    return launch_segs(p, segs, nseg, E, K, st);
+    return launch_segs(p, sc, segs, nseg, E, K, st);
 }

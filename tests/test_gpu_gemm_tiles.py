@@ -78,6 +78,56 @@ def test_long_shares_and_cut_tiles(ty, N, K, M):
     check(got[0].cpu().numpy(), want, size, K)
 
 
+def extreme_blocks(ty, kind, N, rng):
+    """blocks of one scale factor 1 whose sums are as large as the format allows, or pass through such sums on their way to a small one"""
+    blk = np.zeros((N, 144 if ty == orc.TYPE_Q4_K else 210), np.uint8)
+    one = np.array([1.0], np.float16).view(np.uint8)
+    top = kind != "near" # "near": every scale and code near its end of the range
+    if ty == orc.TYPE_Q4_K:
+        sc, q = (np.full((N, 8), 63), np.full((N, 256), 15)) if top else (rng.integers(56, 64, (N, 8)), rng.integers(12, 16, (N, 256)))
+        blk[:, 0:2] = one
+        blk[:, 4:8] = sc[:, :4] | (sc[:, 4:] >> 4) << 6
+        blk[:, 12:16] = sc[:, 4:] & 15
+        q = q.reshape(N, 4, 2, 32)
+        blk[:, 16:] = (q[:, :, 0] | q[:, :, 1] << 4).reshape(N, 128)
+    else:
+        sc, q = (np.full((N, 16), -128), np.zeros((N, 256), int)) if top else (rng.integers(-128, -119, (N, 16)), rng.integers(0, 4, (N, 256)))
+        q = q.reshape(N, 2, 2, 2, 32)  # [half][low or high nibble][32 of 64][..]
+        blk[:, :128] = ((q[:, :, 0] & 15) | (q[:, :, 1] & 15) << 4).reshape(N, 128)
+        quarters = q.reshape(N, 2, 4, 32) >> 4
+        blk[:, 128:192] = (quarters[:, :, 0] | quarters[:, :, 1] << 2 | quarters[:, :, 2] << 4 | quarters[:, :, 3] << 6).reshape(N, 64)
+        blk[:, 192:208] = sc.astype(np.int8).view(np.uint8)
+        blk[:, 208:210] = one
+    return blk
+
+
+@pytest.mark.parametrize("ty", [orc.TYPE_Q6_K], ids=["q6_k"])
+@pytest.mark.parametrize("kind", ["top", "near", "cancelling"])
+@pytest.mark.parametrize("M", [1, 8, 9, 77, 300])
+def test_largest_block_sums(ty, kind, M):
+    """one block, scale factors 1: the result is the block's integer sum, up to 3.1e7 (Q4_K) or 1.3e8 (Q6_K), rounded to f32 once: off by
+    half a spacing of f32 at most, and not at all below 2^24"""
+    import torch
+
+    from mesh_llm_b200 import ops
+
+    rng = np.random.default_rng(M)
+    N, K = 130, 256
+    W = extreme_blocks(ty, kind, N, rng)
+    x = np.full((M, K), 127.0, np.float32) if kind == "top" else rng.integers(120, 128, (M, K)).astype(np.float32)
+    x[:, 0] = 127.0  # the Q8 scale is 1
+    if kind == "cancelling":
+        x[:, 128:] *= -1
+    x[1::2] *= -1
+    q, d, bs = orc.quantize_act(x)
+    assert np.all(d == 1.0) and np.array_equal(q.astype(np.float32), x)
+    si, _ = orc.block_sums(ty, W, q, bs, N, K)
+    want = si.astype(np.float64).reshape(M, N)
+    assert kind == "cancelling" or np.abs(want).min() > 2.0 ** 24
+    got = ops.mul_mat(ty, ops.upload_weights(ty, W, N, K), torch.from_numpy(x).cuda(), N, K).cpu().numpy()
+    assert np.all(np.abs(got.astype(np.float64) - want) <= np.where(np.abs(want) < 2.0 ** 24, 0.0, np.spacing(np.abs(want).astype(np.float32)) / 2))
+
+
 def test_more_tokens_than_a_slab():
     import torch
 
