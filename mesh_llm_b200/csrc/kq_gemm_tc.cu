@@ -2,8 +2,10 @@
 // y[m][n] = sum_k W[n][k] x[m][k], W in Q4_K / Q6_K blocks, x in Q8 blocks of 256.
 //
 // The integer scale of a sub-block is folded into the weight, and the products of a 256-element block are added up as integers.
-// Q4_K: w' = sc_j q is at most 945, exact in f16, and so is a Q8 code, so one tcgen05.mma of kind::f16 per 16 elements adds up
-// sum_j sc_j sum_i q_ij a_ij  in f32, exactly while it stays below 2^24.  The min term sum_j m_j bsum_j is one more MMA (K = 16) into an
+// Q4_K: w' = sc_j q goes in as sc_j q - k_j, |.| <= 512, with k_j about 8 sc_j: exact in f16, as a Q8 code is, so one
+// tcgen05.mma of kind::f16 per 16 elements adds up  sum_j sum_i (sc_j q_ij - k_j) a_ij  in f32, and no partial sum exceeds 2^24: exact.
+// One more MMA (K = 16) adds sum_j k_j bsum_j, which makes it the block's integer sum: above 2^24 that one addition rounds, by half a
+// spacing at most as a conversion from int32 would.  The min term sum_j m_j bsum_j is another MMA into an
 // accumulator of its own.  Per block an output then takes y += d_a (d_w main - d_min min) in f32.
 // Q6_K: w' = sc (q - 32) has 14 bits with its sign, w' = 64 hi + lo with |hi| <= 64 and 0 <= lo < 64.  Both are bytes, and two tcgen05.mma of
 // kind::i8 per 32 elements, each into an int32 accumulator of its own, give the sum of the block whatever its size; it is rounded once, to f32.
@@ -24,8 +26,8 @@
 // What bounds it, in clocks per block of 128 rows x 256 tokens: the MMAs 2900 in either type (42 each at N = 64, where 32 would be the tensor
 // rate), the drains about 1000 of every scheduler.  Measured about 5500 for 256 tokens and 2600 (Q4_K) or 4000 (Q6_K) for 16, where the decoding is
 // what is left: one warp of each scheduler walks through it.  The same decoding unrolled four times made the whole kernel 10 % slower.
-// Q4_K: two int8 planes per weight out of shared memory (the form before this one) took 1659 us where this takes 1240, for 2048 tokens x 28672 x
-// 8192, 547 against 315 at 512 tokens, 169 against 66 at 16.  Q6_K, whose two planes came from shared memory as well: 1637 against 1324,
+// Q4_K: two int8 planes per weight out of shared memory (the form before this one) took 1659 us where this takes 1204, for 2048 tokens x 28672 x
+// 8192, 547 against 317 at 512 tokens, 169 against 67 at 16 (without the k_j, exact below 2^24 only: 1201, 316, 66).  Q6_K, whose two planes came from shared memory as well: 1637 against 1324,
 // 624 against 351, 248 against 110; as two f16 addends into one f32 accumulator, with the decoded operand in a single buffer, it
 // took 2125, 512 and 155, and was exact only below 2^24.
 // Every wait is bounded; on a time-out the kernel records an error, lets its copies and MMAs end, frees its TMEM and returns.
@@ -51,9 +53,10 @@ template <bool Q6>
 struct Cfg {
     static constexpr int RAW_BYTES = Q6 ? 13 * ROWS * 32 : ROWS * KQ_Q4K_BYTES; // Q6_K: two blocks of each row
     static constexpr int TOK_BYTES = Q6 ? TOK8 : TOK16, B_BYTES = CHUNK * TOK_BYTES;
-    static constexpr int RAW_STAGES = Q6 ? 2 : 4, B_STAGES = Q6 ? 6 : 4;
+    static constexpr int RAW_STAGES = Q6 ? 2 : 3, B_STAGES = Q6 ? 6 : 4;
+    static constexpr int AMIN_BYTES = 8192; // Q4_K, per block: the operands m_j and k_j for the sums of 16, each twice
     static constexpr int SM_B = 0, SM_RAW = B_STAGES * B_BYTES, SM_AMIN = SM_RAW + RAW_STAGES * RAW_BYTES,
-                         SM_DA = SM_AMIN + (Q6 ? 0 : 2 * 4096), SM_SC = SM_DA + DA_RING * CHUNK * 4, SMEM = SM_SC + SC_RING * ROWS * 4;
+                         SM_DA = SM_AMIN + (Q6 ? 0 : 2 * AMIN_BYTES), SM_SC = SM_DA + DA_RING * CHUNK * 4, SMEM = SM_SC + SC_RING * ROWS * 4;
     static_assert(SM_RAW % 128 == 0 && RAW_BYTES % 128 == 0 && SM_AMIN % 16 == 0, "TMA destinations are 128-byte aligned");
     static_assert(SMEM <= 226 * 1024, "shared memory of a CTA");
     // the two issuing warps take alternate chunks: with an even number a stage is always the same warp's, which then waits for every phase of it
@@ -119,6 +122,8 @@ __device__ __forceinline__ __half2 h2(uint32_t v) { return *reinterpret_cast<__h
 __device__ __forceinline__ uint32_t u2(__half2 v) { return *reinterpret_cast<uint32_t *>(&v); }
 // byte b of v as an f16 pair, 1024 + byte in both halves
 __device__ __forceinline__ __half2 byte_pair(uint32_t v, int b) { return h2(__byte_perm(v, 0x64646464u, 0x4040u | (b << 8) | b)); }
+// bytes b and b + 1 of v as f16
+__device__ __forceinline__ __half2 two_bytes(uint32_t v, int b) { return __hsub2(h2(__byte_perm(v, 0x64646464u, 0x4040u | ((b + 1) << 8) | b)), __float2half2_rn(1024.f)); }
 
 #define TMEM_ST4(taddr, r) \
     asm volatile("tcgen05.st.sync.aligned.32x32b.x4.b32 [%0], {%1,%2,%3,%4};" ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]) : "memory")
@@ -296,7 +301,9 @@ __global__ void __launch_bounds__(NTHREADS, 1) gemm_kq_kernel(const __grid_const
                         } else {
 #pragma unroll 4
                             for (int i = 0; i < 16; i++) tc_mma_ts(acc, a + i * 8, bd + i * 16, id, i > 0);
-                            tc_mma_ss(acc + CHUNK, nosw_desc(smem_u32(smem + C::SM_AMIN + sa * 4096), 2048, 128), bd + 256, id, 0);
+                            const uint32_t mins = smem_u32(smem + C::SM_AMIN + sa * C::AMIN_BYTES);
+                            tc_mma_ss(acc, nosw_desc(mins + 4096, 2048, 128), bd + 256, id, 1); // last: the others are exact
+                            tc_mma_ss(acc + CHUNK, nosw_desc(mins, 2048, 128), bd + 256, id, 0);
                         }
                         if (last) tc_commit(smem_u32(&a_empty[sa]));
                     }
@@ -337,22 +344,24 @@ __global__ void __launch_bounds__(NTHREADS, 1) gemm_kq_kernel(const __grid_const
                 const uint8_t *blk = smem + C::SM_RAW + s * C::RAW_BYTES + row * KQ_Q4K_BYTES;
                 const uint4 hdr = *reinterpret_cast<const uint4 *>(blk);
                 const uint32_t sc_lo = hdr.y & 0x3F3F3F3Fu, sc_hi = (hdr.w & 0x0F0F0F0Fu) | ((hdr.y >> 2) & 0x30303030u);
-                {
+                { // m_j, then k_j, in order of j, for the sums of 16 of even and of odd place
                     const uint32_t m_lo = hdr.z & 0x3F3F3F3Fu, m_hi = ((hdr.w >> 4) & 0x0F0F0F0Fu) | ((hdr.z >> 2) & 0x30303030u);
-                    uint4 *am = reinterpret_cast<uint4 *>(smem + C::SM_AMIN + sa * 4096 + (row >> 3) * 128 + (row & 7) * 16);
-                    am[0] = make_uint4(u2(__hsub2(byte_pair(m_lo, 0), k1024)), u2(__hsub2(byte_pair(m_lo, 1), k1024)),
-                                       u2(__hsub2(byte_pair(m_lo, 2), k1024)), u2(__hsub2(byte_pair(m_lo, 3), k1024)));
-                    am[128] = make_uint4(u2(__hsub2(byte_pair(m_hi, 0), k1024)), u2(__hsub2(byte_pair(m_hi, 1), k1024)),
-                                         u2(__hsub2(byte_pair(m_hi, 2), k1024)), u2(__hsub2(byte_pair(m_hi, 3), k1024)));
+                    uint4 *am = reinterpret_cast<uint4 *>(smem + C::SM_AMIN + sa * C::AMIN_BYTES + (row >> 3) * 128 + (row & 7) * 16);
+                    am[0] = am[128] = make_uint4(u2(two_bytes(m_lo, 0)), u2(two_bytes(m_lo, 2)), u2(two_bytes(m_hi, 0)), u2(two_bytes(m_hi, 2)));
+                    auto k = [&](__half2 sc) { // what the decoding below takes off two neighbouring sub-blocks
+                        return u2(__hfma2(sc, __floats2half2_rn(-1024.f, 0.f), __hmul2(sc, __floats2half2_rn(1032.f, 8.f))));
+                    };
+                    am[256] = am[384] = make_uint4(k(two_bytes(sc_lo, 0)), k(two_bytes(sc_lo, 2)), k(two_bytes(sc_hi, 0)), k(two_bytes(sc_hi, 2)));
                     *reinterpret_cast<uint32_t *>(smem + C::SM_SC + ((u % SC_RING) * ROWS + row) * 4) = hdr.x;
                 }
 #pragma unroll 1
                 for (int g = 0; g < 4; g++) { // 64 elements: sub-block 2g in the low nibbles, 2g + 1 in the high ones
                     const uint32_t scw = (g < 2 ? sc_lo : sc_hi) >> (16 * (g & 1));
                     const __half2 s0 = __hsub2(byte_pair(scw, 0), k1024), s1 = __hsub2(byte_pair(scw, 1), k1024);
-                    // (1024 + q) sc - 1024 sc and (1024 + 16 q) sc / 16 - 64 sc: one rounding, of an exact result
-                    const __half2 o0 = __hmul2(s0, __float2half2_rn(-1024.f)), t1 = __hmul2(s1, __float2half2_rn(0.0625f)),
-                                  o1 = __hmul2(s1, __float2half2_rn(-64.f));
+                    // (1024 + q) sc - f16(1032 sc) and (1024 + 16 q) sc / 16 - 72 sc: one rounding, of an exact result.  f16(1032 sc) - 1024 sc = k is
+                    // within 16 of 8 sc and a multiple of 32 from sc = 32 on: -512 <= sc q - k <= 441 for every scale
+                    const __half2 o0 = __hmul2(s0, __float2half2_rn(-1032.f)), t1 = __hmul2(s1, __float2half2_rn(0.0625f)),
+                                  o1 = __hmul2(s1, __float2half2_rn(-72.f));
                     uint32_t o[32];
 #pragma unroll
                     for (int h = 0; h < 2; h++) {
@@ -641,12 +650,13 @@ __global__ void __launch_bounds__(288) act_image_kernel(const __grid_constant__ 
                     o.y = u2(__hsub2(h2(((x >> 8) & 0x00FF00FFu) | 0x64006400u), k1152));
                     o.z = u2(__hsub2(h2((y & 0x00FF00FFu) | 0x64006400u), k1152));
                     o.w = u2(__hsub2(h2(((y >> 8) & 0x00FF00FFu) | 0x64006400u), k1152));
-                } else { // |sum of 16| <= 2048: exact
-                    const int4 s8 = *reinterpret_cast<const int4 *>(p.bs + m * 16 + 8 * (kc - 32));
-                    const int16_t *s = reinterpret_cast<const int16_t *>(&s8);
+                } else { // |sum of 16| <= 2048: exact.  Those of even place, then those of odd place
+                    const int4 *sums = reinterpret_cast<const int4 *>(p.bs + m * 16);
+                    const int4 s8[2] = {sums[0], sums[1]};
+                    const int16_t *s = reinterpret_cast<const int16_t *>(&s8[0]);
                     __half h[8];
 #pragma unroll
-                    for (int j = 0; j < 8; j++) h[j] = __int2half_rn((int)s[j]);
+                    for (int j = 0; j < 8; j++) h[j] = __int2half_rn((int)(kc == 32 ? s[2 * j] : s[2 * j + 1]));
                     o = *reinterpret_cast<uint4 *>(&h[0]);
                 }
             }

@@ -2,6 +2,7 @@
 import os
 import re
 
+import numpy as np
 import pytest
 
 SRC = os.path.join(os.path.dirname(__file__), "..", "mesh_llm_b200", "csrc", "kq_gemm_tc.cu")
@@ -75,3 +76,21 @@ def test_rings_without_an_empty_barrier(q6, chunks):
         u = q
         last = (u - 2) * chunks + chunks - 1  # its last chunk
         assert (u - c["SC_RING"]) * chunks + chunks - 1 <= drained_when_issued(last)
+
+
+def test_decoded_q4_weights_are_exact_in_f16():
+    """sc q - k by the two multiply-adds of the decoder, for every scale and code: the integer itself, at most 512, so that 256 of them times
+    a code of 128 stay within 2^24; and k, exact"""
+    h = np.float16
+    decoder = source()[source().index("auto k = [&](__half2 sc)"):]
+    assert re.findall(r"__floats2half2_rn\((-?[\d.]+)f, (-?[\d.]+)f\)", decoder)[:2] == [("-1024.", "0."), ("1032.", "8.")]
+    assert re.findall(r"__float2half2_rn\((-?[\d.]+)f\)", decoder)[:3] == ["-1032.", "0.0625", "-72."]
+    fma = lambda a, b, c: h(float(a) * float(b) + float(c))  # one rounding: product and sum are exact in double
+    for sc in range(64):
+        o0, o1 = h(h(sc) * h(-1032.0)), h(h(sc) * h(-72.0))
+        k0, k1 = fma(h(sc), h(-1024.0), h(h(sc) * h(1032.0))), h(h(sc) * h(8.0))
+        assert np.isfinite(o0) and float(o0) == -1024 * sc - float(k0) and float(o1) == -72 * sc and float(k1) == 8 * sc
+        for q in range(16):
+            low, high = fma(h(1024 + q), h(sc), o0), fma(h(1024 + 16 * q), h(h(sc) * h(0.0625)), o1)
+            assert float(low) == sc * q - float(k0) and float(high) == sc * q - float(k1)
+            assert max(abs(float(low)), abs(float(high))) * 128 * 256 <= 2 ** 24

@@ -101,7 +101,7 @@ def extreme_blocks(ty, kind, N, rng):
     return blk
 
 
-@pytest.mark.parametrize("ty", [orc.TYPE_Q6_K], ids=["q6_k"])
+@pytest.mark.parametrize("ty", [orc.TYPE_Q4_K, orc.TYPE_Q6_K], ids=["q4_k", "q6_k"])
 @pytest.mark.parametrize("kind", ["top", "near", "cancelling"])
 @pytest.mark.parametrize("M", [1, 8, 9, 77, 300])
 def test_largest_block_sums(ty, kind, M):
