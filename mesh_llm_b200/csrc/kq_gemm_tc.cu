@@ -874,11 +874,44 @@ b200_status add_seg(Params &p, int i, const KqGemvSeg &g, int64_t experts, int64
 // 1457 / 1468 / 1633 us at 2 / 4 / 8, 16 users of the experts' model 1073 / 1089 / 1132; large products do not depend on it.
 constexpr int MIN_SHARE = 2;
 
-// one launch per weight type for the matrices that read the images in sc
+// Token tiles of a dense product, by the time they should take in tenths of a microsecond.  A (tile, block) pair costs its decoding and, per 64 tokens,
+// its MMAs and drains (Q4_K 1.6 us at 64 tokens, 3.6 at 256; Q6_K 2.4 and 4.0); adding up a tile that was cut costs its last CTA about 1 us
+// per part and 64 tokens.  Wide tiles decode a weight less often; narrow ones are more pairs, hence fewer parts and a shorter end where a product
+// is too small to keep the GPU busy: 256 x 2048 at 1024 tokens in Q4_K 32.4 us as tiles of 256 tokens, 19.7 as tiles of 64; 1024 x 5120 at 512 50.6 and
+// 27.6, at 2048 62.4 and (tiles of 128) 55.2; 5120 x 5120 at 1024 96 and 131.
+struct TokTiles {
+    int n, tok;
+};
+TokTiles token_tiles(bool q6, int64_t M, int64_t row_tiles, int64_t nb) {
+    TokTiles best = {0, 0};
+    int64_t best_cost = INT64_MAX;
+    for (int chunks = MAX_CHUNKS; chunks >= 1; chunks--) {
+        int c, cw;
+        chunks_of((int)kq_div_up(M, kq_div_up(M, chunks * CHUNK)), c, cw);
+        const int64_t tiles = kq_div_up(M, c * cw), pairs = tiles * row_tiles * nb, ctas = std::max<int64_t>(1, std::min<int64_t>(kq_sm_count(), pairs / MIN_SHARE));
+        const int64_t share = kq_div_up(pairs, ctas), per_pair = (q6 ? 19 : 8) * CHUNK + (q6 ? 5 : 7) * c * cw;
+        const int64_t cost = share * per_pair + (pairs % ctas == 0 && share % nb == 0 ? 0 : 10 * c * cw * nb / share);
+        if (cost < best_cost) best_cost = cost, best = {(int)tiles, c * cw};
+    }
+    return best;
+}
+// the same for a call's matrices of one type; none: no tiles
+TokTiles token_tiles_of(uint32_t type, const KqGemvSeg *segs, int nseg, int64_t M, int64_t nb) {
+    int64_t row_tiles = 0;
+    for (int i = 0; i < nseg; i++)
+        if (segs[i].type == type) row_tiles += kq_div_up(segs[i].n_rows, ROWS);
+    return row_tiles ? token_tiles(type == B200_TYPE_Q6_K, M, row_tiles, nb) : TokTiles{0, 0};
+}
+
+// one launch per weight type for the matrices that read the images in sc; dense products cut the tokens by type
 b200_status launch_segs(Params p, const Scratch &sc, const KqGemvSeg *segs, int nseg, int64_t experts, int64_t K, cudaStream_t st) {
     for (const uint32_t type : {(uint32_t)B200_TYPE_Q4_K, (uint32_t)B200_TYPE_Q6_K}) {
         int n = 0;
         p.row_tiles = 0;
+        if (!p.row_src) {
+            const TokTiles t = token_tiles_of(type, segs, nseg, p.M, p.nb);
+            p.tok_tiles = t.n, p.tile_tok = t.tok;
+        }
         p.img = type == B200_TYPE_Q4_K ? sc.img16 : sc.img8, p.da = sc.da, p.part = sc.part;
         for (int i = 0; i < nseg; i++)
             if (segs[i].type == type) KQ_TRY(add_seg(p, n++, segs[i], experts, K));
@@ -917,7 +950,9 @@ int kq_gemm_error_fetch() {
     return v;
 }
 
-constexpr int64_t SLAB = 4096; // tokens whose images are held at a time
+// Tokens whose images are held at a time: every row tile reads the images again, so they should stay in L2 (126 MB) beside the weights that
+// stream by.  2048 and 4096 tokens x 8192 x 28672 in Q4_K, 125 and 250 MB at once: 1363 and 2788 us; in slabs of 62 MB 1200 and 2406.
+constexpr int64_t SLAB_BYTES = 64 << 20, SLAB_MIN = MAX_CHUNKS * CHUNK;
 
 b200_status kq_launch_gemm_tc(const KqGemvSeg *segs, int nseg, const int8_t *q, const float *d, const int16_t *bs, int64_t M, int64_t K,
                               const float *residual, cudaStream_t st) {
@@ -925,16 +960,19 @@ b200_status kq_launch_gemm_tc(const KqGemvSeg *segs, int nseg, const int8_t *q, 
     KQ_TRY(check_segs(segs, nseg, q, K, &dev));
     KQ_REQUIRE(M > 0 && (!residual || nseg == 1), "gemm: bad shape");
     const int64_t nb = K / 256;
-    for (int64_t m0 = 0; m0 < M; m0 += SLAB) {
-        const int64_t mc = std::min(SLAB, M - m0);
+    int64_t token_bytes = 0;
+    for (const uint32_t type : {(uint32_t)B200_TYPE_Q4_K, (uint32_t)B200_TYPE_Q6_K})
+        if (token_tiles_of(type, segs, nseg, M, nb).n) token_bytes += nb * (type == B200_TYPE_Q4_K ? TOK16 : TOK8);
+    const int64_t slab = std::max(SLAB_MIN, SLAB_BYTES / token_bytes / SLAB_MIN * SLAB_MIN);
+    for (int64_t m0 = 0, mc; m0 < M; m0 += mc) {
+        mc = kq_div_up(M - m0, kq_div_up(M - m0, slab)); // of equal size
+        if (mc < M - m0) mc = kq_div_up(mc, SLAB_MIN) * SLAB_MIN;
         Params p = {};
-        int c, cw;
-        p.tok_tiles = (int)kq_div_up(mc, MAX_CHUNKS * CHUNK);
-        chunks_of((int)kq_div_up(mc, p.tok_tiles), c, cw);
-        p.tile_tok = c * cw;
-        p.tok_tiles = (int)kq_div_up(mc, p.tile_tok);
-        p.m_pad = p.tok_tiles * p.tile_tok;
         p.M = (int32_t)mc, p.nb = (int32_t)nb;
+        for (const uint32_t type : {(uint32_t)B200_TYPE_Q4_K, (uint32_t)B200_TYPE_Q6_K}) {
+            const TokTiles t = token_tiles_of(type, segs, nseg, mc, nb);
+            p.m_pad = std::max(p.m_pad, t.n * t.tok);
+        }
         Scratch sc;
         KQ_TRY(scratch_for(dev, segs, nseg, p.m_pad, nb, &sc));
         const ImageParams ip = {q + m0 * K, d + m0 * nb, bs + m0 * nb * 16, sc.img16, sc.img8, sc.da, (int32_t)mc, (int32_t)nb, p.m_pad, 1, nullptr, nullptr, nullptr};

@@ -78,6 +78,22 @@ def test_long_shares_and_cut_tiles(ty, N, K, M):
     check(got[0].cpu().numpy(), want, size, K)
 
 
+@pytest.mark.parametrize("ty", [orc.TYPE_Q4_K, orc.TYPE_Q6_K], ids=["q4_k", "q6_k"])
+@pytest.mark.parametrize("N,K,M", [(6000, 2816, 257), (6000, 2816, 400), (6000, 2816, 500), (3000, 512, 513), (1024, 5120, 77), (70, 27648, 1100)])
+def test_widths_of_token_tiles(ty, N, K, M):
+    """sizes whose tokens are cut into tiles of one to four chunks, with a shorter last one, and into slabs (rows of 27648)"""
+    import torch
+
+    from mesh_llm_b200 import capi, ops
+
+    W = blocks_of(ty, N, K, 11)
+    x = np.random.default_rng(12).standard_normal((M, K)).astype(np.float32)
+    want, size = exact(ty, W, x, N, K)
+    got = ops.mul_mat(ty, ops.upload_weights(ty, W, N, K), torch.from_numpy(x).cuda(), N, K).cpu().numpy()
+    assert capi.lib().b200_check_device_waits() == 0
+    check(got, want, size, K)
+
+
 def extreme_blocks(ty, kind, N, rng):
     """blocks of one scale factor 1 whose sums are as large as the format allows, or pass through such sums on their way to a small one"""
     blk = np.zeros((N, 144 if ty == orc.TYPE_Q4_K else 210), np.uint8)
