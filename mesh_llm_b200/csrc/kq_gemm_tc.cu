@@ -89,6 +89,7 @@ struct Params {
     int64_t w_row;
     // products with experts: token tile t belongs to expert tile_expert[t] and holds the tile_count[t] pairs row_src[128 t ..]
     const int32_t *row_src, *tile_expert, *tile_count, *n_tiles;
+    int32_t first_tile; // of the token tiles that n_tiles counts, the one that is tile 0 of this launch
 };
 
 __host__ __device__ __forceinline__ void chunks_of(int n, int &c, int &cw) { // n tokens as c chunks of cw
@@ -208,7 +209,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) gemm_kq_kernel(const __grid_const
     const uint32_t tmem = s_tmem;
     // this CTA's share of the (tile, block) pairs: per pairs, one more for the first rem CTAs
     const int nb = p.nb;
-    const uint32_t units = (uint32_t)(p.row_src ? *p.n_tiles : p.tok_tiles) * p.row_tiles * nb;
+    const uint32_t units = (uint32_t)(p.row_src ? max(0, min(*p.n_tiles - p.first_tile, p.tok_tiles)) : p.tok_tiles) * p.row_tiles * nb;
     const uint32_t ctas = max(1u, min(gridDim.x, units / p.min_share)), per = units / ctas, rem = units - per * ctas;
     const uint32_t u0 = blockIdx.x * per + min(blockIdx.x, rem);
     const int total = blockIdx.x < ctas ? per + (blockIdx.x < rem) : 0, tile0 = total ? u0 / nb : 0, b0 = u0 - tile0 * nb;
@@ -618,6 +619,7 @@ struct ImageParams {
     float *da;
     int32_t M, nb, m_pad, act_div;
     const int32_t *row_src, *tile_count, *n_tiles; // products with experts
+    int32_t first_tile;
 };
 __global__ void __launch_bounds__(288) act_image_kernel(const __grid_constant__ ImageParams p) {
     KQ_PDL_ENTER();
@@ -627,7 +629,7 @@ __global__ void __launch_bounds__(288) act_image_kernel(const __grid_constant__ 
     int n_live = p.M - base; // tokens of this run
     if (p.row_src) {
         const int tile = base / 128;
-        if (tile >= *p.n_tiles) return;
+        if (tile >= *p.n_tiles - p.first_tile) return;
         const int n = p.tile_count[tile];
         int c, cw;
         chunks_of(n, c, cw);
@@ -788,39 +790,58 @@ b200_status kq_tmap_encode(void *map128, int elem_bytes, int rank, const void *b
 
 namespace {
 // Images, scales and parts of cut tiles, per device.  Launches that share them are ordered by the library's rule (one stream per device
-// at a time).  A buffer that has become too small is kept: a captured graph may hold its address; the next one is at
-// least twice as large, so all of them together stay below twice the largest.
+// at a time).  A buffer grows to what is needed and the old one is given back, unless a stream was being captured when it was handed out: the graph
+// holds its address, so it is kept, and the next one is twice as large (up to the largest that a call asks for), so that all that are kept
+// stay below that size together.
+constexpr int64_t SLAB_BYTES = 64 << 20, GROUP_BYTES = 256 << 20; // images of one launch: dense products, products with experts
+
 struct Scratch {
     uint8_t *img16, *img8;
     float *da, *part;
 };
-b200_status scratch(int dev, size_t img16_bytes, size_t img8_bytes, size_t da_bytes, Scratch *out) {
+b200_status scratch(int dev, size_t img16_bytes, size_t img8_bytes, size_t da_bytes, cudaStream_t st, Scratch *out) {
     static std::mutex mu;
     static void *buf[MAX_DEVICES][4];
     static size_t cap[MAX_DEVICES][4];
-    static bool attr[MAX_DEVICES];
+    static bool captured[MAX_DEVICES][4], attr[MAX_DEVICES];
     std::lock_guard<std::mutex> lock(mu);
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    KQ_CUDA(cudaStreamIsCapturing(st, &cs));
+    const bool capturing = cs != cudaStreamCaptureStatusNone;
     const size_t need[4] = {img16_bytes, img8_bytes, da_bytes, (size_t)kq_sm_count() * 2 * TILE_OUT * 4};
     for (int i = 0; i < 4; i++) {
-        if (need[i] <= cap[dev][i]) continue;
-        size_t bytes = std::max(need[i], cap[dev][i] * 2);
-        void *b = nullptr;
-        // an allocation is no work of the stream that is being captured
-        cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
-        KQ_CUDA(cudaThreadExchangeStreamCaptureMode(&mode));
-        cudaError_t e = cudaMalloc(&b, bytes);
-        if (e != cudaSuccess && bytes > need[i]) {
-            cudaGetLastError();
-            e = cudaMalloc(&b, bytes = need[i]);
+        if (need[i] > cap[dev][i]) {
+            // an allocation is no work of the stream that is being captured
+            cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+            KQ_CUDA(cudaThreadExchangeStreamCaptureMode(&mode));
+            size_t bytes = need[i];
+            cudaError_t e = cudaSuccess;
+            if (buf[dev][i]) {
+                if (captured[dev][i] || capturing) {
+                    bytes = std::max(bytes, std::min(2 * cap[dev][i], (size_t)GROUP_BYTES));
+                } else {
+                    e = cudaDeviceSynchronize();
+                    if (e == cudaSuccess) e = cudaFree(buf[dev][i]);
+                }
+                buf[dev][i] = nullptr;
+                cap[dev][i] = 0;
+                captured[dev][i] = false;
+            }
+            if (e == cudaSuccess) e = cudaMalloc(&buf[dev][i], bytes);
+            if (e != cudaSuccess && bytes > need[i]) {
+                cudaGetLastError();
+                e = cudaMalloc(&buf[dev][i], bytes = need[i]);
+            }
+            cudaThreadExchangeStreamCaptureMode(&mode);
+            if (e != cudaSuccess) {
+                cudaGetLastError();
+                buf[dev][i] = nullptr;
+                kq_set_error("gemm: cudaMalloc(%zu) failed: %s", need[i], cudaGetErrorString(e));
+                return B200_ERR_ALLOC;
+            }
+            cap[dev][i] = bytes;
         }
-        cudaThreadExchangeStreamCaptureMode(&mode);
-        if (e != cudaSuccess) {
-            cudaGetLastError();
-            kq_set_error("gemm: cudaMalloc(%zu) failed: %s", need[i], cudaGetErrorString(e));
-            return B200_ERR_ALLOC;
-        }
-        buf[dev][i] = b;
-        cap[dev][i] = bytes;
+        if (need[i] && capturing) captured[dev][i] = true;
     }
     if (!attr[dev]) {
         cudaFuncAttributes a4, a6;
@@ -836,11 +857,14 @@ b200_status scratch(int dev, size_t img16_bytes, size_t img8_bytes, size_t da_by
     return B200_OK;
 }
 
-// images of m_pad tokens in the forms that the matrices read
-b200_status scratch_for(int dev, const KqGemvSeg *segs, int nseg, int64_t m_pad, int64_t nb, Scratch *out) {
-    bool q4 = false, q6 = false;
-    for (int i = 0; i < nseg; i++) (segs[i].type == B200_TYPE_Q4_K ? q4 : q6) = true;
-    return scratch(dev, q4 ? (size_t)(m_pad * nb * TOK16) : 0, q6 ? (size_t)(m_pad * nb * TOK8) : 0, (size_t)(m_pad * nb * 4), out);
+// bytes of a token's images in the forms that the matrices read
+int64_t token_bytes(const KqGemvSeg *segs, int nseg, int64_t nb, bool q6) {
+    for (int i = 0; i < nseg; i++)
+        if ((segs[i].type == B200_TYPE_Q6_K) == q6) return nb * (q6 ? TOK8 : TOK16);
+    return 0;
+}
+b200_status scratch_for(int dev, const KqGemvSeg *segs, int nseg, int64_t m_pad, int64_t nb, cudaStream_t st, Scratch *out) {
+    return scratch(dev, (size_t)(m_pad * token_bytes(segs, nseg, nb, false)), (size_t)(m_pad * token_bytes(segs, nseg, nb, true)), (size_t)(m_pad * nb * 4), st, out);
 }
 
 b200_status add_seg(Params &p, int i, const KqGemvSeg &g, int64_t experts, int64_t K) {
@@ -952,7 +976,7 @@ int kq_gemm_error_fetch() {
 
 // Tokens whose images are held at a time: every row tile reads the images again, so they should stay in L2 (126 MB) beside the weights that
 // stream by.  2048 and 4096 tokens x 8192 x 28672 in Q4_K, 125 and 250 MB at once: 1363 and 2788 us; in slabs of 62 MB 1200 and 2406.
-constexpr int64_t SLAB_BYTES = 64 << 20, SLAB_MIN = MAX_CHUNKS * CHUNK;
+constexpr int64_t SLAB_MIN = MAX_CHUNKS * CHUNK;
 
 b200_status kq_launch_gemm_tc(const KqGemvSeg *segs, int nseg, const int8_t *q, const float *d, const int16_t *bs, int64_t M, int64_t K,
                               const float *residual, cudaStream_t st) {
@@ -960,10 +984,8 @@ b200_status kq_launch_gemm_tc(const KqGemvSeg *segs, int nseg, const int8_t *q, 
     KQ_TRY(check_segs(segs, nseg, q, K, &dev));
     KQ_REQUIRE(M > 0 && (!residual || nseg == 1), "gemm: bad shape");
     const int64_t nb = K / 256;
-    int64_t token_bytes = 0;
-    for (const uint32_t type : {(uint32_t)B200_TYPE_Q4_K, (uint32_t)B200_TYPE_Q6_K})
-        if (token_tiles_of(type, segs, nseg, M, nb).n) token_bytes += nb * (type == B200_TYPE_Q4_K ? TOK16 : TOK8);
-    const int64_t slab = std::max(SLAB_MIN, SLAB_BYTES / token_bytes / SLAB_MIN * SLAB_MIN);
+    const int64_t per_token = token_bytes(segs, nseg, nb, false) + token_bytes(segs, nseg, nb, true);
+    int64_t slab = std::max(SLAB_MIN, SLAB_BYTES / per_token / SLAB_MIN * SLAB_MIN);
     for (int64_t m0 = 0, mc; m0 < M; m0 += mc) {
         mc = kq_div_up(M - m0, kq_div_up(M - m0, slab)); // of equal size
         if (mc < M - m0) mc = kq_div_up(mc, SLAB_MIN) * SLAB_MIN;
@@ -974,8 +996,14 @@ b200_status kq_launch_gemm_tc(const KqGemvSeg *segs, int nseg, const int8_t *q, 
             p.m_pad = std::max(p.m_pad, t.n * t.tok);
         }
         Scratch sc;
-        KQ_TRY(scratch_for(dev, segs, nseg, p.m_pad, nb, &sc));
-        const ImageParams ip = {q + m0 * K, d + m0 * nb, bs + m0 * nb * 16, sc.img16, sc.img8, sc.da, (int32_t)mc, (int32_t)nb, p.m_pad, 1, nullptr, nullptr, nullptr};
+        const b200_status rc = scratch_for(dev, segs, nseg, p.m_pad, nb, st, &sc);
+        if (rc == B200_ERR_ALLOC && mc > SLAB_MIN) { // no room for these images: fewer at a time
+            slab = kq_div_up(mc, 2 * SLAB_MIN) * SLAB_MIN;
+            mc = 0;
+            continue;
+        }
+        KQ_TRY(rc);
+        const ImageParams ip = {q + m0 * K, d + m0 * nb, bs + m0 * nb * 16, sc.img16, sc.img8, sc.da, (int32_t)mc, (int32_t)nb, p.m_pad, 1, nullptr, nullptr, nullptr, 0};
         KQ_CUDA(kq_launch(act_image_kernel, dim3((unsigned)(p.m_pad / 16), (unsigned)nb), dim3(288), 0, st, ip));
         KQ_COUNT_LAUNCH();
         KqGemvSeg sg[MAX_SEGS];
@@ -1022,13 +1050,25 @@ b200_status kq_launch_gemm_grouped(const KqGemvSeg *segs, int nseg, const int8_t
         KQ_REQUIRE(segs[i].expert_stride == kq_device_row_bytes(segs[i].type, K) * segs[i].n_rows && segs[i].expert_stride % 16 == 0,
                    "grouped gemm: expert matrices must be contiguous and 16-byte aligned");
     const int64_t nb = K / 256, mt = moe_max_tiles(n_pairs, E);
-    Params p = {};
-    p.M = p.m_pad = (int32_t)(mt * TM), p.nb = (int32_t)nb, p.tok_tiles = (int)mt;
-    Scratch sc;
-    KQ_TRY(scratch_for(dev, segs, nseg, p.m_pad, nb, &sc));
-    p.n_tiles = sorted, p.tile_expert = sorted + 1, p.row_src = sorted + 1 + mt, p.tile_count = sorted + 1 + mt + mt * TM;
-    const ImageParams ip = {q, d, bs, sc.img16, sc.img8, sc.da, 0, (int32_t)nb, p.m_pad, act_div, p.row_src, p.tile_count, p.n_tiles};
-    KQ_CUDA(kq_launch(act_image_kernel, dim3((unsigned)(p.m_pad / 16), (unsigned)nb), dim3(288), 0, st, ip));
-    KQ_COUNT_LAUNCH();
-    return launch_segs(p, sc, segs, nseg, E, K, st);
+    const int64_t per_token = token_bytes(segs, nseg, nb, false) + token_bytes(segs, nseg, nb, true);
+    int64_t slab = std::max<int64_t>(1, GROUP_BYTES / (per_token * TM));
+    for (int64_t t0 = 0, tc; t0 < mt; t0 += tc) {
+        tc = kq_div_up(mt - t0, kq_div_up(mt - t0, slab));
+        Params p = {};
+        p.M = p.m_pad = (int32_t)(tc * TM), p.nb = (int32_t)nb, p.tok_tiles = (int)tc, p.first_tile = (int)t0;
+        Scratch sc;
+        const b200_status rc = scratch_for(dev, segs, nseg, p.m_pad, nb, st, &sc);
+        if (rc == B200_ERR_ALLOC && tc > 1) {
+            slab = kq_div_up(tc, 2);
+            tc = 0;
+            continue;
+        }
+        KQ_TRY(rc);
+        p.n_tiles = sorted, p.tile_expert = sorted + 1 + t0, p.row_src = sorted + 1 + mt + t0 * TM, p.tile_count = sorted + 1 + mt + mt * TM + t0;
+        const ImageParams ip = {q, d, bs, sc.img16, sc.img8, sc.da, 0, (int32_t)nb, p.m_pad, act_div, p.row_src, p.tile_count, p.n_tiles, p.first_tile};
+        KQ_CUDA(kq_launch(act_image_kernel, dim3((unsigned)(p.m_pad / 16), (unsigned)nb), dim3(288), 0, st, ip));
+        KQ_COUNT_LAUNCH();
+        KQ_TRY(launch_segs(p, sc, segs, nseg, E, K, st));
+    }
+    return B200_OK;
 }

@@ -232,3 +232,80 @@ def test_greedy_token(n):
         capi.check(L.b200_logit_signals(capi.ptr(xd), 5, n, None, None, capi.ptr(out), capi.ptr(scratch), scratch.numel(), capi.cur_stream()))
     got = out.cpu().numpy()
     assert np.array_equal(got, [int(np.argmax(np.where(np.isnan(r), -np.inf, r))) for r in x])
+
+
+MEMORY = """
+import torch
+from mesh_llm_b200 import capi, ops
+from oracle import binding as orc
+
+def free():
+    torch.cuda.synchronize()
+    return torch.cuda.mem_get_info()[0]
+
+def product(M, K, N=128):
+    W = torch.zeros(N * K // 256 * 144, dtype=torch.uint8, device="cuda")
+    q, d = torch.ones((M, K), dtype=torch.int8, device="cuda"), torch.ones((M, K // 256), device="cuda")
+    bs, y = torch.full((M, K // 16), 16, dtype=torch.int16, device="cuda"), torch.full((M, N), 7.0, device="cuda")
+    return lambda: ops.mul_mat_q8(orc.TYPE_Q4_K, W, q, d, bs, N, K, out=y)
+
+MB = 1 << 20
+first = product(16, 256)
+first()
+"""
+GROWTH = MEMORY + """
+calls = [product(M, 8192) for M in (256, 512, 1024, 2048, 3000)]
+before = free()
+for c in calls:
+    c()
+used = before - free()
+# 3000 tokens x 32 blocks x 544 bytes and their scales, in allocations of 2 MB
+assert used <= 3000 * 32 * (544 + 4) + 6 * MB, used
+"""
+NO_ROOM = MEMORY + """
+import ctypes
+c = product(3000, 8192)
+cu, at = ctypes.CDLL("libcuda.so.1"), ctypes.c_uint64()
+take = lambda n: cu.cuMemAlloc_v2(ctypes.byref(at), ctypes.c_size_t(n)) == 0
+assert take(16 * MB)
+hole, size = at.value, 1 << 34
+while size >= 2 * MB:
+    if not take(size):
+        size //= 2
+assert cu.cuMemFree_v2(ctypes.c_uint64(hole)) == 0 and not take(3000 * 32 * 544)
+y = c()
+torch.cuda.synchronize()
+assert capi.lib().b200_check_device_waits() == 0 and bool((y == 0).all())
+"""
+
+
+@pytest.mark.parametrize("script", [GROWTH, NO_ROOM], ids=["growth", "no_room"])
+def test_memory_of_images(script):
+    """calls of growing size leave the device with the largest one's images, not with all of them; and where the images of a call do not fit,
+    it takes fewer tokens at a time"""
+    import os
+    import subprocess
+    import sys
+
+    r = subprocess.run([sys.executable, "-c", script], cwd=os.path.join(os.path.dirname(__file__), ".."), capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stderr[-2000:]
+
+
+def test_experts_in_slabs():
+    """images of more than 256 MB: the tiles of the routed pairs in several launches"""
+    import torch
+
+    from mesh_llm_b200 import capi, ops
+
+    ty, rows, ku, E, N, K = orc.TYPE_Q4_K, 1200, 8, 256, 128, 7168
+    rng = np.random.default_rng(13)
+    W = np.tile(blocks_of(ty, 2 * N, K, 14), (E // 2, 1))  # two matrices in turn
+    x = rng.standard_normal((rows, K)).astype(np.float32)
+    ids = rng.integers(0, E, rows * ku).astype(np.int32)
+    dev, xd = ops.upload_weights(ty, W, E * N, K), torch.from_numpy(x).cuda()
+    got = ops.mul_mat_id(ty, dev, E, xd, torch.from_numpy(ids).cuda(), N, K).cpu().numpy()
+    assert capi.lib().b200_check_device_waits() == 0
+    for e in (0, 1, 100, 201, 254, 255):
+        at = np.nonzero(ids == e)[0]
+        want, size = exact(ty, W[e * N:(e + 1) * N], x[at // ku], N, K)
+        check(got[at], want, size, K)
