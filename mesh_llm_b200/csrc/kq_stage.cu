@@ -65,8 +65,10 @@ __global__ void __launch_bounds__(128) router_logits_kernel(const float *W, cons
 
 // The same for many tokens, sum for sum (a lane's terms and the order of the lanes' sums are those above): a warp takes 8 tokens x 8
 // experts, so that 16 loads feed 64 products instead of 2 one.  1024 tokens x 128 experts x 2048: 128 -> 46 us (what is left
-// is the reading of both operands out of L2, 268 MB by 14 warps an SM).  Below 64 tokens there are too few such warps.
-constexpr int ROUTER_TILE = 8, ROUTER_MIN_T = 64;
+// is the reading of both operands out of L2, 268 MB by 14 warps an SM).  A warp takes 12, 21 or 33 us for rows of 2048, 4096 or 7168, so it wants
+// more than one of them per SM: 128 tiles take 12 / 21 / 33 us where a warp per pair takes 10 / 16 / 25 (64 experts at 128 tokens, 8 at 1024), 256 tiles
+// take as long as 128 and the warps per pair 14 / 23 / 37.
+constexpr int ROUTER_TILE = 8, ROUTER_MIN_TILES = 256;
 __global__ void __launch_bounds__(128) router_logits_tile_kernel(const float *W, const float *x, int T, int E, int h, float *out) {
     KQ_PDL_ENTER();
     const int lane = threadIdx.x & 31, e_tiles = (E + ROUTER_TILE - 1) / ROUTER_TILE;
@@ -322,8 +324,8 @@ b200_status forward_body(b200_stage *st, const int32_t *tokens, const float *hid
             if (!fused_small) {
             OTHER_(kq_rms_norm(st->x, L.ffn_norm, rows, h, c.rms_eps, st->xn, st->aq, st->ad, st->abs16, s));
             if (classes & CLS_OTHER) {
-            if (rows >= ROUTER_MIN_T)
-                kq_launch(router_logits_tile_kernel, (unsigned)kq_div_up(kq_div_up(rows, ROUTER_TILE) * kq_div_up(E, ROUTER_TILE), 4), 128, 0, s,
+            if (const int64_t tiles = kq_div_up(rows, ROUTER_TILE) * kq_div_up(E, ROUTER_TILE); tiles >= ROUTER_MIN_TILES)
+                kq_launch(router_logits_tile_kernel, (unsigned)kq_div_up(tiles, 4), 128, 0, s,
                           L.router, st->xn, rows, E, h, st->rl);
             else
                 kq_launch(router_logits_kernel, (unsigned)kq_div_up((int64_t)rows * E, 4), 128, 0, s, L.router, st->xn, rows, E, h, st->rl);

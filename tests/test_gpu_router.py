@@ -1,0 +1,33 @@
+"""The router of a micro-batch in its two forms: tiles of 8 tokens x 8 experts per warp from 256 tiles on, a warp per pair below."""
+import numpy as np
+import pytest
+
+from oracle import binding as orc
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("E,T", [(20, 1030), (8, 2049), (130, 129)])
+def test_both_forms_route_alike(E, T):
+    """one layer of experts over T tokens at once (tiles, the last ones of them part empty) and in four parts (warps per pair).  The logits of the two
+    forms are equal sum for sum, so a token takes the same experts.  What differs are sums of the products in another order, which put Q8 codes beside a
+    tie on its other side: one code in a hundred moved by 1 / 127 of a block's largest value, which is about three times its rms, is 2.4e-3 of a row, in
+    each of the layer's four quantisers.  A wrong expert moves a row by its whole expert part"""
+    import torch
+
+    from mesh_llm_b200.stage import Stage
+
+    cfg = dict(n_layer=1, n_embd=512, n_head=8, n_head_kv=2, head_dim=64, n_ff=0, n_vocab=256, n_ctx=2304, n_expert=E, n_expert_used=4, n_ff_exp=256, qk_norm=1)
+    part = dict(layer_begin=0, layer_end=1, has_embd=0, has_output=0)
+    m = orc.Model(**cfg)
+    m.generate(3)
+    st = Stage(**cfg, **part, n_ubatch=T)
+    for n in orc.Model(**cfg, **part).tensor_names():
+        st.set_tensor(n, *m.tensor(n)[:2])
+    x = torch.from_numpy(np.random.default_rng(E).standard_normal((T, cfg["n_embd"])).astype(np.float32)).cuda()
+    whole = st.forward(hidden_in=x, n_seq=1, T=T, pos0=0)[0].double().clone()
+    step = -(-T // 4)
+    parts = torch.cat([st.forward(hidden_in=x[i:i + step].contiguous(), n_seq=1, T=min(step, T - i), pos0=i)[0].double().clone() for i in range(0, T, step)])
+    st.close()
+    change = whole - x.double()  # what the layer adds
+    assert float((whole - parts).norm(dim=1).max() / change.norm(dim=1).mean()) <= 2e-2
