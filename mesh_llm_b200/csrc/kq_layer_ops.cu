@@ -245,8 +245,12 @@ __device__ __forceinline__ void rec_coeff(float r, float i, float u, float decay
 constexpr int RC = 128, RCHUNK = 16, RCHUNKS = 64; // channels per CTA, positions per chunk at least, chunks at most
 // Positions per chunk.  A thread's walk through its chunk is a chain of dependent steps, and many short chunks hide it; the second pass reads the
 // maps of all chunks in front of its own, so there are not more than 64 of them (a call of 1000 x 3072: 16 chunks of 64 positions
-// take 49 + 42 us, 63 of 16 take 19 + 20).
-__host__ inline int rec_chunk(int T) { return std::max(RCHUNK, (int)kq_div_up(kq_div_up(T, RCHUNKS), RCHUNK) * RCHUNK); }
+// take 49 + 42 us, 63 of 16 take 19 + 20), and not more than 512 over all sequences, where the other sequences hide the chain as well (16 sequences of 1000 x
+// 2560: 362 -> 349, 347 as 16 chunks of 64).
+__host__ inline int rec_chunk(int T, int n_seq) {
+    const int chunks = std::max(8, std::min(RCHUNKS, 512 / n_seq));
+    return std::max(RCHUNK, (int)kq_div_up(kq_div_up(T, chunks), RCHUNK) * RCHUNK);
+}
 __global__ void __launch_bounds__(RC) recurrence_chunks_kernel(const __grid_constant__ KqRecW w, KqRecState st, float *r, float *ig, int64_t ldr, const float *u,
                                                                int64_t ldu, int T, const int32_t *pos0_dev, int pos0_val, int chunk, float *maps) {
     KQ_PDL_ENTER();
@@ -449,7 +453,7 @@ b200_status kq_linear_recurrence(const KqRecW &w, const KqRecState &s, float *r,
                                  float *scratch, size_t scratch_bytes, cudaStream_t st) {
     const b200_status rc = check_rec(w, n_seq, T);
     if (rc != B200_OK) return rc;
-    const int chunk = rec_chunk(T);
+    const int chunk = rec_chunk(T, n_seq);
     const unsigned chunks = (unsigned)kq_div_up(T, chunk);
     KQ_REQUIRE(scratch && scratch_bytes >= (size_t)n_seq * (chunks + 1) * 2 * w.width * 4, "recurrence: scratch");
     const int64_t cols = z16 ? std::max<int64_t>(w.width, ld16) : w.width;
