@@ -388,11 +388,11 @@ b200_status kq_gemm_bf16(const KqDense &c, const uint16_t *a, int64_t lda, int p
         return t;
     };
     const int64_t sms = kq_sm_count();
-    const int64_t w256 = kq_div_up((int64_t)p.mt * n_tiles(256) * c.groups, sms) * 20, w128 = kq_div_up((int64_t)p.mt * n_tiles(128) * c.groups, sms) * 13,
-                  w64 = kq_div_up((int64_t)p.mt * n_tiles(64) * c.groups, sms) * 9;
-    // 192 rows fill waves that 256 leave part empty (1000 tokens x 3072 rows: 128 tiles instead of 96 on 148 SMs; with K = 9216 74 -> 67 us, with K = 3072 36 -> 32; 6144 rows 61 -> 51)
-    const int64_t w192 = kq_div_up((int64_t)p.mt * n_tiles(192) * c.groups, sms) * 16;
-    const int tn = w256 <= w192 && w256 <= w128 && w256 <= w64 ? 256 : w192 <= w128 && w192 <= w64 ? 192 : w128 <= w64 ? 128 : 64;
+    // A wave of each width by its measured share of one of 256 rows (12288 x 4096 at 2048 tokens: 6 waves of 256 rows 182 us, 7 of 192 190).  192 rows fill waves that
+    // 256 leave part empty: 1000 tokens x 3072 rows are 128 tiles instead of 96 on 148 SMs (K = 9216 74 -> 67 us, K = 3072 36 -> 32; 6144 rows 61 -> 51)
+    auto waves = [&](int rows) { return kq_div_up((int64_t)p.mt * n_tiles(rows) * c.groups, sms); };
+    const int64_t cost[4] = {waves(256) * 40, waves(192) * 36, waves(128) * 26, waves(64) * 18};
+    const int width[4] = {256, 192, 128, 64}, tn = width[std::min_element(cost, cost + 4) - cost];
     p.nt = n_tiles(tn);
     {
         const uint64_t dims[3] = {(uint64_t)lda, (uint64_t)c.M, (uint64_t)parts};
