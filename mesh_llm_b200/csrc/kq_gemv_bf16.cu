@@ -18,6 +18,7 @@ namespace {
 
 constexpr int NT = 256, NW = NT / 32, SB = 64; // threads, warps, rows between two combines
 constexpr int MAX_X_BYTES = 192 * 1024;       // activations in shared memory, next to 32 KB of partial sums at 8 rows
+constexpr size_t SM_BYTES = 228 * 1024, CTA_BYTES = 1024; // shared memory of an SM, and what the system takes of it for each CTA
 
 struct GemvParams {
     KqDense c;
@@ -242,12 +243,15 @@ __global__ void __launch_bounds__(NT) gemv_grouped_bf16_kernel(const __grid_cons
 
 template <int M>
 b200_status launch_gemv(const GemvParams &p, size_t smem, cudaStream_t st) {
-    static bool attr[16];
+    static int regs_fit[16]; // CTAs of an SM by registers and threads; 0: not asked yet
     int dev = 0;
     KQ_CUDA(cudaGetDevice(&dev));
-    if (dev < 0 || dev >= 16 || !attr[dev]) {
+    int fit = dev >= 0 && dev < 16 ? regs_fit[dev] : 0;
+    if (!fit) { // (asking for the occupancy at this call's shared memory would cost every launch a call of the runtime)
         KQ_CUDA(cudaFuncSetAttribute(gemv_bf16_kernel<M>, cudaFuncAttributeMaxDynamicSharedMemorySize, MAX_X_BYTES));
-        if (dev >= 0 && dev < 16) attr[dev] = true;
+        KQ_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit, gemv_bf16_kernel<M>, NT, 0));
+        fit = std::max(1, fit);
+        if (dev >= 0 && dev < 16) regs_fit[dev] = fit;
     }
     static int mul = -1; // B200_GEMV16_CTAS: CTAs per SM of the decode projections
     if (mul < 0) {
@@ -258,8 +262,7 @@ b200_status launch_gemv(const GemvParams &p, size_t smem, cudaStream_t st) {
     const int64_t want = std::max<int64_t>(1, kq_div_up(units * (p.c.glu ? 2 : 1), 4));
     // no more CTAs than run at the same time: every one prepares the activations for itself, and 8 rows of 3072 leave room for one per SM
     // (8 rows, 2 x 9216 rows of weights of 3072: 153 us in four waves, 92 in one)
-    int fit = 1;
-    KQ_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit, gemv_bf16_kernel<M>, NT, smem));
+    fit = std::min<int>(fit, (int)(SM_BYTES / (smem + sizeof(float) * (2 * NW * SB * M + NW) + CTA_BYTES)));
     const unsigned grid = (unsigned)std::min<int64_t>(want, (int64_t)kq_sm_count() * std::max(1, std::min(mul, fit)));
     kq_launch(gemv_bf16_kernel<M>, grid, NT, smem, st, p);
     KQ_COUNT_LAUNCH();
