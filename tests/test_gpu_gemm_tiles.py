@@ -197,7 +197,7 @@ def test_norm_of_short_rows(h):
 @pytest.mark.parametrize("M", [300, 900, 1000])
 @pytest.mark.parametrize("N,K", [(3072, 128), (3000, 200), (6200, 64)])
 def test_bf16_tiles(M, N, K):
-    """sizes that choose every tile width, the one of 192 rows among them; bf16 operands, f32 sums of at most 200 terms (truncating: 2^-22 each)"""
+    """sizes around the tiles (every width: test_gpu_bf16_tiles.py); bf16 operands, f32 sums of at most 200 terms (truncating: 2^-22 each)"""
     import torch
 
     from mesh_llm_b200 import ops

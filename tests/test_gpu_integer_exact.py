@@ -10,7 +10,7 @@ accumulation), and it must equal the CPU oracle's int32 block sums bit for bit.
 
 Token counts select the kernels: M = 1, 2 the streaming decode GEMV (gemv_block_kernel<type, 1|2>),
 M = 3..8 its mma.m16n8k32 batch form (Q4_K) or the dp4a kernel (Q6_K), M > 8 the tcgen05 prefill
-GEMM with its two-plane recombination (from 384 tokens on in its form with pre-unpacked operand images).
+GEMM (9, 130 and 390 tokens: one token tile and several; sums above 2^24 in test_gpu_gemm_tiles.py).
 """
 import numpy as np
 import pytest
