@@ -349,7 +349,7 @@ b200_status forward_body(b200_stage *st, const int32_t *tokens, const float *hid
                 const char *v = getenv("B200_MOE_GROUPED");
                 grouped_on = !(v && v[0] == '0');
             }
-            bool grouped = grouped_on && rows > 8 && fe % 64 == 0 && h % 64 == 0 && classes == CLS_ALL;
+            bool grouped = grouped_on && rows > 8 && classes == CLS_ALL;
             if (grouped) {
                 KQ_TRY(kq_moe_sort(st->rid, pairs, E, st->moe_sorted, st->moe_sorted_bytes, s));
                 const KqGemvSeg both[2] = {gu[0], {gu[1].W, gu[1].type, fe, st->hp2, nullptr, fe, kq_device_row_bytes(gu[1].type, h) * fe}};
