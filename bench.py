@@ -760,8 +760,8 @@ def prefill_gemm_roofline():
     """The prefill GEMM against a tensor-core ceiling measured in the same run: the useful int8 rate
     (2 M N K per launch) of the 32B shape's FFN matmuls at M = 2048, and a bare loop of the kernel's own
     tcgen05.mma kind::i8 instruction on all SMs (b200_probe_int8_mma).  The kernel folds the sub-block
-    scale into the weight and multiplies in f16 (Q6_K: as two addends), which takes the tensor core as long as two int8
-    products, so the rate that is compared is twice the useful one."""
+    scale into the weight and multiplies once in f16 (Q4_K), which takes the tensor core as long as two int8 products, or in two planes
+    of int8 (Q6_K), so the rate that is compared is twice the useful one."""
     from mesh_llm_b200 import ops
 
     peak, _ = ops.probe_int8_mma(65536, 5)

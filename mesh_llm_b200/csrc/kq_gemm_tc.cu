@@ -24,8 +24,10 @@
 // tile; nobody waits, and no barrier stands between a wait that can give up and the end of the kernel.
 //
 // What bounds it, in clocks per block of 128 rows x 256 tokens: the MMAs 2900 in either type (42 each at N = 64, where 32 would be the tensor
-// rate), the drains about 1000 of every scheduler.  Measured about 5500 for 256 tokens and 2600 (Q4_K) or 4000 (Q6_K) for 16, where the decoding is
-// what is left: one warp of each scheduler walks through it.  The same decoding unrolled four times made the whole kernel 10 % slower.
+// rate), the drains about 1000 of every scheduler.  Measured about 5500 for 256 tokens, where no unit is near its limit (of the clocks the tensor pipe is
+// active in 38 % for Q4_K and 31 % for Q6_K, the schedulers issue in 58 % and 64 %): what is left are the hand-overs between the roles.  With 16 tokens
+// about 2600 (Q4_K) or 4200 (Q6_K), the decoding: one warp of each scheduler walks through it.  The same decoding unrolled four times
+// made the whole kernel 10 % slower.
 // Q4_K: two int8 planes per weight out of shared memory (the form before this one) took 1659 us where this takes 1204, for 2048 tokens x 28672 x
 // 8192, 547 against 317 at 512 tokens, 169 against 67 at 16 (without the k_j, exact below 2^24 only: 1201, 316, 66).  Q6_K, whose two planes came from shared memory as well: 1637 against 1324,
 // 624 against 351, 248 against 110; as two f16 addends into one f32 accumulator, with the decoded operand in a single buffer, it
