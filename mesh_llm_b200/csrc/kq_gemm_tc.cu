@@ -14,8 +14,10 @@
 // up to 64.  Packed blocks arrive by TMA; a warpgroup (a thread per row) decodes them into TMEM, two bytes per weight in both types, from where
 // the MMAs take them as their A operand, so that decoded weights never pass through shared memory.  The token operand is an image that
 // act_image_kernel writes (f16 codes and sums of 16 for Q4_K, the codes themselves for Q6_K): one bulk copy per chunk and block.  Two warps issue MMAs in turn, each with an accumulator of its own;
-// two warpgroups drain the accumulators into the running f32 result, which stays in registers for the whole tile.  Lanes of a
+// the draining warps add the accumulators to the running f32 result, which stays in registers for the whole tile.  Lanes of a
 // warp hold neighbouring rows of W, so results leave in full lines.
+// With tiles of two or four chunks one warpgroup decodes and two drain, half of every chunk each.  Narrow tiles are one chunk: their blocks take the decoding longer
+// than anything else, so two warpgroups decode, block by block in turn, and one drains.
 //
 // Up to three matrices that read the same tokens (q / k / v, gate / up) share the image and, type by type, the launch: the small ones would
 // leave most of the GPU idle (256 x 2048 at 77 tokens: 19 us alone, two of them in the launch of q: none).
@@ -23,11 +25,14 @@
 // that was cut is added up, in the order of its parts, by the CTA that arrives last, each draining warp its own rows and tokens of the
 // tile; nobody waits, and no barrier stands between a wait that can give up and the end of the kernel.
 //
-// What bounds it, in clocks per block of 128 rows x 256 tokens: the MMAs 2900 in either type (42 each at N = 64, where 32 would be the tensor
-// rate), the drains about 1000 of every scheduler.  Measured about 5500 for 256 tokens, where no unit is near its limit (of the clocks the tensor pipe is
-// active in 38 % for Q4_K and 31 % for Q6_K, the schedulers issue in 58 % and 64 %): what is left are the hand-overs between the roles.  With 16 tokens
-// about 2600 (Q4_K) or 4200 (Q6_K), the decoding: one warp of each scheduler walks through it.  The same decoding unrolled four times
-// made the whole kernel 10 % slower.
+// What bounds it.  Wide tiles: a chunk of 64 tokens takes 756 clocks of MMAs in either type (18 of 42; 32 would be the tensor rate) and about 1000 in fact: an accumulator
+// goes round MMAs, drain (300) and two hand-overs, and TMEM has room for two beside the two decoded blocks.  28672 x 8192 at 512 tokens: 250 us in Q4_K (960 TFLOP/s),
+// 271 in Q6_K; 316 and 349 while the loop over the blocks also held the end of the tile and unrolled chunks, whose turn cost a draining warp a thousand clocks beside
+// the additions, and while it waited for the scales' barriers beside the accumulator's.  Narrow tiles: the decoding, 1100 clocks a block and warpgroup in Q4_K and twice that in Q6_K, and
+// the way of a decoded block's place through decoding and MMAs: 16 tokens 49 us in Q4_K, 78 in Q6_K (one decoding warpgroup: 67 and 110), 64 tokens 58 and 87 (78 and 117).
+// A thread takes all its codes into registers before it waits for the place of the decoded block (64 tokens 68 -> 64 us), and stores of 16 registers let the next
+// ones be computed meanwhile.  A wait tries its barrier 64 times before it looks at the clock (250 against 255 us).  Not kept: chunks to the draining warpgroups in turn (263), a
+// packed block's place given back as soon as its codes are in registers (64 -> 68 us with 64 tokens), sleeps between tries.
 // Q4_K: two int8 planes per weight out of shared memory (the form before this one) took 1659 us where this takes 1204, for 2048 tokens x 28672 x
 // 8192, 547 against 317 at 512 tokens, 169 against 67 at 16 (without the k_j, exact below 2^24 only: 1201, 316, 66).  Q6_K, whose two planes came from shared memory as well: 1637 against 1324,
 // 624 against 351, 248 against 110; as two f16 addends into one f32 accumulator, with the decoded operand in a single buffer, it
@@ -49,10 +54,16 @@ constexpr int TOK16 = 544, TOK8 = 256;
 constexpr int TILE_OUT = MAX_CHUNKS * CHUNK * ROWS; // outputs of a tile
 constexpr int MAX_CTAS = 256, MAX_DEVICES = 16, DRAIN_WARPS = 8;
 constexpr uint64_t LIMIT = 5 * KQ_WAIT_LIMIT_NS;
-constexpr int REG_EPI = 208, REG_UNPACK = 56, REG_REST = 40; // 2 x 208 + 56 + 40 = 512 = 4 x 128
 
-template <bool Q6>
+// NARROW: tiles of one chunk.  Their blocks take the decoding longer than anything else, so two warpgroups decode, block by block in turn, and one drains;
+// otherwise one decodes and each of two drains half of every chunk.
+template <bool Q6, bool NARROW>
 struct Cfg {
+    static constexpr int DRAIN_WG = NARROW ? 1 : 2, DECODE_WG = 3 - DRAIN_WG;
+    static constexpr int GROUPS = NARROW ? 4 : 8; // groups of 16 tokens whose results a draining thread holds
+    static constexpr int REG_DRAIN = NARROW ? 184 : 208, REG_DECODE = NARROW ? 144 : 56, REG_REST = 40;
+    static constexpr int REG_SUM = DRAIN_WG * REG_DRAIN + DECODE_WG * REG_DECODE + REG_REST;
+    static_assert(REG_SUM <= 512, "registers of 512 threads, 128 each at the launch");
     static constexpr int RAW_BYTES = Q6 ? 13 * ROWS * 32 : ROWS * KQ_Q4K_BYTES; // Q6_K: two blocks of each row
     static constexpr int TOK_BYTES = Q6 ? TOK8 : TOK16, B_BYTES = CHUNK * TOK_BYTES;
     static constexpr int RAW_STAGES = Q6 ? 2 : 3, B_STAGES = Q6 ? 6 : 4;
@@ -63,7 +74,7 @@ struct Cfg {
     static_assert(SMEM <= 226 * 1024, "shared memory of a CTA");
     // the two issuing warps take alternate chunks: with an even number a stage is always the same warp's, which then waits for every phase of it
     static_assert(B_STAGES % 2 == 0, "a wait by parity must not miss a phase");
-    // chunk q - 2 has been drained when chunk q is issued, and a stage is filled again when its chunk's MMAs are over: what the rings without
+    // the one before it on its accumulator, q - 2, has been drained when chunk q is issued, and a stage is filled again when its chunk's MMAs are over: what the rings without
     // barriers of their own rely on
     static_assert(DA_RING >= B_STAGES + 2 && SC_RING >= 4, "rings");
 };
@@ -89,13 +100,14 @@ struct Params {
     const float *residual; // with one matrix only
     int32_t M, nb, m_pad, row_tiles, tok_tiles, tile_tok, min_share;
     int64_t w_row;
-    // products with experts: token tile t belongs to expert tile_expert[t] and holds the tile_count[t] pairs row_src[128 t ..]
+    // products with experts: token tile t belongs to expert tile_expert[t] and holds the tile_count[t] pairs row_src[tile_tok t ..]
     const int32_t *row_src, *tile_expert, *tile_count, *n_tiles;
     int32_t first_tile; // of the token tiles that n_tiles counts, the one that is tile 0 of this launch
 };
 
-__host__ __device__ __forceinline__ void chunks_of(int n, int &c, int &cw) { // n tokens as c chunks of cw
-    c = (n + CHUNK - 1) / CHUNK;
+// n tokens as c chunks of cw: one, or an even number, so that each accumulator and its issuing warp have the chunks of one parity
+__host__ __device__ __forceinline__ void chunks_of(bool narrow, int n, int &c, int &cw) {
+    c = narrow ? 1 : n <= 2 * CHUNK ? 2 : 4;
     cw = ((n + c - 1) / c + 15) & ~15;
 }
 
@@ -104,17 +116,16 @@ struct TilePos {
 };
 // selects, not indexing: parameters indexed by a variable are read through generic loads
 __device__ __forceinline__ int seg_rows(const Params &p, int s) { return s == 0 ? p.seg[0].N : s == 1 ? p.seg[1].N : p.seg[2].N; }
+template <bool NARROW>
 __device__ __forceinline__ TilePos tile_at(const Params &p, int tile) {
     TilePos t;
     const int tt = tile / p.row_tiles, rt = tile - tt * p.row_tiles;
     t.seg = (rt >= p.seg[0].tile_end) + (rt >= p.seg[1].tile_end);
     t.n0 = (rt - (t.seg == 0 ? 0 : t.seg == 1 ? p.seg[0].tile_end : p.seg[1].tile_end)) * ROWS;
-    if (p.row_src) {
-        t.t0 = tt * 128, t.n = p.tile_count[tt], t.expert = p.tile_expert[tt];
-    } else {
-        t.t0 = tt * p.tile_tok, t.n = min(p.tile_tok, p.M - t.t0), t.expert = 0;
-    }
-    chunks_of(t.n, t.c, t.cw);
+    t.t0 = tt * p.tile_tok;
+    if (p.row_src) t.n = p.tile_count[tt], t.expert = p.tile_expert[tt];
+    else t.n = min(p.tile_tok, p.M - t.t0), t.expert = 0;
+    chunks_of(NARROW, t.n, t.c, t.cw);
     return t;
 }
 
@@ -128,6 +139,13 @@ __device__ __forceinline__ __half2 byte_pair(uint32_t v, int b) { return h2(__by
 // bytes b and b + 1 of v as f16
 __device__ __forceinline__ __half2 two_bytes(uint32_t v, int b) { return __hsub2(h2(__byte_perm(v, 0x64646464u, 0x4040u | ((b + 1) << 8) | b)), __float2half2_rn(1024.f)); }
 
+#define TMEM_LD8(taddr, r)                                                                                              \
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"                                \
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])       \
+                 : "r"(taddr)                                                                                           \
+                 : "memory")
+__device__ __forceinline__ void tmem_ld(uint32_t at, uint32_t (&r)[8]) { TMEM_LD8(at, r); }
+__device__ __forceinline__ void tmem_ld(uint32_t at, uint32_t (&r)[16]) { TMEM_LD16(at, r); }
 #define TMEM_ST4(taddr, r) \
     asm volatile("tcgen05.st.sync.aligned.32x32b.x4.b32 [%0], {%1,%2,%3,%4};" ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]) : "memory")
 
@@ -167,10 +185,14 @@ __device__ __forceinline__ bool try_wait(uint32_t bar, uint32_t parity, int lane
     return __all_sync(0xffffffffu, ok) != 0;
 }
 __device__ __forceinline__ bool wait_on(uint32_t bar, uint32_t parity, int lane, int n, volatile int *give_up, int code) {
-    if (try_wait(bar, parity, lane, n)) return true;
-    const uint64_t t0 = kq_globaltimer_ns();
-    while (!try_wait(bar, parity, lane, n)) {
-        const bool late = kq_globaltimer_ns() - t0 > LIMIT;
+    uint64_t t0 = 0;
+    while (true) {
+#pragma unroll 1
+        for (int i = 0; i < 64; i++)
+            if (try_wait(bar, parity, lane, n)) return true;
+        const uint64_t now = kq_globaltimer_ns();
+        if (!t0) t0 = now;
+        const bool late = now - t0 > LIMIT;
         if (__any_sync(0xffffffffu, *give_up || late)) {
             *give_up = 1;
             if (late) atomicExch(&g_gemm_error, code);
@@ -180,23 +202,23 @@ __device__ __forceinline__ bool wait_on(uint32_t bar, uint32_t parity, int lane,
     return true;
 }
 
-template <bool Q6>
+template <bool Q6, bool NARROW>
 __global__ void __launch_bounds__(NTHREADS, 1) gemm_kq_kernel(const __grid_constant__ Params p) {
-    using C = Cfg<Q6>;
+    using C = Cfg<Q6, NARROW>;
+    constexpr int RAW_FULL = !Q6 && NARROW ? 2 * C::RAW_STAGES : C::RAW_STAGES; // blocks decoded in turn: a barrier per stage and warpgroup, which then sees each phase of its own
     extern __shared__ __align__(1024) uint8_t smem[];
-    __shared__ uint64_t raw_full[C::RAW_STAGES], raw_empty[C::RAW_STAGES], b_full[C::B_STAGES], b_empty[C::B_STAGES];
-    __shared__ uint64_t da_full[DA_RING], sc_full[SC_RING], a_full[2], a_empty[2], acc_full[2], acc_empty[2], s_end[2];
+    __shared__ uint64_t raw_full[RAW_FULL], raw_empty[C::RAW_STAGES], b_full[C::B_STAGES], b_empty[C::B_STAGES];
+    __shared__ uint64_t a_full[2], a_empty[2], acc_full[2], acc_empty[2], s_end[2];
     __shared__ uint32_t s_tmem;
     __shared__ int s_abort;
     KQ_PDL_TRIGGER();
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     if (tid == 0) {
-        for (int i = 0; i < C::RAW_STAGES; i++) bar_init(&raw_full[i], 1), bar_init(&raw_empty[i], 4);
+        for (int i = 0; i < RAW_FULL; i++) bar_init(&raw_full[i], 1);
+        for (int i = 0; i < C::RAW_STAGES; i++) bar_init(&raw_empty[i], Q6 && NARROW ? 8 : 4); // Q6_K: both warpgroups read a pair of blocks
         for (int i = 0; i < C::B_STAGES; i++) bar_init(&b_full[i], 1), bar_init(&b_empty[i], 1);
-        for (int i = 0; i < DA_RING; i++) bar_init(&da_full[i], 1);
-        for (int i = 0; i < SC_RING; i++) bar_init(&sc_full[i], 4);
-        for (int i = 0; i < 2; i++)
-            bar_init(&a_full[i], 4), bar_init(&a_empty[i], 2), bar_init(&acc_full[i], 1), bar_init(&acc_empty[i], 8), bar_init(&s_end[i], 1);
+        for (int i = 0; i < 2; i++) // acc_full: the MMAs, and the issuing warp for the scales that it has waited for
+            bar_init(&a_full[i], 4), bar_init(&a_empty[i], NARROW ? 1 : 2), bar_init(&acc_full[i], 2), bar_init(&acc_empty[i], 4 * C::DRAIN_WG), bar_init(&s_end[i], 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         s_abort = 0;
     }
@@ -218,11 +240,11 @@ __global__ void __launch_bounds__(NTHREADS, 1) gemm_kq_kernel(const __grid_const
     auto wait = [&](uint64_t *bar, uint32_t parity, int code) { return wait_on(smem_u32(bar), parity, lane, 1, &s_abort, code); };
 
     if (warp >= 12) {
-        asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(REG_REST));
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(C::REG_REST));
         const bool lead = tc_elect();
         int tile = tile0, b = b0, k = 0;
         TilePos t = {};
-        if (total) t = tile_at(p, tile);
+        if (total) t = tile_at<NARROW>(p, tile);
         bool ok = true;
         if (warp == 12) { // packed weights
             for (int u = 0; u < total; u++) {
@@ -230,8 +252,9 @@ __global__ void __launch_bounds__(NTHREADS, 1) gemm_kq_kernel(const __grid_const
                     const int s = k % C::RAW_STAGES, round = k / C::RAW_STAGES;
                     if (round > 0 && !(ok = wait(&raw_empty[s], (round - 1) & 1, 1))) break;
                     if (lead) {
-                        bar_expect(&raw_full[s], C::RAW_BYTES);
-                        const uint32_t dst = smem_u32(smem + C::SM_RAW + s * C::RAW_BYTES), bar = smem_u32(&raw_full[s]);
+                        uint64_t *full = &raw_full[k % RAW_FULL];
+                        bar_expect(full, C::RAW_BYTES);
+                        const uint32_t dst = smem_u32(smem + C::SM_RAW + s * C::RAW_BYTES), bar = smem_u32(full);
                         const int row = t.expert * seg_rows(p, t.seg) + t.n0;
                         if (Q6) {
                             const int grp = b / KQ_Q6_GROUP, full = nb / KQ_Q6_GROUP, x = (b % KQ_Q6_GROUP) / 2 * 32;
@@ -250,11 +273,11 @@ __global__ void __launch_bounds__(NTHREADS, 1) gemm_kq_kernel(const __grid_const
                 }
                 if (++b == nb) {
                     b = 0;
-                    if (u + 1 < total) t = tile_at(p, ++tile);
+                    if (u + 1 < total) t = tile_at<NARROW>(p, ++tile);
                 }
             }
             if (!ok && lead) // copies that were posted must land before the CTA goes away
-                for (int i = max(0, k - C::RAW_STAGES); i < k; i++) kq_mbar_wait(smem_u32(&raw_full[i % C::RAW_STAGES]), (i / C::RAW_STAGES) & 1, KQ_WAIT_LIMIT_NS);
+                for (int i = max(0, k - C::RAW_STAGES); i < k; i++) kq_mbar_wait(smem_u32(&raw_full[i % RAW_FULL]), (i / RAW_FULL) & 1, KQ_WAIT_LIMIT_NS);
         } else if (warp == 13) { // token images and scales
             const int64_t block_bytes = (int64_t)p.m_pad * C::TOK_BYTES;
             for (int u = 0; u < total && ok; u++) {
@@ -263,38 +286,35 @@ __global__ void __launch_bounds__(NTHREADS, 1) gemm_kq_kernel(const __grid_const
                     if (round > 0 && !(ok = wait(&b_empty[s], (round - 1) & 1, 2))) break;
                     if (lead) {
                         const int tok = t.t0 + c * t.cw, d = k % DA_RING;
-                        bar_expect(&b_full[s], t.cw * C::TOK_BYTES);
+                        bar_expect(&b_full[s], t.cw * (C::TOK_BYTES + 4));
                         bulk_in(smem_u32(smem + C::SM_B + s * C::B_BYTES), p.img + b * block_bytes + (int64_t)tok * C::TOK_BYTES, t.cw * C::TOK_BYTES, &b_full[s]);
-                        bar_expect(&da_full[d], t.cw * 4);
-                        bulk_in(smem_u32(smem + C::SM_DA + d * CHUNK * 4), p.da + (int64_t)b * p.m_pad + tok, t.cw * 4, &da_full[d]);
+                        bulk_in(smem_u32(smem + C::SM_DA + d * CHUNK * 4), p.da + (int64_t)b * p.m_pad + tok, t.cw * 4, &b_full[s]);
                     }
                     __syncwarp();
                 }
                 if (++b == nb) {
                     b = 0;
-                    if (u + 1 < total) t = tile_at(p, ++tile);
+                    if (u + 1 < total) t = tile_at<NARROW>(p, ++tile);
                 }
             }
             if (!ok && lead)
-                for (int i = max(0, k - DA_RING); i < k; i++) {
-                    if (i >= k - C::B_STAGES) kq_mbar_wait(smem_u32(&b_full[i % C::B_STAGES]), (i / C::B_STAGES) & 1, KQ_WAIT_LIMIT_NS);
-                    kq_mbar_wait(smem_u32(&da_full[i % DA_RING]), (i / DA_RING) & 1, KQ_WAIT_LIMIT_NS);
-                }
-        } else { // MMAs: one warp waits while the other one issues
+                for (int i = max(0, k - C::B_STAGES); i < k; i++) kq_mbar_wait(smem_u32(&b_full[i % C::B_STAGES]), (i / C::B_STAGES) & 1, KQ_WAIT_LIMIT_NS);
+        } else { // MMAs: a warp per accumulator, for the chunks of its parity (NARROW: blocks of its parity)
             const int w = warp & 1;
+            int n = 0; // chunks this warp has issued
             for (int u = 0; u < total && ok; u++) {
                 const uint32_t id = Q6 ? idesc_i8(128, t.cw, true) : tc_idesc(128, t.cw, false, false), sa = u & 1, pa = (u >> 1) & 1;
-                for (int c = (k & 1) ^ w; c < t.c; c += 2) {
+                for (int c = NARROW ? (sa ^ w) : w; c < t.c; c += 2, n++) {
                     const int q = k + c, s = q % C::B_STAGES;
-                    // decoded weights, tokens, the accumulator (free from the start)
-                    const uint32_t bar = smem_u32(lane == 0 ? &a_full[sa] : lane == 1 ? &b_full[s] : &acc_empty[w]);
-                    const uint32_t par = lane == 0 ? pa : lane == 1 ? (q / C::B_STAGES) & 1 : (q / 2 - 1) & 1;
-                    if (!(ok = wait_on(bar, par, lane, q < 2 ? 2 : 3, &s_abort, 3))) break;
+                    // tokens with their scales, the accumulator (free from the start), and once a block the decoded weights
+                    const uint32_t bar = smem_u32(lane == 1 && n ? &acc_empty[w] : lane == 2 ? &a_full[sa] : &b_full[s]);
+                    const uint32_t par = lane == 1 && n ? (n - 1) & 1 : lane == 2 ? pa : (q / C::B_STAGES) & 1;
+                    if (!(ok = wait_on(bar, par, lane, NARROW || c == w ? 3 : 2, &s_abort, 3))) break;
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                     const uint64_t bd = nosw_desc(smem_u32(smem + C::SM_B + s * C::B_BYTES), 128, 8 * C::TOK_BYTES);
                     const uint32_t acc = tmem + 256 + w * 2 * CHUNK, a = tmem + sa * 128;
-                    const bool last = c + 2 >= t.c; // this warp's last use of the decoded weights
                     if (lead) {
+                        bar_arrive(&acc_full[w]); // hands on what this warp has waited for: the scales of the tokens and of the weights
                         if (Q6) {
 #pragma unroll 4
                             for (int i = 0; i < 8; i++) mma_i8_ts(acc, a + i * 8, bd + i * 16, id, i > 0);
@@ -308,23 +328,16 @@ __global__ void __launch_bounds__(NTHREADS, 1) gemm_kq_kernel(const __grid_const
                             tc_mma_ss(acc, nosw_desc(mins + 4096, 2048, 128), bd + 256, id, 1); // last: the others are exact
                             tc_mma_ss(acc + CHUNK, nosw_desc(mins, 2048, 128), bd + 256, id, 0);
                         }
-                        if (last) tc_commit(smem_u32(&a_empty[sa]));
-                    }
-                    if (lead) {
                         tc_commit(smem_u32(&acc_full[w]));
+                        if (c + 2 >= t.c) tc_commit(smem_u32(&a_empty[sa])); // this warp's last use of the decoded weights
                         tc_commit(smem_u32(&b_empty[s]));
                     }
                     __syncwarp();
                 }
-                if (ok && ((k & 1) ^ w) >= t.c) { // no chunk of this block for this warp; it still sees every phase of a_full, and arrives once per phase of a_empty
-                    ok = wait(&a_full[sa], pa, 3);
-                    if (ok && lead) bar_arrive(&a_empty[sa]);
-                }
-                __syncwarp();
                 k += t.c;
                 if (++b == nb) {
                     b = 0;
-                    if (u + 1 < total) t = tile_at(p, ++tile);
+                    if (u + 1 < total) t = tile_at<NARROW>(p, ++tile);
                 }
             }
             if (!ok && lead) { // MMAs in flight end before TMEM is freed
@@ -333,20 +346,26 @@ __global__ void __launch_bounds__(NTHREADS, 1) gemm_kq_kernel(const __grid_const
             }
         }
         __syncwarp();
-    } else if (warp >= 8) { // decode the packed blocks into TMEM, a thread per row
-        asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(REG_UNPACK));
-        const int row = tid & 127;
+    } else if (warp >= 4 * C::DRAIN_WG) { // decode the packed blocks into TMEM, a thread per row
+        if (NARROW) asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(C::REG_DECODE));
+        else asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(C::REG_DECODE));
+        const int row = tid & 127, turn = NARROW ? (warp >> 2) - 1 : 0; // NARROW: this warpgroup takes the blocks of its parity
         const uint32_t tl = tmem + ((uint32_t)((warp & 3) * 32) << 16);
         if (!Q6) {
             const __half2 k1024 = __float2half2_rn(1024.f);
-            for (int u = 0; u < total; u++) {
+            for (int u = turn; u < total; u += C::DECODE_WG) {
                 const int s = u % C::RAW_STAGES, sa = u & 1;
-                // the packed blocks, and the place of the decoded ones (free from the start)
-                if (!wait_on(smem_u32(lane == 0 ? &raw_full[s] : &a_empty[sa]), lane == 0 ? (u / C::RAW_STAGES) & 1 : ((u >> 1) - 1) & 1, lane, u < 2 ? 1 : 2, &s_abort, 6)) break;
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                if (!wait(&raw_full[u % RAW_FULL], (u / RAW_FULL) & 1, 6)) break;
                 const uint8_t *blk = smem + C::SM_RAW + s * C::RAW_BYTES + row * KQ_Q4K_BYTES;
                 const uint4 hdr = *reinterpret_cast<const uint4 *>(blk);
                 const uint32_t sc_lo = hdr.y & 0x3F3F3F3Fu, sc_hi = (hdr.w & 0x0F0F0F0Fu) | ((hdr.y >> 2) & 0x30303030u);
+                uint4 codes[8];
+                if (NARROW)
+#pragma unroll
+                    for (int i = 0; i < 8; i++) codes[i] = *reinterpret_cast<const uint4 *>(blk + 16 + 16 * i);
+                // the place of the decoded blocks (free from the start)
+                if (u >= 2 && !wait(&a_empty[sa], ((u >> 1) - 1) & 1, 7)) break;
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 { // m_j, then k_j, in order of j, for the sums of 16 of even and of odd place
                     const uint32_t m_lo = hdr.z & 0x3F3F3F3Fu, m_hi = ((hdr.w >> 4) & 0x0F0F0F0Fu) | ((hdr.z >> 2) & 0x30303030u);
                     uint4 *am = reinterpret_cast<uint4 *>(smem + C::SM_AMIN + sa * C::AMIN_BYTES + (row >> 3) * 128 + (row & 7) * 16);
@@ -357,7 +376,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) gemm_kq_kernel(const __grid_const
                     am[256] = am[384] = make_uint4(k(two_bytes(sc_lo, 0)), k(two_bytes(sc_lo, 2)), k(two_bytes(sc_hi, 0)), k(two_bytes(sc_hi, 2)));
                     *reinterpret_cast<uint32_t *>(smem + C::SM_SC + ((u % SC_RING) * ROWS + row) * 4) = hdr.x;
                 }
-#pragma unroll 1
+#pragma unroll (NARROW ? 4 : 1)
                 for (int g = 0; g < 4; g++) { // 64 elements: sub-block 2g in the low nibbles, 2g + 1 in the high ones
                     const uint32_t scw = (g < 2 ? sc_lo : sc_hi) >> (16 * (g & 1));
                     const __half2 s0 = __hsub2(byte_pair(scw, 0), k1024), s1 = __hsub2(byte_pair(scw, 1), k1024);
@@ -368,7 +387,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) gemm_kq_kernel(const __grid_const
                     uint32_t o[32];
 #pragma unroll
                     for (int h = 0; h < 2; h++) {
-                        const uint4 w4 = *reinterpret_cast<const uint4 *>(blk + 16 + 32 * g + 16 * h);
+                        const uint4 w4 = NARROW ? codes[2 * g + h] : *reinterpret_cast<const uint4 *>(blk + 16 + 32 * g + 16 * h);
                         const uint32_t w[4] = {w4.x, w4.y, w4.z, w4.w};
 #pragma unroll
                         for (int i = 0; i < 4; i++) {
@@ -379,13 +398,14 @@ __global__ void __launch_bounds__(NTHREADS, 1) gemm_kq_kernel(const __grid_const
                             o[16 + 8 * h + 2 * i + 1] = u2(__hfma2(h2((v & 0x00F000F0u) | 0x64006400u), t1, o1));
                         }
                     }
-                    TMEM_ST32(tl + sa * 128 + g * 32, o);
+                    TMEM_ST16(tl + sa * 128 + g * 32, o);
+                    TMEM_ST16(tl + sa * 128 + g * 32 + 16, (o + 16));
                 }
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); // the min operand, for the MMA
                 asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
                 asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
                 __syncwarp();
-                if (lane == 0) bar_arrive(&a_full[sa]), bar_arrive(&sc_full[u % SC_RING]), bar_arrive(&raw_empty[s]);
+                if (lane == 0) bar_arrive(&a_full[sa]), bar_arrive(&raw_empty[s]);
             }
         } else {
             int tile = tile0, b = b0, k = -1;
@@ -394,7 +414,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) gemm_kq_kernel(const __grid_const
             for (int u = 0; u < total; u++) {
                 const int sa = u & 1;
                 if (u == 0 || b == 0) {
-                    const TilePos t = tile_at(p, tile);
+                    const TilePos t = tile_at<NARROW>(p, tile);
                     const int n = seg_rows(p, t.seg);
                     wr = (t.seg == 0 ? p.seg[0].W : t.seg == 1 ? p.seg[1].W : p.seg[2].W) + ((int64_t)t.expert * n + min(t.n0 + row, n - 1)) * p.w_row;
                 }
@@ -404,18 +424,20 @@ __global__ void __launch_bounds__(NTHREADS, 1) gemm_kq_kernel(const __grid_const
                     k++;
                     if (!wait(&raw_full[k % C::RAW_STAGES], (k / C::RAW_STAGES) & 1, 6)) break;
                 }
+                const int s = k % C::RAW_STAGES;
+                if (!NARROW || sa == turn) {
                 if (u >= 2 && !wait(&a_empty[sa], ((u >> 1) - 1) & 1, 7)) break;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const int s = k % C::RAW_STAGES;
                 const uint8_t *blk = smem + C::SM_RAW + s * C::RAW_BYTES + row * 32 + (b & 1) * 16; // chunk i of the block 4096 i further
                 const uint4 sc4 = *reinterpret_cast<const uint4 *>(blk + 12 * 4096);
                 const int b8 = b % KQ_Q6_GROUP;
                 const uint32_t dw = b8 < 2 ? dv.x : b8 < 4 ? dv.y : b8 < 6 ? dv.z : dv.w;
                 *reinterpret_cast<uint32_t *>(smem + C::SM_SC + ((u % SC_RING) * ROWS + row) * 4) = (b8 & 1 ? dw >> 16 : dw) & 0xFFFFu;
-#pragma unroll 1
+#pragma unroll (NARROW ? 2 : 1)
                 for (int hh = 0; hh < 2; hh++) { // 128 elements
                     const uint32_t sc_a = hh ? sc4.z : sc4.x, sc_b = hh ? sc4.w : sc4.y;
-#pragma unroll 1
+                    uint32_t wide_hi[NARROW ? 32 : 4], wide_lo[NARROW ? 32 : 4]; // NARROW: 128 elements at a time, for more independent work
+#pragma unroll (NARROW ? 2 : 1)
                     for (int h = 0; h < 2; h++) { // elements 128 hh + 32 q + 16 h + ..
                         const uint4 a4 = *reinterpret_cast<const uint4 *>(blk + (4 * hh + h) * 4096), c4 = *reinterpret_cast<const uint4 *>(blk + (4 * hh + 2 + h) * 4096),
                                     q4 = *reinterpret_cast<const uint4 *>(blk + (8 + 2 * hh + h) * 4096);
@@ -426,7 +448,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) gemm_kq_kernel(const __grid_const
                             // other.  Its upper byte is hi + 128, its lower one 4 lo.
                             const int sc = (int)((q < 2 ? sc_a : sc_b) << (24 - 8 * ((2 * q) & 3) - 8 * h)) >> 24;
                             const uint32_t k4 = 4u * (uint32_t)sc, base = 0x80008000u - 0x00800080u * (uint32_t)sc;
-                            uint32_t hi[4], lo[4];
+                            uint32_t *hi = wide_hi + (NARROW ? 8 * q + 4 * h : 0), *lo = wide_lo + (NARROW ? 8 * q + 4 * h : 0);
 #pragma unroll
                             for (int i = 0; i < 4; i++) {
                                 const uint32_t n = q & 1 ? c[i] : a[i], top = q == 0 ? qh[i] << 4 : q == 1 ? qh[i] << 2 : q == 2 ? qh[i] : qh[i] >> 2;
@@ -436,77 +458,92 @@ __global__ void __launch_bounds__(NTHREADS, 1) gemm_kq_kernel(const __grid_const
                                 lo[i] = __byte_perm(even, odd, 0x6240);
                             }
                             const uint32_t at = tl + sa * 128 + 32 * hh + 8 * q + 4 * h;
-                            TMEM_ST4(at, hi);
-                            TMEM_ST4(at + 64, lo);
+                            if (!NARROW) {
+                                TMEM_ST4(at, hi);
+                                TMEM_ST4(at + 64, lo);
+                            }
                         }
+                    }
+                    if constexpr (NARROW) {
+                        TMEM_ST32(tl + sa * 128 + 32 * hh, wide_hi);
+                        TMEM_ST32(tl + sa * 128 + 32 * hh + 64, wide_lo);
                     }
                 }
                 asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
                 asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
                 __syncwarp();
-                if (lane == 0) {
-                    bar_arrive(&a_full[sa]), bar_arrive(&sc_full[u % SC_RING]);
-                    if (b % 2 == 1 || b == nb - 1) bar_arrive(&raw_empty[s]);
+                if (lane == 0) bar_arrive(&a_full[sa]);
                 }
+                if (lane == 0 && (b % 2 == 1 || b == nb - 1)) bar_arrive(&raw_empty[s]);
                 if (++b == nb) b = 0, tile++;
             }
         }
         __syncwarp();
     } else { // add the accumulators to the running result
-        asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(REG_EPI));
-        const int row = tid & 127, wg = warp >> 2; // this warpgroup takes the groups of 16 tokens wg, wg + 2 of every chunk
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(C::REG_DRAIN));
+        const int row = tid & 127, half = NARROW ? 0 : (warp >> 2) * (CHUNK / 2); // of two warpgroups each takes half of every chunk
         const uint32_t tl = tmem + 256 + ((uint32_t)((warp & 3) * 32) << 16);
-        float y[8][16]; // [chunk, group][token]
+        constexpr int STEP = 16, PART = CHUNK / C::DRAIN_WG;
+        float y[C::GROUPS][16]; // [chunk, group of its part][token]
+        int tile = tile0, b = b0, n = 0, u = 0;
+        bool ok = true;
+        while (u < total) { // a tile, or this CTA's part of it
+            const TilePos t = tile_at<NARROW>(p, tile);
+            const int end = u + min(nb - b, total - u);
+            const bool whole = b == 0 && end - u == nb;
 #pragma unroll
-        for (int i = 0; i < 128; i++) y[i / 16][i % 16] = 0.f;
-        int tile = tile0, b = b0, q = 0;
-        TilePos t = {};
-        if (total) t = tile_at(p, tile);
-        for (int u = 0; u < total; u++) {
-            bool ok = true;
+            for (int i = 0; i < C::GROUPS * 16; i++) y[i / 16][i % 16] = 0.f;
+            // the loop over the blocks holds nothing else: with the tile's end inside it a turn took a thousand clocks more
+#pragma unroll 1
+            for (; u < end; u++) {
 #pragma unroll
-            for (int c = 0; c < MAX_CHUNKS; c++) {
-                if (c >= t.c || !ok) continue;
-                const int slot = q & 1, ks = u % SC_RING, kd = q % DA_RING;
-                const uint32_t bar = smem_u32(lane == 0 ? &acc_full[slot] : lane == 1 ? &da_full[kd] : &sc_full[ks]);
-                if (!(ok = wait_on(bar, lane == 0 ? (q >> 1) & 1 : lane == 1 ? (q / DA_RING) & 1 : (u / SC_RING) & 1, lane, 3, &s_abort, 9))) continue;
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const uint32_t dd = *reinterpret_cast<const uint32_t *>(smem + C::SM_SC + (ks * ROWS + row) * 4);
-                float2 df = __half22float2(h2(dd)); // d_w, d_min
-                if (Q6) df.x *= 0.25f; // the sums come four times
-                const float *da = reinterpret_cast<const float *>(smem + C::SM_DA + kd * CHUNK * 4) + wg * 16;
-                const uint32_t ta = tl + slot * 2 * CHUNK + wg * 16;
-                auto add16 = [&](float (&acc)[16], int g2) { // acc += d_a (d_w main - d_min min), or d_a d_w (64 hi + lo)
-                    if ((2 * g2 + wg) * 16 >= t.cw) return;
-                    uint32_t m[16], n[16];
-                    TMEM_LD16(ta + g2 * 32, m);
-                    TMEM_LD16(ta + g2 * 32 + CHUNK, n);
+                for (int c = 0; c < (NARROW ? 1 : MAX_CHUNKS); c++) {
+                    if (c >= t.c) break;
+                    const int slot = n & 1;
+                    if (!(ok = wait(&acc_full[slot], (n >> 1) & 1, 9))) break;
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                    const uint32_t ta = tl + slot * 2 * CHUNK + half;
+                    const float *da = reinterpret_cast<const float *>(smem + C::SM_DA + n % DA_RING * CHUNK * 4) + half;
+                    uint32_t m[2][STEP], l[2][STEP]; // two steps: one on its way while the other is added
+                    tmem_ld(ta, m[0]);
+                    tmem_ld(ta + CHUNK, l[0]);
+                    float2 df = __half22float2(h2(*reinterpret_cast<const uint32_t *>(smem + C::SM_SC + ((u % SC_RING) * ROWS + row) * 4))); // d_w, d_min
+                    if (Q6) df.x *= 0.25f; // the sums come four times
                     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-                    for (int j = 0; j < 16; j += 4) {
-                        const float4 da4 = *reinterpret_cast<const float4 *>(da + g2 * 32 + j);
-#pragma unroll
-                        for (int e = 0; e < 4; e += 2) { // two tokens per instruction: 28672 x 8192 at 512 tokens 325 -> 316 us
-                            const float2 main = Q6 ? make_float2(__int2float_rn((int)(m[j + e] * 256u + n[j + e])), __int2float_rn((int)(m[j + e + 1] * 256u + n[j + e + 1])))
-                                                   : make_float2(__uint_as_float(m[j + e]), __uint_as_float(m[j + e + 1]));
-                            float2 v = __fmul2_rn(make_float2(df.x, df.x), main);
-                            if (!Q6) v = __ffma2_rn(make_float2(-df.y, -df.y), make_float2(__uint_as_float(n[j + e]), __uint_as_float(n[j + e + 1])), v);
-                            const float2 r = __ffma2_rn(e ? make_float2(da4.z, da4.w) : make_float2(da4.x, da4.y), v, make_float2(acc[j + e], acc[j + e + 1]));
-                            acc[j + e] = r.x, acc[j + e + 1] = r.y;
+                    for (int st = 0; st < PART / STEP; st++) { // y += d_a (d_w main - d_min min), or d_a d_w (64 hi + lo)
+                        if (half + st * STEP >= t.cw) break;
+                        if (st + 1 < PART / STEP) { // behind the last step it loads what nobody uses
+                            tmem_ld(ta + (st + 1) * STEP, m[(st + 1) & 1]);
+                            tmem_ld(ta + (st + 1) * STEP + CHUNK, l[(st + 1) & 1]);
                         }
+                        const uint32_t(&mv)[STEP] = m[st & 1], (&lv)[STEP] = l[st & 1];
+#pragma unroll
+                        for (int j = 0; j < STEP; j += 4) {
+                            const float4 da4 = *reinterpret_cast<const float4 *>(da + st * STEP + j);
+                            float *acc = &y[c * (PART / 16) + st][j];
+#pragma unroll
+                            for (int e = 0; e < 4; e += 2) { // two tokens per instruction: 28672 x 8192 at 512 tokens 325 -> 316 us
+                                const float2 main = Q6 ? make_float2(__int2float_rn((int)(mv[j + e] * 256u + lv[j + e])), __int2float_rn((int)(mv[j + e + 1] * 256u + lv[j + e + 1])))
+                                                       : make_float2(__uint_as_float(mv[j + e]), __uint_as_float(mv[j + e + 1]));
+                                float2 v = __fmul2_rn(make_float2(df.x, df.x), main);
+                                if (!Q6) v = __ffma2_rn(make_float2(-df.y, -df.y), make_float2(__uint_as_float(lv[j + e]), __uint_as_float(lv[j + e + 1])), v);
+                                const float2 r = __ffma2_rn(e ? make_float2(da4.z, da4.w) : make_float2(da4.x, da4.y), v, make_float2(acc[e], acc[e + 1]));
+                                acc[e] = r.x, acc[e + 1] = r.y;
+                            }
+                        }
+                        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
                     }
-                };
-                add16(y[2 * c], 0);
-                add16(y[2 * c + 1], 1);
-                asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-                __syncwarp();
-                if (lane == 0) bar_arrive(&acc_empty[slot]);
-                q++;
+                    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                    __syncwarp();
+                    if (lane == 0) bar_arrive(&acc_empty[slot]);
+                    n++;
+                }
+                if (!ok) break;
             }
             if (!ok) break;
-            if (b == nb - 1 || u == total - 1) { // the end of this CTA's part of the tile
+            { // the end of this CTA's part of the tile
                 const uint32_t first = (uint32_t)tile * nb, big = rem * (per + 1);
-                const bool whole = b == nb - 1 && first >= u0;
                 // the CTAs that hold the tile's first and last block
                 auto cta_of = [&](uint32_t v) { return v < big ? v / (per + 1) : rem + (v - big) / per; };
                 const uint32_t c0 = cta_of(first), c1 = cta_of(first + nb - 1);
@@ -543,9 +580,9 @@ __global__ void __launch_bounds__(NTHREADS, 1) gemm_kq_kernel(const __grid_const
                         if (j < live) *dst = v[j];
                 };
 #pragma unroll 1
-                for (int i = 0; i < 8; i++) { // one copy of this code for all of y: it runs once per tile
-                    const int g16 = (2 * (i & 1) + wg) * 16, col0 = (i >> 1) * t.cw + g16;
-                    if ((i >> 1) >= t.c || g16 >= t.cw || col0 >= t.n) continue;
+                for (int i = 0; i < C::GROUPS; i++) { // one copy of this code for all of y: it runs once per tile
+                    const int c = i / (PART / 16), g16 = half + i % (PART / 16) * 16, col0 = c * t.cw + g16;
+                    if (c >= t.c || g16 >= t.cw || col0 >= t.n) continue;
                     float v[16];
 #define TAKE(I) case I: { _Pragma("unroll") for (int j = 0; j < 16; j++) v[j] = y[I][j]; } break
                     switch (i) {
@@ -553,18 +590,20 @@ __global__ void __launch_bounds__(NTHREADS, 1) gemm_kq_kernel(const __grid_const
                         TAKE(1);
                         TAKE(2);
                         TAKE(3);
-                        TAKE(4);
-                        TAKE(5);
-                        TAKE(6);
                     default:
-#pragma unroll
-                        for (int j = 0; j < 16; j++) v[j] = y[7][j];
+                        if constexpr (!NARROW)
+                            switch (i) {
+                                TAKE(4);
+                                TAKE(5);
+                                TAKE(6);
+                                TAKE(7);
+                            }
                     }
 #undef TAKE
                     if (whole) {
                         put(v, col0);
                     } else {
-                        float *dst = p.part + ((int64_t)blockIdx.x * 2 + (first >= u0 ? 1 : 0)) * TILE_OUT + (i * 2 + wg) * 16 * ROWS + row;
+                        float *dst = p.part + ((int64_t)blockIdx.x * 2 + (first >= u0 ? 1 : 0)) * TILE_OUT + (c * CHUNK + g16) * ROWS + row;
 #pragma unroll
                         for (int j = 0; j < 16; j++) __stcg(dst + j * ROWS, v[j]);
                     }
@@ -578,37 +617,42 @@ __global__ void __launch_bounds__(NTHREADS, 1) gemm_kq_kernel(const __grid_const
                     if (before == (int)(c1 - c0)) { // this warp's part of the tile is complete
                         __threadfence();
 #pragma unroll 1
-                        for (int i = 0; i < 8; i++) {
-                            const int g16 = (2 * (i & 1) + wg) * 16, col0 = (i >> 1) * t.cw + g16;
-                            if ((i >> 1) >= t.c || g16 >= t.cw || col0 >= t.n) continue;
+                        for (int i = 0; i < C::GROUPS; i++) {
+                            const int c = i / (PART / 16), g16 = half + i % (PART / 16) * 16, col0 = c * t.cw + g16;
+                            if (c >= t.c || g16 >= t.cw || col0 >= t.n) continue;
                             float v[16];
 #pragma unroll
                             for (int j = 0; j < 16; j++) v[j] = 0.f;
-                            const float *src = p.part + ((int64_t)c0 * 2 + 1) * TILE_OUT + (i * 2 + wg) * 16 * ROWS + row;
-                            uint32_t step = TILE_OUT; // the first CTA's second part, then the first parts of the others
+                            const float *src = p.part + ((int64_t)c0 * 2 + 1) * TILE_OUT + (c * CHUNK + g16) * ROWS + row;
+                            // the first CTA's second part, then the first parts of the others; eight at a time, so that their trips to L2 overlap
 #pragma unroll 1
-                            for (uint32_t cc = c0; cc <= c1; cc++) {
+                            for (uint32_t cc = c0; cc <= c1; cc += 8) {
+                                float part[8][16];
 #pragma unroll
-                                for (int j = 0; j < 16; j++) v[j] += __ldcg(src + j * ROWS);
-                                src += step, step = 2 * TILE_OUT;
+                                for (int r = 0; r < 8; r++) {
+                                    const float *from = src + (cc + r == c0 ? 0 : (int64_t)(2 * (cc + r - c0) - 1) * TILE_OUT);
+#pragma unroll
+                                    for (int j = 0; j < 16; j++) part[r][j] = cc + r <= c1 ? __ldcg(from + j * ROWS) : 0.f;
+                                }
+#pragma unroll
+                                for (int r = 0; r < 8; r++)
+                                    if (cc + r <= c1)
+#pragma unroll
+                                        for (int j = 0; j < 16; j++) v[j] += part[r][j];
                             }
                             put(v, col0);
                         }
                     }
                 }
-#pragma unroll
-                for (int i = 0; i < 128; i++) y[i / 16][i % 16] = 0.f;
             }
-            if (++b == nb) {
-                b = 0;
-                if (u + 1 < total) t = tile_at(p, ++tile);
-            }
+            b = 0, tile++;
         }
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     if (warp == 15) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512) : "memory");
 }
+
 
 // Q8 rows -> the token operand, in the forms that the call's matrices read.  A thread writes 16 bytes of a token: eight codes (or sums of 16) as
 // f16, in the order in which Q4_K weights are decoded (0 2 1 3 of every four), or 16 codes.  grid (runs of 16 tokens, blocks); tokens past
@@ -621,7 +665,7 @@ struct ImageParams {
     float *da;
     int32_t M, nb, m_pad, act_div;
     const int32_t *row_src, *tile_count, *n_tiles; // products with experts
-    int32_t first_tile;
+    int32_t first_tile, tile_tok, narrow;
 };
 __global__ void __launch_bounds__(288) act_image_kernel(const __grid_constant__ ImageParams p) {
     KQ_PDL_ENTER();
@@ -630,13 +674,13 @@ __global__ void __launch_bounds__(288) act_image_kernel(const __grid_constant__ 
     const int b = blockIdx.y, base = blockIdx.x * 16;
     int n_live = p.M - base; // tokens of this run
     if (p.row_src) {
-        const int tile = base / 128;
+        const int tile = base / p.tile_tok, at = base - tile * p.tile_tok;
         if (tile >= *p.n_tiles - p.first_tile) return;
         const int n = p.tile_count[tile];
         int c, cw;
-        chunks_of(n, c, cw);
-        if (base - tile * 128 >= c * cw) return;
-        n_live = n - (base - tile * 128);
+        chunks_of(p.narrow, n, c, cw);
+        if (at >= c * cw) return;
+        n_live = n - at;
     }
     const __half2 k1152 = __float2half2_rn(1152.f);
     auto source_row = [&](int at) { return (int64_t)(p.row_src ? p.row_src[base + at] / p.act_div : base + at) * p.nb + b; };
@@ -684,8 +728,8 @@ __global__ void __launch_bounds__(288) act_image_kernel(const __grid_constant__ 
 // order inside an expert is the pair order whatever the timing (with 8 warps and a serial table of tiles 55 us
 // for 8192 pairs and 128 experts, now 27).  Output: n_tiles, the expert of each
 // tile, and for each tile row the pair it holds.
-constexpr int TM = 128, SORT_WARPS = 16, SORT_MAX_E = 256;
-__global__ void __launch_bounds__(SORT_WARPS * 32) moe_sort_kernel(const int32_t *ids, int n_pairs, int E,
+constexpr int SORT_WARPS = 16, SORT_MAX_E = 256;
+__global__ void __launch_bounds__(SORT_WARPS * 32) moe_sort_kernel(const int32_t *ids, int n_pairs, int E, int TM,
                                                                    int32_t *n_tiles_out, int32_t *tile_expert, int32_t *row_src,
                                                                    int32_t *tile_count) {
     KQ_PDL_ENTER();
@@ -846,13 +890,18 @@ b200_status scratch(int dev, size_t img16_bytes, size_t img8_bytes, size_t da_by
         if (need[i] && capturing) captured[dev][i] = true;
     }
     if (!attr[dev]) {
-        cudaFuncAttributes a4, a6;
-        KQ_CUDA(cudaFuncSetAttribute(gemm_kq_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<false>::SMEM));
-        KQ_CUDA(cudaFuncSetAttribute(gemm_kq_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<true>::SMEM));
-        KQ_CUDA(cudaFuncGetAttributes(&a4, gemm_kq_kernel<false>));
-        KQ_CUDA(cudaFuncGetAttributes(&a6, gemm_kq_kernel<true>));
-        // setmaxnreg moves registers of the launch between the warpgroups: more than it was launched with would wait for ever
-        KQ_REQUIRE(4 * std::min(a4.numRegs, a6.numRegs) >= 2 * REG_EPI + REG_UNPACK + REG_REST, "gemm: built with %d / %d registers", a4.numRegs, a6.numRegs);
+        auto prepare = [](const void *f, int smem, int regs) {
+            cudaFuncAttributes a;
+            KQ_CUDA(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+            KQ_CUDA(cudaFuncGetAttributes(&a, f));
+            // setmaxnreg moves registers of the launch between the warpgroups: more than it was launched with would wait for ever
+            KQ_REQUIRE(4 * a.numRegs >= regs, "gemm: built with %d registers", a.numRegs);
+            return B200_OK;
+        };
+        KQ_TRY(prepare((const void *)gemm_kq_kernel<false, false>, Cfg<false, false>::SMEM, Cfg<false, false>::REG_SUM));
+        KQ_TRY(prepare((const void *)gemm_kq_kernel<false, true>, Cfg<false, true>::SMEM, Cfg<false, true>::REG_SUM));
+        KQ_TRY(prepare((const void *)gemm_kq_kernel<true, false>, Cfg<true, false>::SMEM, Cfg<true, false>::REG_SUM));
+        KQ_TRY(prepare((const void *)gemm_kq_kernel<true, true>, Cfg<true, true>::SMEM, Cfg<true, true>::REG_SUM));
         attr[dev] = true;
     }
     *out = {img16_bytes ? (uint8_t *)buf[dev][0] : nullptr, img8_bytes ? (uint8_t *)buf[dev][1] : nullptr, (float *)buf[dev][2], (float *)buf[dev][3]};
@@ -896,28 +945,36 @@ b200_status add_seg(Params &p, int i, const KqGemvSeg &g, int64_t experts, int64
     return B200_OK;
 }
 
-// Blocks of a CTA at least: shorter shares are shorter chains, but more parts to add up.  77 tokens through nine layers of the 3B shape take
-// 1457 / 1468 / 1633 us at 2 / 4 / 8, 16 users of the experts' model 1073 / 1089 / 1132; large products do not depend on it.
+// Blocks of a CTA at least, in products with experts: shorter shares are shorter chains, but more parts to add up.
 constexpr int MIN_SHARE = 2;
 
-// Token tiles of a dense product, by the time they should take in tenths of a microsecond.  A (tile, block) pair costs its decoding and, per 64 tokens,
-// its MMAs and drains (Q4_K 1.6 us at 64 tokens, 3.6 at 256; Q6_K 2.4 and 4.0); adding up a tile that was cut costs its last CTA about 1 us
-// per part and 64 tokens.  Wide tiles decode a weight less often; narrow ones are more pairs, hence fewer parts and a shorter end where a product
-// is too small to keep the GPU busy: 256 x 2048 at 1024 tokens in Q4_K 32.4 us as tiles of 256 tokens, 19.7 as tiles of 64; 1024 x 5120 at 512 50.6 and
-// 27.6, at 2048 62.4 and (tiles of 128) 55.2; 5120 x 5120 at 1024 96 and 131.
+// Token tiles of a dense product and the least share of a CTA, by the time they should take, in hundredths of a microsecond.  A (tile, block) pair
+// costs its decoding or its MMAs, whichever is longer, and the drains' turns (28672 x 8192, the pairs of a CTA one after another: Q4_K 0.9 us with 16 tokens,
+// 1.1 with 64, 1.6 with 128, 2.5 with 256; Q6_K 1.5, 1.7, 2.3, 2.7).  A tile that was cut is added up by its last CTA: a trip to L2 for every
+// eight parts and 16 tokens of a warp, and its parts come in at the rate of one SM.  Wide tiles decode a weight less often; narrow ones are more pairs, hence fewer parts and a shorter end where
+// a product is too small to keep the GPU busy: 1024 x 5120 in Q4_K with 512 tokens 41 us as tiles of 256, 25 as tiles of 128; 5120 x 5120
+// with 1024 tokens 81 and 86, with 64 tokens 24 as a tile of two chunks and 22 as one of one.
 struct TokTiles {
     int n, tok;
+    bool narrow;
+    int min_share;
 };
 TokTiles token_tiles(bool q6, int64_t M, int64_t row_tiles, int64_t nb) {
-    TokTiles best = {0, 0};
+    TokTiles best = {0, 0, false, 0};
     int64_t best_cost = INT64_MAX;
-    for (int chunks = MAX_CHUNKS; chunks >= 1; chunks--) {
+    for (int chunks = MAX_CHUNKS; chunks >= 1; chunks /= 2) {
+        const bool narrow = chunks == 1;
         int c, cw;
-        chunks_of((int)kq_div_up(M, kq_div_up(M, chunks * CHUNK)), c, cw);
-        const int64_t tiles = kq_div_up(M, c * cw), pairs = tiles * row_tiles * nb, ctas = std::max<int64_t>(1, std::min<int64_t>(kq_sm_count(), pairs / MIN_SHARE));
-        const int64_t share = kq_div_up(pairs, ctas), per_pair = (q6 ? 19 : 8) * CHUNK + (q6 ? 5 : 7) * c * cw;
-        const int64_t cost = share * per_pair + (pairs % ctas == 0 && share % nb == 0 ? 0 : 10 * c * cw * nb / share);
-        if (cost < best_cost) best_cost = cost, best = {(int)tiles, c * cw};
+        chunks_of(narrow, (int)kq_div_up(M, kq_div_up(M, chunks * CHUNK)), c, cw);
+        const int64_t tok = c * cw, tiles = kq_div_up(M, tok), pairs = tiles * row_tiles * nb;
+        const int64_t per_pair = narrow ? (q6 ? 130 + tok / 4 : 80 + tok / 4) : c == 2 ? (q6 ? 175 : 110) + tok * 3 / 10 : (q6 ? 240 + tok / 7 : 178 + tok * 2 / 7);
+        const int64_t groups = narrow ? cw / 16 : c * kq_div_up(std::min(cw, CHUNK / 2), 16); // of 16 tokens that a draining warp has
+        for (const int min_share : {2, 3, 4, 6, 8}) {
+            const int64_t ctas = std::max<int64_t>(1, std::min<int64_t>(kq_sm_count(), pairs / min_share)), share = kq_div_up(pairs, ctas);
+            const int64_t parts = pairs % ctas == 0 && nb % share == 0 ? nb / share : kq_div_up(nb - 1, share) + 1;
+            const int64_t cost = share * per_pair + (pairs % ctas == 0 && share % nb == 0 ? 0 : 150 + 50 * groups * kq_div_up(parts, 8) + parts * tok * (narrow ? 50 : 40) / CHUNK);
+            if (cost < best_cost) best_cost = cost, best = {(int)tiles, (int)tok, narrow, min_share};
+        }
     }
     return best;
 }
@@ -926,29 +983,30 @@ TokTiles token_tiles_of(uint32_t type, const KqGemvSeg *segs, int nseg, int64_t 
     int64_t row_tiles = 0;
     for (int i = 0; i < nseg; i++)
         if (segs[i].type == type) row_tiles += kq_div_up(segs[i].n_rows, ROWS);
-    return row_tiles ? token_tiles(type == B200_TYPE_Q6_K, M, row_tiles, nb) : TokTiles{0, 0};
+    return row_tiles ? token_tiles(type == B200_TYPE_Q6_K, M, row_tiles, nb) : TokTiles{0, 0, false, 0};
 }
 
 // one launch per weight type for the matrices that read the images in sc; dense products cut the tokens by type
-b200_status launch_segs(Params p, const Scratch &sc, const KqGemvSeg *segs, int nseg, int64_t experts, int64_t K, cudaStream_t st) {
+b200_status launch_segs(Params p, bool narrow, const Scratch &sc, const KqGemvSeg *segs, int nseg, int64_t experts, int64_t K, cudaStream_t st) {
     for (const uint32_t type : {(uint32_t)B200_TYPE_Q4_K, (uint32_t)B200_TYPE_Q6_K}) {
         int n = 0;
         p.row_tiles = 0;
         if (!p.row_src) {
             const TokTiles t = token_tiles_of(type, segs, nseg, p.M, p.nb);
-            p.tok_tiles = t.n, p.tile_tok = t.tok;
+            p.tok_tiles = t.n, p.tile_tok = t.tok, p.min_share = t.min_share, narrow = t.narrow;
         }
         p.img = type == B200_TYPE_Q4_K ? sc.img16 : sc.img8, p.da = sc.da, p.part = sc.part;
         for (int i = 0; i < nseg; i++)
             if (segs[i].type == type) KQ_TRY(add_seg(p, n++, segs[i], experts, K));
         if (!n) continue;
-        p.min_share = MIN_SHARE;
         const int64_t units = (int64_t)p.tok_tiles * p.row_tiles * p.nb;
         KQ_REQUIRE(units < (int64_t)1 << 31, "gemm: bad shape");
         // with experts the number of tiles is known on the device only
         const int grid = p.row_src ? kq_sm_count() : (int)std::min<int64_t>(kq_sm_count(), std::max<int64_t>(1, units / p.min_share));
-        if (type == B200_TYPE_Q4_K) KQ_CUDA(kq_launch(gemm_kq_kernel<false>, dim3(grid), dim3(NTHREADS), Cfg<false>::SMEM, st, p));
-        else KQ_CUDA(kq_launch(gemm_kq_kernel<true>, dim3(grid), dim3(NTHREADS), Cfg<true>::SMEM, st, p));
+        if (type == B200_TYPE_Q4_K && narrow) KQ_CUDA(kq_launch(gemm_kq_kernel<false, true>, dim3(grid), dim3(NTHREADS), Cfg<false, true>::SMEM, st, p));
+        else if (type == B200_TYPE_Q4_K) KQ_CUDA(kq_launch(gemm_kq_kernel<false, false>, dim3(grid), dim3(NTHREADS), Cfg<false, false>::SMEM, st, p));
+        else if (narrow) KQ_CUDA(kq_launch(gemm_kq_kernel<true, true>, dim3(grid), dim3(NTHREADS), Cfg<true, true>::SMEM, st, p));
+        else KQ_CUDA(kq_launch(gemm_kq_kernel<true, false>, dim3(grid), dim3(NTHREADS), Cfg<true, false>::SMEM, st, p));
         KQ_COUNT_LAUNCH();
         KQ_LAUNCH_CHECK();
     }
@@ -1005,7 +1063,7 @@ b200_status kq_launch_gemm_tc(const KqGemvSeg *segs, int nseg, const int8_t *q, 
             continue;
         }
         KQ_TRY(rc);
-        const ImageParams ip = {q + m0 * K, d + m0 * nb, bs + m0 * nb * 16, sc.img16, sc.img8, sc.da, (int32_t)mc, (int32_t)nb, p.m_pad, 1, nullptr, nullptr, nullptr, 0};
+        const ImageParams ip = {q + m0 * K, d + m0 * nb, bs + m0 * nb * 16, sc.img16, sc.img8, sc.da, (int32_t)mc, (int32_t)nb, p.m_pad, 1, nullptr, nullptr, nullptr, 0, 0, 0};
         KQ_CUDA(kq_launch(act_image_kernel, dim3((unsigned)(p.m_pad / 16), (unsigned)nb), dim3(288), 0, st, ip));
         KQ_COUNT_LAUNCH();
         KqGemvSeg sg[MAX_SEGS];
@@ -1014,7 +1072,7 @@ b200_status kq_launch_gemm_tc(const KqGemvSeg *segs, int nseg, const int8_t *q, 
             sg[i].y += m0 * sg[i].n_rows;
         }
         p.residual = residual ? residual + m0 * segs[0].n_rows : nullptr;
-        KQ_TRY(launch_segs(p, sc, sg, nseg, 1, K, st));
+        KQ_TRY(launch_segs(p, false, sc, sg, nseg, 1, K, st));
     }
     return B200_OK;
 }
@@ -1022,11 +1080,15 @@ b200_status kq_launch_gemm_tc(const KqGemvSeg *segs, int nseg, const int8_t *q, 
 // ---- MUL_MAT_ID over many tokens: pairs gathered per expert, one grouped launch of the tensor-core kernel ----
 // Scratch of the sort, in int32 words: [0] number of live tiles, [1 .. 1 + max_tiles) expert per tile,
 // [1 + max_tiles ..) pair per tile row, then pairs per tile; max_tiles = ceil(n_pairs / 128) + n_expert bounds sum_e ceil(c_e / 128).
-static inline int64_t moe_max_tiles(int64_t n_pairs, int64_t E) { return kq_div_up(n_pairs, TM) + E; }
+// Pairs of a tile: with few pairs an expert narrow tiles (128 experts, one pair each: a layer's step of 16 users 754 us in four layers, as tiles of two chunks 930); from about
+// as many as fill one, wide ones, where most experts are one tile (64 pairs each: two layers 1246 us, 1308 as narrow tiles).  Narrow tiles need no more
+// room for the sort than wide ones: at most 48 E / 64 + E tiles of 64 rows against E of 128.
+static inline int moe_tile(int64_t n_pairs, int64_t E) { return n_pairs <= 48 * E ? CHUNK : 2 * CHUNK; }
+static inline int64_t moe_max_tiles(int64_t n_pairs, int64_t E) { return kq_div_up(n_pairs, moe_tile(n_pairs, E)) + E; }
 
 size_t kq_moe_sort_scratch_bytes(int64_t n_pairs, int64_t E) {
     const int64_t mt = moe_max_tiles(n_pairs, E);
-    return (size_t)(1 + mt + mt * TM + mt + 64) * sizeof(int32_t);
+    return (size_t)(1 + mt + mt * moe_tile(n_pairs, E) + mt + 64) * sizeof(int32_t);
 }
 
 b200_status kq_moe_sort(const int32_t *ids, int64_t n_pairs, int64_t E, int32_t *scratch, size_t scratch_bytes, cudaStream_t st) {
@@ -1034,7 +1096,8 @@ b200_status kq_moe_sort(const int32_t *ids, int64_t n_pairs, int64_t E, int32_t 
     KQ_REQUIRE(scratch_bytes >= kq_moe_sort_scratch_bytes(n_pairs, E), "moe_sort: scratch of %zu bytes, %zu needed", scratch_bytes,
                kq_moe_sort_scratch_bytes(n_pairs, E));
     const int64_t mt = moe_max_tiles(n_pairs, E);
-    kq_launch(moe_sort_kernel, 1, SORT_WARPS * 32, 0, st, ids, (int)n_pairs, (int)E, scratch, scratch + 1, scratch + 1 + mt,
+    const int TM = moe_tile(n_pairs, E);
+    kq_launch(moe_sort_kernel, 1, SORT_WARPS * 32, 0, st, ids, (int)n_pairs, (int)E, TM, scratch, scratch + 1, scratch + 1 + mt,
               scratch + 1 + mt + mt * TM);
     KQ_COUNT_LAUNCH();
     KQ_LAUNCH_CHECK();
@@ -1052,12 +1115,14 @@ b200_status kq_launch_gemm_grouped(const KqGemvSeg *segs, int nseg, const int8_t
         KQ_REQUIRE(segs[i].expert_stride == kq_device_row_bytes(segs[i].type, K) * segs[i].n_rows && segs[i].expert_stride % 16 == 0,
                    "grouped gemm: expert matrices must be contiguous and 16-byte aligned");
     const int64_t nb = K / 256, mt = moe_max_tiles(n_pairs, E);
+    const int TM = moe_tile(n_pairs, E);
+    const bool narrow = TM == CHUNK;
     const int64_t per_token = token_bytes(segs, nseg, nb, false) + token_bytes(segs, nseg, nb, true);
     int64_t slab = std::max<int64_t>(1, GROUP_BYTES / (per_token * TM));
     for (int64_t t0 = 0, tc; t0 < mt; t0 += tc) {
         tc = kq_div_up(mt - t0, kq_div_up(mt - t0, slab));
         Params p = {};
-        p.M = p.m_pad = (int32_t)(tc * TM), p.nb = (int32_t)nb, p.tok_tiles = (int)tc, p.first_tile = (int)t0;
+        p.M = p.m_pad = (int32_t)(tc * TM), p.nb = (int32_t)nb, p.tok_tiles = (int)tc, p.first_tile = (int)t0, p.tile_tok = TM, p.min_share = MIN_SHARE;
         Scratch sc;
         const b200_status rc = scratch_for(dev, segs, nseg, p.m_pad, nb, st, &sc);
         if (rc == B200_ERR_ALLOC && tc > 1) {
@@ -1067,10 +1132,10 @@ b200_status kq_launch_gemm_grouped(const KqGemvSeg *segs, int nseg, const int8_t
         }
         KQ_TRY(rc);
         p.n_tiles = sorted, p.tile_expert = sorted + 1 + t0, p.row_src = sorted + 1 + mt + t0 * TM, p.tile_count = sorted + 1 + mt + mt * TM + t0;
-        const ImageParams ip = {q, d, bs, sc.img16, sc.img8, sc.da, 0, (int32_t)nb, p.m_pad, act_div, p.row_src, p.tile_count, p.n_tiles, p.first_tile};
+        const ImageParams ip = {q, d, bs, sc.img16, sc.img8, sc.da, 0, (int32_t)nb, p.m_pad, act_div, p.row_src, p.tile_count, p.n_tiles, p.first_tile, TM, narrow};
         KQ_CUDA(kq_launch(act_image_kernel, dim3((unsigned)(p.m_pad / 16), (unsigned)nb), dim3(288), 0, st, ip));
         KQ_COUNT_LAUNCH();
-        KQ_TRY(launch_segs(p, sc, segs, nseg, E, K, st));
+        KQ_TRY(launch_segs(p, narrow, sc, segs, nseg, E, K, st));
     }
     return B200_OK;
 }

@@ -309,3 +309,41 @@ def test_experts_in_slabs():
         at = np.nonzero(ids == e)[0]
         want, size = exact(ty, W[e * N:(e + 1) * N], x[at // ku], N, K)
         check(got[at], want, size, K)
+
+
+@pytest.mark.parametrize("ty", [orc.TYPE_Q4_K, orc.TYPE_Q6_K], ids=["q4_k", "q6_k"])
+@pytest.mark.parametrize("N,K", [(20000, 512), (2000, 2816)])
+def test_tiles_of_one_two_and_four_chunks(ty, N, K):
+    """every edge between tiles of one chunk (two warpgroups decode in turn), of two and of four, with many and with few row tiles"""
+    import torch
+
+    from mesh_llm_b200 import capi, ops
+
+    W = blocks_of(ty, N, K, 21)
+    dev = ops.upload_weights(ty, W, N, K)
+    x = np.random.default_rng(22).standard_normal((260, K)).astype(np.float32)
+    want, size = exact(ty, W, x, N, K)
+    for M in (9, 31, 33, 49, 64, 65, 97, 128, 129, 192, 193, 255, 260):
+        got = ops.mul_mat(ty, dev, torch.from_numpy(x[:M]).cuda(), N, K).cpu().numpy()
+        assert capi.lib().b200_check_device_waits() == 0
+        check(got, want[:M], size[:M], K)
+
+
+@pytest.mark.parametrize("ty", [orc.TYPE_Q4_K, orc.TYPE_Q6_K], ids=["q4_k", "q6_k"])
+@pytest.mark.parametrize("pairs", [9, 47, 48 * 5, 48 * 5 + 1, 700])
+def test_experts_with_narrow_and_wide_tiles(ty, pairs):
+    """five experts, one of them without a pair and one with most of them, on both sides of the number of pairs from which tiles are wide"""
+    import torch
+
+    from mesh_llm_b200 import capi, ops
+
+    E, N, K = 5, 200, 768
+    rng = np.random.default_rng(pairs)
+    W = blocks_of(ty, E * N, K, 23)
+    ids = rng.choice([0, 1, 3, 4], pairs, p=[0.7, 0.1, 0.15, 0.05]).astype(np.int32)
+    x = rng.standard_normal((pairs, K)).astype(np.float32)
+    want, size = exact(ty, W, x, E * N, K)
+    pick = lambda v: v.reshape(pairs, E, N)[np.arange(pairs), ids]
+    got = ops.mul_mat_id(ty, ops.upload_weights(ty, W, E * N, K), E, torch.from_numpy(x).cuda(), torch.from_numpy(ids[:, None]).cuda(), N, K).cpu().numpy()
+    assert capi.lib().b200_check_device_waits() == 0
+    check(got.reshape(pairs, N), pick(want), pick(size), K)
