@@ -222,28 +222,65 @@ __device__ __forceinline__ int kq_act_code(float x, float id) {
 
 // The quantiser applied to one block by one warp (b200_quantize_act and every fused form of it).
 // One warp per 256-element block.  Lane l owns elements 8l .. 8l+7 (values in v[8]).
-__device__ __forceinline__ void kq_quantize_block_warp(const float (&v)[8], int lane, int8_t *qb,
-                                                    float *d_out, int16_t *bs_out) {
+struct KqQ8Codes {
+    int c[8]; // this lane's codes
+    uint2 pk; // the same in bytes
+    int sum;  // of the 16 codes of this lane and its neighbour (lane ^ 1)
+    float d;
+};
+__device__ __forceinline__ KqQ8Codes kq_quantize_codes_warp(const float (&v)[8]) {
+    KqQ8Codes o;
     float amax = 0.f;
 #pragma unroll
     for (int i = 0; i < 8; i++) amax = fmaxf(amax, fabsf(v[i]));
     amax = kq_warp_max(amax);
-    const float d = kq_act_scale(amax), id = kq_act_inv(d);
-    int c[8], s = 0;
+    o.d = kq_act_scale(amax);
+    const float id = kq_act_inv(o.d);
+    o.sum = 0;
 #pragma unroll
     for (int i = 0; i < 8; i++) {
-        c[i] = kq_act_code(v[i], id);
-        s += c[i];
+        o.c[i] = kq_act_code(v[i], id);
+        o.sum += o.c[i];
     }
-    uint2 pk;
-    pk.x = (uint32_t)(c[0] & 0xFF) | ((uint32_t)(c[1] & 0xFF) << 8) | ((uint32_t)(c[2] & 0xFF) << 16) |
-           ((uint32_t)(c[3] & 0xFF) << 24);
-    pk.y = (uint32_t)(c[4] & 0xFF) | ((uint32_t)(c[5] & 0xFF) << 8) | ((uint32_t)(c[6] & 0xFF) << 16) |
-           ((uint32_t)(c[7] & 0xFF) << 24);
-    *reinterpret_cast<uint2 *>(qb + lane * 8) = pk;
-    s += __shfl_xor_sync(0xffffffffu, s, 1);
-    if ((lane & 1) == 0) bs_out[lane >> 1] = (int16_t)s;
-    if (lane == 0) *d_out = d;
+    const int(&c)[8] = o.c;
+    o.pk.x = (uint32_t)(c[0] & 0xFF) | ((uint32_t)(c[1] & 0xFF) << 8) | ((uint32_t)(c[2] & 0xFF) << 16) |
+             ((uint32_t)(c[3] & 0xFF) << 24);
+    o.pk.y = (uint32_t)(c[4] & 0xFF) | ((uint32_t)(c[5] & 0xFF) << 8) | ((uint32_t)(c[6] & 0xFF) << 16) |
+             ((uint32_t)(c[7] & 0xFF) << 24);
+    o.sum += __shfl_xor_sync(0xffffffffu, o.sum, 1);
+    return o;
+}
+__device__ __forceinline__ void kq_quantize_block_warp(const float (&v)[8], int lane, int8_t *qb,
+                                                    float *d_out, int16_t *bs_out) {
+    const KqQ8Codes o = kq_quantize_codes_warp(v);
+    *reinterpret_cast<uint2 *>(qb + lane * 8) = o.pk;
+    if ((lane & 1) == 0) bs_out[lane >> 1] = (int16_t)o.sum;
+    if (lane == 0) *d_out = o.d;
+}
+#endif
+
+// The tokens as the tensor-core product reads them, [block][groups of 8 tokens][chunks of 16 bytes][8 tokens]: 256 f16 codes (0 2 1 3 of every four)
+// and 16 f16 sums (those of even, then those of odd place) of a token and block in img16, for Q4_K weights, or 256 int8 codes in img8, for Q6_K; scales
+// [block][m_pad].  Tokens from n_tok to m_pad are zeros.  Who writes it also clears `parts`.  img16, img8: null when no matrix reads that form; both null: no image.
+constexpr int KQ_TOK16 = 544, KQ_TOK8 = 256;
+struct KqTokenImage {
+    uint8_t *img16, *img8;
+    float *da;
+    int4 *parts;
+    int32_t n_parts, m_pad, n_tok;
+};
+#ifdef __CUDACC__
+// one token's part of a group of eight, by one warp: p16 / p8 point at the token's 16 bytes of the group's first chunk; chunks are `pitch` bytes apart
+__device__ __forceinline__ void kq_image_put(uint8_t *p16, uint8_t *p8, int pitch, int lane, const KqQ8Codes &o) {
+    if (p16) {
+        __half2 h[4];
+#pragma unroll
+        for (int i = 0; i < 4; i++) h[i] = __halves2half2(__int2half_rn(o.c[(i >> 1) * 4 + (i & 1)]), __int2half_rn(o.c[(i >> 1) * 4 + (i & 1) + 2]));
+        *reinterpret_cast<uint4 *>(p16 + lane * pitch) = *reinterpret_cast<const uint4 *>(&h[0]);
+        if ((lane & 1) == 0) // sum j = lane / 2: |.| <= 2032, exact
+            *reinterpret_cast<__half *>(p16 + (32 + ((lane >> 1) & 1)) * pitch + (lane >> 2) * 2) = __int2half_rn(o.sum);
+    }
+    if (p8) *reinterpret_cast<uint2 *>(p8 + (lane >> 1) * pitch + (lane & 1) * 8) = o.pk;
 }
 #endif
 
@@ -307,6 +344,13 @@ b200_status kq_launch_gemv_stream(const KqGemvSeg *segs, int nseg, const int8_t 
 bool kq_gemv_batch_parts(uint32_t type, int64_t K); // 5 to 8 tokens of K values take launches over ranges of K
 b200_status kq_rms_norm(const float *x, const float *w, int64_t T, int64_t h, float eps, float *y, int8_t *q,
                         float *d, int16_t *bs, cudaStream_t st, int64_t x_row_stride);
+// Where the tokens of a product may be written by the kernel that makes them, as the product reads them; *im without an image when they go out in the usual form instead
+bool kq_gemm_takes_images();
+b200_status kq_gemm_image(const KqGemvSeg *segs, int nseg, int64_t M, int64_t K, cudaStream_t st, KqTokenImage *im);
+b200_status kq_launch_gemm_image(const KqGemvSeg *segs, int nseg, const KqTokenImage &im, int64_t K, const float *residual, cudaStream_t st);
+b200_status kq_rms_norm_image(const float *x, const float *w, int64_t h, float eps, const KqTokenImage &im, cudaStream_t st);
+// x, or silu(x) * up, of [im.n_tok][K]; y (may be x): the latter in f32
+b200_status kq_act_image(const float *x, const float *up, float *y, int64_t K, const KqTokenImage &im, cudaStream_t st);
 // MUL_MAT_ID over many tokens: stable expert-major order of the (token, slot) pairs, then one grouped
 // launch of the tensor-core GEMM per expert-packed matrix (y[pair][N] = W[expert(pair)] . x[pair / act_div])
 size_t kq_moe_sort_scratch_bytes(int64_t n_pairs, int64_t E);

@@ -8,14 +8,18 @@
 b200_status kq_launch_gemm_tc(const KqGemvSeg *segs, int nseg, const int8_t *q, const float *d, const int16_t *bs, int64_t M, int64_t K,
                               const float *residual, cudaStream_t st);
 
-b200_status kq_launch_gemm(const KqGemvSeg *segs, int nseg, const int8_t *q, const float *d, const int16_t *bs, int64_t M, int64_t K,
-                           const float *residual, cudaStream_t st) {
+bool kq_gemm_takes_images() { // the tensor-core product is on
     static int use_tc = -1;
     if (use_tc < 0) {
         const char *v = getenv("B200_GEMM_TC");
         use_tc = !(v && v[0] == '0');
     }
-    if (use_tc) return kq_launch_gemm_tc(segs, nseg, q, d, bs, M, K, residual, st);
+    return use_tc != 0;
+}
+
+b200_status kq_launch_gemm(const KqGemvSeg *segs, int nseg, const int8_t *q, const float *d, const int16_t *bs, int64_t M, int64_t K,
+                           const float *residual, cudaStream_t st) {
+    if (kq_gemm_takes_images()) return kq_launch_gemm_tc(segs, nseg, q, d, bs, M, K, residual, st);
     const int64_t nb = K / 256;
     for (int i = 0; i < nseg; i++)
         for (int64_t m0 = 0; m0 < M; m0 += 8) {

@@ -50,7 +50,7 @@ namespace {
 
 constexpr int NTHREADS = 512, CHUNK = 64, MAX_CHUNKS = 4, ROWS = 128, DA_RING = 8, SC_RING = 8;
 // bytes of a token and block in an image: 256 f16 codes and 16 f16 sums (Q4_K), or 256 codes (Q6_K); eight tokens are [chunks of 16 bytes][8 tokens]
-constexpr int TOK16 = 544, TOK8 = 256;
+constexpr int TOK16 = KQ_TOK16, TOK8 = KQ_TOK8;
 constexpr int TILE_OUT = MAX_CHUNKS * CHUNK * ROWS; // outputs of a tile
 constexpr int MAX_CTAS = 256, MAX_DEVICES = 16, DRAIN_WARPS = 8;
 constexpr uint64_t LIMIT = 5 * KQ_WAIT_LIMIT_NS;
@@ -844,12 +844,14 @@ constexpr int64_t SLAB_BYTES = 64 << 20, GROUP_BYTES = 256 << 20; // images of o
 struct Scratch {
     uint8_t *img16, *img8;
     float *da, *part;
+    int4 *parts_done;
 };
 b200_status scratch(int dev, size_t img16_bytes, size_t img8_bytes, size_t da_bytes, cudaStream_t st, Scratch *out) {
     static std::mutex mu;
     static void *buf[MAX_DEVICES][4];
     static size_t cap[MAX_DEVICES][4];
     static bool captured[MAX_DEVICES][4], attr[MAX_DEVICES];
+    static int4 *parts_done[MAX_DEVICES];
     std::lock_guard<std::mutex> lock(mu);
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     KQ_CUDA(cudaStreamIsCapturing(st, &cs));
@@ -902,9 +904,10 @@ b200_status scratch(int dev, size_t img16_bytes, size_t img8_bytes, size_t da_by
         KQ_TRY(prepare((const void *)gemm_kq_kernel<false, true>, Cfg<false, true>::SMEM, Cfg<false, true>::REG_SUM));
         KQ_TRY(prepare((const void *)gemm_kq_kernel<true, false>, Cfg<true, false>::SMEM, Cfg<true, false>::REG_SUM));
         KQ_TRY(prepare((const void *)gemm_kq_kernel<true, true>, Cfg<true, true>::SMEM, Cfg<true, true>::REG_SUM));
+        KQ_CUDA(cudaGetSymbolAddress((void **)&parts_done[dev], g_parts_done));
         attr[dev] = true;
     }
-    *out = {img16_bytes ? (uint8_t *)buf[dev][0] : nullptr, img8_bytes ? (uint8_t *)buf[dev][1] : nullptr, (float *)buf[dev][2], (float *)buf[dev][3]};
+    *out = {img16_bytes ? (uint8_t *)buf[dev][0] : nullptr, img8_bytes ? (uint8_t *)buf[dev][1] : nullptr, (float *)buf[dev][2], (float *)buf[dev][3], parts_done[dev]};
     return B200_OK;
 }
 
@@ -1037,6 +1040,41 @@ int kq_gemm_error_fetch() {
 // Tokens whose images are held at a time: every row tile reads the images again, so they should stay in L2 (126 MB) beside the weights that
 // stream by.  2048 and 4096 tokens x 8192 x 28672 in Q4_K, 125 and 250 MB at once: 1363 and 2788 us; in slabs of 62 MB 1200 and 2406.
 constexpr int64_t SLAB_MIN = MAX_CHUNKS * CHUNK;
+static int64_t slab_tokens(int64_t per_token) { return std::max(SLAB_MIN, SLAB_BYTES / per_token / SLAB_MIN * SLAB_MIN); }
+static int32_t padded_tokens(const KqGemvSeg *segs, int nseg, int64_t M, int64_t nb) {
+    int32_t pad = 0;
+    for (const uint32_t type : {(uint32_t)B200_TYPE_Q4_K, (uint32_t)B200_TYPE_Q6_K}) {
+        const TokTiles t = token_tiles_of(type, segs, nseg, M, nb);
+        pad = std::max(pad, t.n * t.tok);
+    }
+    return pad;
+}
+
+b200_status kq_gemm_image(const KqGemvSeg *segs, int nseg, int64_t M, int64_t K, cudaStream_t st, KqTokenImage *im) {
+    *im = KqTokenImage{};
+    int dev = 0;
+    KQ_TRY(check_segs(segs, nseg, nullptr, K, &dev));
+    const int64_t nb = K / 256;
+    if (M > slab_tokens(token_bytes(segs, nseg, nb, false) + token_bytes(segs, nseg, nb, true))) return B200_OK; // in slabs
+    const int32_t pad = padded_tokens(segs, nseg, M, nb);
+    Scratch sc;
+    const b200_status rc = scratch_for(dev, segs, nseg, pad, nb, st, &sc);
+    if (rc != B200_OK) return rc == B200_ERR_ALLOC ? B200_OK : rc;
+    *im = {sc.img16, sc.img8, sc.da, sc.parts_done, 2 * MAX_CTAS * DRAIN_WARPS / 4, pad, (int32_t)M};
+    return B200_OK;
+}
+
+b200_status kq_launch_gemm_image(const KqGemvSeg *segs, int nseg, const KqTokenImage &im, int64_t K, const float *residual, cudaStream_t st) {
+    int dev = 0;
+    KQ_TRY(check_segs(segs, nseg, nullptr, K, &dev));
+    KQ_REQUIRE(im.n_tok > 0 && (im.img16 || im.img8) && (!residual || nseg == 1), "gemm: bad shape");
+    Params p = {};
+    p.M = im.n_tok, p.nb = (int32_t)(K / 256), p.m_pad = im.m_pad, p.residual = residual;
+    Scratch sc;
+    KQ_TRY(scratch_for(dev, segs, nseg, im.m_pad, p.nb, st, &sc)); // the buffers that kq_gemm_image gave
+    KQ_REQUIRE(sc.img16 == im.img16 && sc.img8 == im.img8 && sc.da == im.da, "gemm: another call came between a token image and its product");
+    return launch_segs(p, false, sc, segs, nseg, 1, K, st);
+}
 
 b200_status kq_launch_gemm_tc(const KqGemvSeg *segs, int nseg, const int8_t *q, const float *d, const int16_t *bs, int64_t M, int64_t K,
                               const float *residual, cudaStream_t st) {
@@ -1045,16 +1083,13 @@ b200_status kq_launch_gemm_tc(const KqGemvSeg *segs, int nseg, const int8_t *q, 
     KQ_REQUIRE(M > 0 && (!residual || nseg == 1), "gemm: bad shape");
     const int64_t nb = K / 256;
     const int64_t per_token = token_bytes(segs, nseg, nb, false) + token_bytes(segs, nseg, nb, true);
-    int64_t slab = std::max(SLAB_MIN, SLAB_BYTES / per_token / SLAB_MIN * SLAB_MIN);
+    int64_t slab = slab_tokens(per_token);
     for (int64_t m0 = 0, mc; m0 < M; m0 += mc) {
         mc = kq_div_up(M - m0, kq_div_up(M - m0, slab)); // of equal size
         if (mc < M - m0) mc = kq_div_up(mc, SLAB_MIN) * SLAB_MIN;
         Params p = {};
         p.M = (int32_t)mc, p.nb = (int32_t)nb;
-        for (const uint32_t type : {(uint32_t)B200_TYPE_Q4_K, (uint32_t)B200_TYPE_Q6_K}) {
-            const TokTiles t = token_tiles_of(type, segs, nseg, mc, nb);
-            p.m_pad = std::max(p.m_pad, t.n * t.tok);
-        }
+        p.m_pad = padded_tokens(segs, nseg, mc, nb);
         Scratch sc;
         const b200_status rc = scratch_for(dev, segs, nseg, p.m_pad, nb, st, &sc);
         if (rc == B200_ERR_ALLOC && mc > SLAB_MIN) { // no room for these images: fewer at a time

@@ -41,12 +41,135 @@ __global__ void __launch_bounds__(128) swiglu_quantize_kernel(const float *g, co
     kq_quantize_block_warp(v, lane, q + blk * 256, d + blk, bs + blk * 16);
 }
 
-// RMSNorm (x * rsqrt(mean(x^2) + eps) * w) with optional f32 output and optional Q8 output.
-// One CTA of 256 threads per row; h is a multiple of 256 when q != null.
-__global__ void __launch_bounds__(256) rms_norm_kernel(const float *x,
-                                                       const float *w, int h, float eps,
-                                                       float *y, int8_t *q, float *d, int16_t *bs,
-                                                       int64_t x_row_stride) {
+// The same for the tensor-core product: eight tokens of a block per CTA, a warp each, gathered in shared memory so that the image is written in full lines.
+// With UP silu(x) * up.  A pass over the codes and a launch less than codes first, image then.
+template <bool UP>
+__global__ void __launch_bounds__(256) act_to_image_kernel(const float *x, const float *up, float *y, int64_t K, const __grid_constant__ KqTokenImage im) {
+    KQ_PDL_ENTER();
+    constexpr int PITCH = 144; // chunks of 128 bytes, 16 further apart: a warp's stores fall on different banks
+    __shared__ __align__(16) uint8_t s16[34 * PITCH], s8[16 * PITCH];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, b = blockIdx.y, t0 = blockIdx.x * 8, t = t0 + warp;
+    if (blockIdx.x == 0 && b == 0)
+        for (int i = tid; i < im.n_parts; i += 256) im.parts[i] = make_int4(0, 0, 0, 0);
+    float v[8] = {};
+    if (t < im.n_tok) {
+        const int64_t at = t * K + b * 256 + lane * 8;
+        const float4 x0 = *reinterpret_cast<const float4 *>(x + at), x1 = *reinterpret_cast<const float4 *>(x + at + 4);
+        v[0] = x0.x, v[1] = x0.y, v[2] = x0.z, v[3] = x0.w, v[4] = x1.x, v[5] = x1.y, v[6] = x1.z, v[7] = x1.w;
+        if (UP) {
+            const float4 u0 = *reinterpret_cast<const float4 *>(up + at), u1 = *reinterpret_cast<const float4 *>(up + at + 4);
+            const float u[8] = {u0.x, u0.y, u0.z, u0.w, u1.x, u1.y, u1.z, u1.w};
+#pragma unroll
+            for (int i = 0; i < 8; i++) v[i] = (v[i] / (1.0f + expf(-v[i]))) * u[i];
+            if (y) {
+                *reinterpret_cast<float4 *>(y + at) = make_float4(v[0], v[1], v[2], v[3]);
+                *reinterpret_cast<float4 *>(y + at + 4) = make_float4(v[4], v[5], v[6], v[7]);
+            }
+        }
+    }
+    const KqQ8Codes o = kq_quantize_codes_warp(v); // of zeros: zeros
+    kq_image_put(im.img16 ? s16 + warp * 16 : nullptr, im.img8 ? s8 + warp * 16 : nullptr, PITCH, lane, o);
+    if (lane == 0) im.da[(int64_t)b * im.m_pad + t] = o.d;
+    __syncthreads();
+    const int64_t group = (int64_t)b * im.m_pad + t0;
+    if (im.img16)
+        for (int i = tid; i < 34 * 8; i += 256)
+            *reinterpret_cast<uint4 *>(im.img16 + group * KQ_TOK16 + i * 16) = *reinterpret_cast<const uint4 *>(s16 + (i >> 3) * PITCH + (i & 7) * 16);
+    if (im.img8)
+        for (int i = tid; i < 16 * 8; i += 256)
+            *reinterpret_cast<uint4 *>(im.img8 + group * KQ_TOK8 + i * 16) = *reinterpret_cast<const uint4 *>(s8 + (i >> 3) * PITCH + (i & 7) * 16);
+}
+
+// RMSNorm and Q8 of a row, W warps: a warp holds up to two of the row's blocks in registers, so that the row is read once, the weights before the
+// kernel waits for the one that writes the row.  Outputs: f32 (y), Q8 (q, d, bs), an image; rows past im.n_tok are zeros of the image.  The sum of squares is
+// carried in double so that the scale does not depend on the order of the reduction: the normalised values, and with them the Q8 codes, are then
+// reproducible.
+template <int W>
+__global__ void __launch_bounds__(W * 32) rms_norm_q8_kernel(const float *x, const float *w, int h, float eps, float *y, int8_t *q, float *d, int16_t *bs,
+                                                             int64_t x_row_stride, const __grid_constant__ KqTokenImage im) {
+    constexpr int R = 2;
+    __shared__ double part[W];
+    const int row = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nb = h / 256;
+    const bool image = im.img16 || im.img8, live = !image || row < im.n_tok;
+    const float *xr = x + (int64_t)row * x_row_stride;
+    KQ_PDL_TRIGGER();
+    float g[R][8], v[R][8];
+    auto load = [&](const float *p, int b, float (&o)[8]) {
+        const float4 a = *reinterpret_cast<const float4 *>(p + b * 256 + lane * 8), c = *reinterpret_cast<const float4 *>(p + b * 256 + lane * 8 + 4);
+        o[0] = a.x, o[1] = a.y, o[2] = a.z, o[3] = a.w, o[4] = c.x, o[5] = c.y, o[6] = c.z, o[7] = c.w;
+    };
+    auto weights = [&](int b, float (&o)[8]) {
+#pragma unroll
+        for (int i = 0; i < 8; i++) o[i] = 1.0f;
+        if (w && b < nb) load(w, b, o);
+    };
+#pragma unroll
+    for (int r = 0; r < R; r++) weights(warp + r * W, g[r]);
+    KQ_PDL_WAIT();
+    if (image && row == 0)
+        for (int i = tid; i < im.n_parts; i += W * 32) im.parts[i] = make_int4(0, 0, 0, 0);
+    double ss = 0.0;
+#pragma unroll
+    for (int r = 0; r < R; r++) {
+#pragma unroll
+        for (int i = 0; i < 8; i++) v[r][i] = 0.f;
+        if (live && warp + r * W < nb) load(xr, warp + r * W, v[r]);
+    }
+    auto add = [&](const float (&u)[8]) {
+#pragma unroll
+        for (int i = 0; i < 8; i++) ss += (double)u[i] * u[i];
+    };
+#pragma unroll
+    for (int r = 0; r < R; r++) add(v[r]);
+    if (live)
+        for (int b = warp + R * W; b < nb; b += W) {
+            float u[8];
+            load(xr, b, u);
+            add(u);
+        }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+    if (lane == 0) part[warp] = ss;
+    __syncthreads();
+    double t = 0.0;
+#pragma unroll
+    for (int i = 0; i < W; i++) t += part[i];
+    const float scale = 1.0f / sqrtf((float)(t / (double)h) + eps);
+    auto emit = [&](int b, const float (&u)[8], const float (&f)[8]) {
+        float n[8];
+#pragma unroll
+        for (int i = 0; i < 8; i++) n[i] = live ? u[i] * scale * f[i] : 0.f;
+        if (y && live) {
+            float *yo = y + (int64_t)row * h + b * 256 + lane * 8;
+            *reinterpret_cast<float4 *>(yo) = make_float4(n[0], n[1], n[2], n[3]);
+            *reinterpret_cast<float4 *>(yo + 4) = make_float4(n[4], n[5], n[6], n[7]);
+        }
+        const KqQ8Codes o = kq_quantize_codes_warp(n);
+        const int64_t gb = (int64_t)row * nb + b;
+        if (q && live) {
+            *reinterpret_cast<uint2 *>(q + gb * 256 + lane * 8) = o.pk;
+            if ((lane & 1) == 0) bs[gb * 16 + (lane >> 1)] = (int16_t)o.sum;
+            if (lane == 0) d[gb] = o.d;
+        }
+        if (image) {
+            const int64_t group = (int64_t)b * im.m_pad + (row & ~7);
+            kq_image_put(im.img16 ? im.img16 + group * KQ_TOK16 + (row & 7) * 16 : nullptr, im.img8 ? im.img8 + group * KQ_TOK8 + (row & 7) * 16 : nullptr, 128, lane, o);
+            if (lane == 0) im.da[(int64_t)b * im.m_pad + row] = o.d;
+        }
+    };
+#pragma unroll
+    for (int r = 0; r < R; r++)
+        if (warp + r * W < nb) emit(warp + r * W, v[r], g[r]);
+    for (int b = warp + R * W; b < nb; b += W) {
+        float u[8] = {}, f[8];
+        if (live) load(xr, b, u);
+        weights(b, f);
+        emit(b, u, f);
+    }
+}
+
+// RMSNorm (x * rsqrt(mean(x^2) + eps) * w) of rows of any length, f32 output.  One CTA of 256 threads per row.
+__global__ void __launch_bounds__(256) rms_norm_kernel(const float *x, const float *w, int h, float eps, float *y, int64_t x_row_stride) {
     KQ_PDL_ENTER();
     __shared__ double part[8];
     __shared__ float s_scale;
@@ -70,26 +193,7 @@ __global__ void __launch_bounds__(256) rms_norm_kernel(const float *x,
     }
     __syncthreads();
     const float scale = s_scale;
-    if (q) {
-        const int nb = h / 256;
-        for (int b = warp; b < nb; b += 8) {
-            const int o = b * 256 + lane * 8;
-            const float4 a = *reinterpret_cast<const float4 *>(xr + o);
-            const float4 c = *reinterpret_cast<const float4 *>(xr + o + 4);
-            float v[8] = {a.x, a.y, a.z, a.w, c.x, c.y, c.z, c.w};
-#pragma unroll
-            for (int i = 0; i < 8; i++) v[i] = v[i] * scale * (w ? w[o + i] : 1.0f);
-            if (y) {
-                float *yo = y + (int64_t)row * h + o;
-                *reinterpret_cast<float4 *>(yo) = make_float4(v[0], v[1], v[2], v[3]);
-                *reinterpret_cast<float4 *>(yo + 4) = make_float4(v[4], v[5], v[6], v[7]);
-            }
-            const int64_t gb = (int64_t)row * nb + b;
-            kq_quantize_block_warp(v, lane, q + gb * 256, d + gb, bs + gb * 16);
-        }
-    } else {
-        for (int i = tid; i < h; i += 256) y[(int64_t)row * h + i] = xr[i] * scale * (w ? w[i] : 1.0f);
-    }
+    for (int i = tid; i < h; i += 256) y[(int64_t)row * h + i] = xr[i] * scale * (w ? w[i] : 1.0f);
 }
 
 // Rows of up to 128 values (one head), f32 output only: a warp per row, with the sums in the order of the kernel above, which gives such a row
@@ -293,6 +397,29 @@ b200_status kq_synth_weights(uint32_t type, void *W, int64_t n_rows, int64_t K, 
     return B200_OK;
 }
 
+// 8 warps for rows of up to 4096, 16 for longer ones
+static b200_status norm_q8(const float *x, const float *w, int64_t rows, int64_t h, float eps, float *y, int8_t *q, float *d, int16_t *bs, int64_t ldx,
+                           const KqTokenImage &im, cudaStream_t st) {
+    if (h <= 4096) kq_launch(rms_norm_q8_kernel<8>, (unsigned)rows, 256, 0, st, x, w, (int)h, eps, y, q, d, bs, ldx, im);
+    else kq_launch(rms_norm_q8_kernel<16>, (unsigned)rows, 512, 0, st, x, w, (int)h, eps, y, q, d, bs, ldx, im);
+    KQ_COUNT_LAUNCH();
+    KQ_LAUNCH_CHECK();
+    return B200_OK;
+}
+b200_status kq_rms_norm_image(const float *x, const float *w, int64_t h, float eps, const KqTokenImage &im, cudaStream_t st) {
+    KQ_REQUIRE(h > 0 && h % 256 == 0 && im.m_pad > 0, "rms_norm: bad shape");
+    return norm_q8(x, w, im.m_pad, h, eps, nullptr, nullptr, nullptr, nullptr, h, im, st);
+}
+b200_status kq_act_image(const float *x, const float *up, float *y, int64_t K, const KqTokenImage &im, cudaStream_t st) {
+    KQ_REQUIRE(K > 0 && K % 256 == 0 && im.m_pad % 8 == 0 && ((uintptr_t)x & 15) == 0 && (((uintptr_t)up | (uintptr_t)y) & 15) == 0, "act_image: bad shape");
+    const dim3 grid((unsigned)(im.m_pad / 8), (unsigned)(K / 256));
+    if (up) kq_launch(act_to_image_kernel<true>, grid, dim3(256), 0, st, x, up, y, K, im);
+    else kq_launch(act_to_image_kernel<false>, grid, dim3(256), 0, st, x, up, y, K, im);
+    KQ_COUNT_LAUNCH();
+    KQ_LAUNCH_CHECK();
+    return B200_OK;
+}
+
 b200_status kq_rms_norm(const float *x, const float *w, int64_t T, int64_t h, float eps, float *y,
                         int8_t *q, float *d, int16_t *bs, cudaStream_t st, int64_t x_row_stride) {
     KQ_REQUIRE(T > 0 && h > 0 && h % 4 == 0, "rms_norm: bad shape");
@@ -305,7 +432,8 @@ b200_status kq_rms_norm(const float *x, const float *w, int64_t T, int64_t h, fl
         KQ_LAUNCH_CHECK();
         return B200_OK;
     }
-    kq_launch(rms_norm_kernel, (unsigned)T, 256, 0, st, x, w, (int)h, eps, y, q, d, bs, x_row_stride ? x_row_stride : h);
+    if (q) return norm_q8(x, w, T, h, eps, y, q, d, bs, ldx, KqTokenImage{}, st);
+    kq_launch(rms_norm_kernel, (unsigned)T, 256, 0, st, x, w, (int)h, eps, y, ldx);
     KQ_COUNT_LAUNCH();
     KQ_LAUNCH_CHECK();
     return B200_OK;

@@ -211,6 +211,11 @@ b200_status forward_body(b200_stage *st, const int32_t *tokens, const float *hid
     const int h = c.n_embd, hd = c.head_dim, nq = c.n_head * hd, nkv = c.n_head_kv * hd;
     const int64_t seq_stride = (int64_t)c.n_ctx * nkv;
     const int32_t *pos_dev = pos_from_dev ? st->pos0_dev : nullptr;
+    // the place of a product's tokens where the kernel that makes them may write them as the product reads them; otherwise none
+    auto image = [&](const KqGemvSeg *segs, int n, int64_t K, KqTokenImage *im) {
+        *im = {};
+        return rows > 8 && classes == CLS_ALL && kq_gemm_takes_images() ? kq_gemm_image(segs, n, rows, K, s, im) : B200_OK;
+    };
     const float *xin;
     if (c.has_embd) {
         OTHER_(b200_get_rows(st->tok_embd->type, st->tok_embd->dev, tokens, rows, h, st->x, s));
@@ -229,13 +234,20 @@ b200_status forward_body(b200_stage *st, const int32_t *tokens, const float *hid
         const KqKvTypes kvt = st->kvt;
         // ---- attention block
         const bool fuse = rows <= 2; // the streaming GEMV normalises and quantises its own input
-        if (!fuse) OTHER_(kq_rms_norm(xin, L.attn_norm, rows, h, c.rms_eps, nullptr, st->aq, st->ad, st->abs16, s));
         KqGemvSeg segs[3] = {
             {(const uint8_t *)L.wq->dev, L.wq->type, nq, st->q, L.bq, nq, 0},
             {(const uint8_t *)L.wk->dev, L.wk->type, nkv, st->k, L.bk, nkv, 0},
             {(const uint8_t *)L.wv->dev, L.wv->type, nkv, st->v, L.bv, nkv, 0},
         };
-        if (rows <= 8) {
+        KqTokenImage im = {};
+        // The norm writes the image itself for up to 256 rows: a row's part of it is scattered, 16 bytes to a line, which costs more
+        // than the launch it saves where there are many (kq_rms_norm_image)
+        if (rows <= 256) KQ_TRY(image(segs, 3, h, &im));
+        if (im.n_tok) KQ_TRY(kq_rms_norm_image(xin, L.attn_norm, h, c.rms_eps, im, s));
+        else if (!fuse) OTHER_(kq_rms_norm(xin, L.attn_norm, rows, h, c.rms_eps, nullptr, st->aq, st->ad, st->abs16, s));
+        if (im.n_tok) {
+            KQ_TRY(kq_launch_gemm_image(segs, 3, im, h, nullptr, s));
+        } else if (rows <= 8) {
             KqActPrep pr = {xin, L.attn_norm, c.rms_eps, 1};
             GEMV_(kq_launch_gemv(segs, 3, st->aq, st->ad, st->abs16, rows, h, nullptr, 0, nullptr, s,
                                  fuse ? &pr : nullptr));
@@ -305,8 +317,15 @@ b200_status forward_body(b200_stage *st, const int32_t *tokens, const float *hid
             KqActPrep pr = {st->att, nullptr, 0.f, 0};
             GEMV_(kq_launch_gemv(&so, 1, st->aq, st->ad, st->abs16, rows, nq, xin, 0, nullptr, s, &pr));
         } else {
-            OTHER_(b200_quantize_act(st->att, rows, nq, st->aq, st->ad, st->abs16, s));
-            GEMV_(mm(st, L.wo, rows, st->x, nullptr, xin, s)); // x = xin + Wo.att
+            const KqGemvSeg so = {(const uint8_t *)L.wo->dev, L.wo->type, h, st->x, nullptr, h, 0};
+            KQ_TRY(image(&so, 1, nq, &im));
+            if (im.n_tok) {
+                KQ_TRY(kq_act_image(st->att, nullptr, nullptr, nq, im, s));
+                KQ_TRY(kq_launch_gemm_image(&so, 1, im, nq, xin, s));
+            } else {
+                OTHER_(b200_quantize_act(st->att, rows, nq, st->aq, st->ad, st->abs16, s));
+                GEMV_(mm(st, L.wo, rows, st->x, nullptr, xin, s)); // x = xin + Wo.att
+            }
         }
         // ---- feed-forward block
         if (ffn_done) {
@@ -361,7 +380,7 @@ b200_status forward_body(b200_stage *st, const int32_t *tokens, const float *hid
                 KQ_TRY(kq_moe_sort(st->rid, pairs, E, st->moe_sorted, st->moe_sorted_bytes, s));
                 const KqGemvSeg both[2] = {gu[0], {gu[1].W, gu[1].type, fe, st->hp2, nullptr, fe, kq_device_row_bytes(gu[1].type, h) * fe}};
                 KQ_TRY(kq_launch_gemm_grouped(both, 2, st->aq, st->ad, st->abs16, ku, pairs, E, h, st->moe_sorted, s));
-                KQ_TRY(kq_swiglu_quantize(st->hp, st->hp2, pairs, fe, st->hp, st->aq, st->ad, st->abs16, s));
+                KQ_TRY(kq_swiglu_quantize(st->hp, st->hp2, pairs, fe, nullptr, st->aq, st->ad, st->abs16, s));
                 const KqGemvSeg down = {(const uint8_t *)L.down_e->dev, L.down_e->type, h, st->yp, nullptr, h, dstride};
                 KQ_TRY(kq_launch_gemm_grouped(&down, 1, st->aq, st->ad, st->abs16, 1, pairs, E, fe, st->moe_sorted, s));
             } else {
@@ -392,12 +411,16 @@ b200_status forward_body(b200_stage *st, const int32_t *tokens, const float *hid
             KQ_LAUNCH_CHECK();
             }
         } else {
-            if (!fuse) OTHER_(kq_rms_norm(st->x, L.ffn_norm, rows, h, c.rms_eps, nullptr, st->aq, st->ad, st->abs16, s));
             KqEmitQ8 emit = {st->aq, st->ad, st->abs16, st->emit_counters, 0};
             KqGemvSeg gu[2] = {
                 {(const uint8_t *)L.gate->dev, L.gate->type, c.n_ff, st->g, nullptr, c.n_ff, 0},
                 {(const uint8_t *)L.up->dev, L.up->type, c.n_ff, rows <= 8 ? st->g : st->u, nullptr, c.n_ff, 0},
             };
+            im = {};
+            if (rows <= 256) KQ_TRY(image(gu, 2, h, &im));
+            if (im.n_tok) KQ_TRY(kq_rms_norm_image(st->x, L.ffn_norm, h, c.rms_eps, im, s));
+            else if (!fuse) OTHER_(kq_rms_norm(st->x, L.ffn_norm, rows, h, c.rms_eps, nullptr, st->aq, st->ad, st->abs16, s));
+            bool down_done = false;
             if (rows <= 8) {
                 KqActPrep pr = {st->x, L.ffn_norm, c.rms_eps, 1};
                 // the launch also leaves the Q8 form of its output for the down projection (B200_GEMV_EMIT_Q8=0: off)
@@ -406,11 +429,21 @@ b200_status forward_body(b200_stage *st, const int32_t *tokens, const float *hid
                 GEMV_(kq_launch_gemv(gu, 2, st->aq, st->ad, st->abs16, rows, h, nullptr, 1, nullptr, s,
                                      fuse ? &pr : nullptr, want ? &emit : nullptr));
             } else {
-                GEMV_(kq_launch_gemm(gu, 2, st->aq, st->ad, st->abs16, rows, h, nullptr, s));
-                // SwiGLU and the Q8 form the down projection reads, in one pass
-                OTHER_(kq_swiglu_quantize(st->g, st->u, rows, c.n_ff, st->g, st->aq, st->ad, st->abs16, s));
+                if (im.n_tok) KQ_TRY(kq_launch_gemm_image(gu, 2, im, h, nullptr, s));
+                else GEMV_(kq_launch_gemm(gu, 2, st->aq, st->ad, st->abs16, rows, h, nullptr, s));
+                // SwiGLU and the form the down projection reads, in one pass
+                const KqGemvSeg sd = {(const uint8_t *)L.down->dev, L.down->type, h, xout, nullptr, h, 0};
+                KQ_TRY(image(&sd, 1, c.n_ff, &im));
+                if (im.n_tok) {
+                    KQ_TRY(kq_act_image(st->g, st->u, st->g, c.n_ff, im, s));
+                    KQ_TRY(kq_launch_gemm_image(&sd, 1, im, c.n_ff, st->x, s));
+                    down_done = true;
+                } else {
+                    OTHER_(kq_swiglu_quantize(st->g, st->u, rows, c.n_ff, st->g, st->aq, st->ad, st->abs16, s));
+                }
             }
-            if (fuse && emit.done) {
+            if (down_done) {
+            } else if (fuse && emit.done) {
                 GEMV_(mm(st, L.down, rows, xout, nullptr, st->x, s)); // reads the Q8 form the gate / up launch wrote
             } else if (fuse) {
                 KqGemvSeg sd = {(const uint8_t *)L.down->dev, L.down->type, h, xout, nullptr, h, 0};

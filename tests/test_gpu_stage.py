@@ -425,3 +425,21 @@ def test_down_projection_input_quantised_by_the_gate_up_launch(cfg, n_seq, monke
         outs.append(torch.stack([g[-n_seq:] if g.shape[0] > n_seq else g for g in got[1:]]))
         st.close()
     assert torch.equal(outs[0], outs[1])
+
+
+@pytest.mark.parametrize("cfg", [DENSE, LLAMA, MOE], ids=["qwen2-dense", "llama-dense", "qwen3-moe"])
+@pytest.mark.parametrize("T", [9, 16, 23, 255, 257])
+def test_rows_written_as_token_images(cfg, T):
+    """products of more than 8 rows read an image of their tokens that the norm (up to 256 rows), the quantiser or the SwiGLU writes: rows that fill groups of
+    eight and tiles or do not, on both sides of 256, each layer's segments against the oracle from the same input"""
+    from layer_oracle import LayerOracle
+    from test_gpu_real_widths import check_layer
+
+    cfg = dict(cfg, n_ctx=288)
+    full = orc.Model(**cfg)
+    full.generate(31)
+    x = (np.random.default_rng(T).standard_normal((T, cfg["n_embd"])) * 0.02).astype(np.float32)
+    for l in range(2):
+        _, st = _load_range(cfg, full, l, l + 1, n_ubatch=288)
+        x, _, _, _ = check_layer("small", f"layer {l}, {T} rows", cfg, LayerOracle(full, cfg, l), st, x, 0)
+        st.close()
