@@ -726,7 +726,7 @@ __global__ void __launch_bounds__(288) act_image_kernel(const __grid_constant__ 
 // expert's token tiles; every expert starts on a tile boundary, the rows behind its last pair are
 // padding (-1).  One CTA of 16 warps; warp w walks a contiguous range of the pairs 32 at a time, so the
 // order inside an expert is the pair order whatever the timing (with 8 warps and a serial table of tiles 55 us
-// for 8192 pairs and 128 experts, now 27).  Output: n_tiles, the expert of each
+// for 8192 pairs and 128 experts, with 16 and a parallel table 27, with the experts asked for ahead and compared once 17).  Output: n_tiles, the expert of each
 // tile, and for each tile row the pair it holds.
 constexpr int SORT_WARPS = 16, SORT_MAX_E = 256;
 __global__ void __launch_bounds__(SORT_WARPS * 32) moe_sort_kernel(const int32_t *ids, int n_pairs, int E, int TM,
@@ -741,13 +741,29 @@ __global__ void __launch_bounds__(SORT_WARPS * 32) moe_sort_kernel(const int32_t
     __syncthreads();
     const int chunk = ((n_pairs + SORT_WARPS - 1) / SORT_WARPS + 31) & ~31;
     const int begin = min(n_pairs, warp * chunk), end = min(n_pairs, begin + chunk);
-    for (int i = begin; i < end; i += 32) {
-        const int pr = i + lane;
-        int e = pr < end ? ids[pr] : -1;
-        if (e < 0 || e >= E) e = -1; // not an expert of this table: the pair is dropped
-        const unsigned same = __match_any_sync(0xffffffffu, e);
-        if (e >= 0 && lane == __ffs(same) - 1) cnt[warp][e] += __popc(same);
-        __syncwarp();
+    // experts of the warp's pairs from i on, AHEAD runs of 32: asked for together, since a run's own trip to L2 would take longer than its work
+    constexpr int AHEAD = 16;
+    int ex[AHEAD];
+    unsigned mates[AHEAD]; // the run's pairs of the same expert: found once, by pairs that fit (with some thirty experts in a run it takes longer than the rest)
+    const bool once = end - begin <= AHEAD * 32;
+    auto fetch = [&](int i) {
+#pragma unroll
+        for (int j = 0; j < AHEAD; j++) {
+            const int pr = i + j * 32 + lane;
+            const int e = pr < end ? ids[pr] : -1;
+            ex[j] = e < E ? max(e, -1) : -1; // not an expert of this table: the pair is dropped
+        }
+    };
+    for (int i0 = begin; i0 < end; i0 += AHEAD * 32) {
+        fetch(i0);
+#pragma unroll
+        for (int j = 0; j < AHEAD; j++) {
+            if (i0 + j * 32 >= end) break;
+            const int e = ex[j];
+            const unsigned same = mates[j] = __match_any_sync(0xffffffffu, e);
+            if (e >= 0 && lane == __ffs(same) - 1) cnt[warp][e] += __popc(same);
+            __syncwarp();
+        }
     }
     __syncthreads();
     if ((int)threadIdx.x < E) {
@@ -783,21 +799,28 @@ __global__ void __launch_bounds__(SORT_WARPS * 32) moe_sort_kernel(const int32_t
     }
     __syncthreads();
     const int live = s_tiles * TM;
-    for (int i = threadIdx.x; i < live; i += blockDim.x) row_src[i] = -1;
+    if (((uintptr_t)row_src & 15) == 0) {
+        for (int i = threadIdx.x; i < live / 4; i += blockDim.x) reinterpret_cast<int4 *>(row_src)[i] = make_int4(-1, -1, -1, -1);
+    } else {
+        for (int i = threadIdx.x; i < live; i += blockDim.x) row_src[i] = -1;
+    }
     __syncthreads();
-    for (int i = begin; i < end; i += 32) {
-        const int pr = i + lane;
-        int e = pr < end ? ids[pr] : -1;
-        if (e < 0 || e >= E) e = -1;
-        const unsigned same = __match_any_sync(0xffffffffu, e);
-        const int leader = __ffs(same) - 1;
-        int base = 0;
-        if (e >= 0 && lane == leader) base = cnt[warp][e];
-        base = __shfl_sync(0xffffffffu, base, leader);
-        if (e >= 0) row_src[tile_start[e] * TM + base + __popc(same & ((1u << lane) - 1u))] = pr;
-        __syncwarp();
-        if (e >= 0 && lane == leader) cnt[warp][e] = base + __popc(same);
-        __syncwarp();
+    for (int i0 = begin; i0 < end; i0 += AHEAD * 32) {
+        if (!once) fetch(i0);
+#pragma unroll
+        for (int j = 0; j < AHEAD; j++) {
+            if (i0 + j * 32 >= end) break;
+            const int e = ex[j];
+            const unsigned same = once ? mates[j] : __match_any_sync(0xffffffffu, e);
+            const int leader = __ffs(same) - 1;
+            int base = 0;
+            if (e >= 0 && lane == leader) base = cnt[warp][e];
+            base = __shfl_sync(0xffffffffu, base, leader);
+            if (e >= 0) row_src[tile_start[e] * TM + base + __popc(same & ((1u << lane) - 1u))] = i0 + j * 32 + lane;
+            __syncwarp();
+            if (e >= 0 && lane == leader) cnt[warp][e] = base + __popc(same);
+            __syncwarp();
+        }
     }
 }
 

@@ -26,6 +26,7 @@ struct RopeTable {
 // q: [rows][n_head][hd] f32 rotated in place.  k (optional): [rows][n_kv][hd] f32 rotated and
 // stored into the cache at the row's position (f16, or q8_0 / q4_0 rows); v likewise without
 // rotation.  seq_stride counts cache elements (positions x kv heads x hd) per sequence.
+template <bool VEC>
 __global__ void rope_store_kernel(float *q, const float *k, const float *v, const int32_t *pos,
                                   const int32_t *pos0_dev, int pos0, int T, int n_head, int n_kv, int hd, int neox,
                                   RopeTable tab, __half *k_cache, __half *v_cache,
@@ -64,6 +65,54 @@ __global__ void rope_store_kernel(float *q, const float *k, const float *v, cons
             uint8_t *dst = reinterpret_cast<uint8_t *>(v_cache) + (cache_row + kh) * kq_kv_row_bytes(kvt.v, hd);
             kq_kv_store_block(kvt.v, v[((int64_t)row * n_kv + kh) * hd + e], dst, hd, blk, lane);
         }
+    }
+    if (VEC) {
+        // head_dim 128, addresses that allow it: a warp turns four heads at a time, whose loads are in flight together (512 rows of 56 heads: a pair per
+        // thread and turn 14 us, now 8)
+        const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5, n = n_head + (k && !kq ? n_kv : 0);
+        const float2 c0 = cs[2 * lane], c1 = cs[2 * lane + 1]; // of this lane's two pairs
+        for (int h0 = warp; h0 < n; h0 += 4 * nw) {
+            float2 a[4], b[4];
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+                const int hi = h0 + j * nw;
+                if (hi >= n) continue;
+                const float *vv = hi < n_head ? q + ((int64_t)row * n_head + hi) * 128 : k + ((int64_t)row * n_kv + hi - n_head) * 128;
+                if (neox) {
+                    a[j] = *reinterpret_cast<const float2 *>(vv + 2 * lane), b[j] = *reinterpret_cast<const float2 *>(vv + 64 + 2 * lane);
+                } else {
+                    const float4 f = *reinterpret_cast<const float4 *>(vv + 4 * lane);
+                    a[j] = make_float2(f.x, f.z), b[j] = make_float2(f.y, f.w);
+                }
+            }
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+                const int hi = h0 + j * nw;
+                if (hi >= n) continue;
+                const float x0 = a[j].x * c0.x - b[j].x * c0.y, y0 = a[j].x * c0.y + b[j].x * c0.x, x1 = a[j].y * c1.x - b[j].y * c1.y,
+                            y1 = a[j].y * c1.y + b[j].y * c1.x;
+                if (hi < n_head) {
+                    float *vv = q + ((int64_t)row * n_head + hi) * 128;
+                    if (neox) {
+                        *reinterpret_cast<float2 *>(vv + 2 * lane) = make_float2(x0, x1), *reinterpret_cast<float2 *>(vv + 64 + 2 * lane) = make_float2(y0, y1);
+                    } else {
+                        *reinterpret_cast<float4 *>(vv + 4 * lane) = make_float4(x0, y0, x1, y1);
+                    }
+                } else {
+                    __half2 *dst = reinterpret_cast<__half2 *>(k_cache + seq * seq_stride + ((int64_t)p * n_kv + hi - n_head) * 128);
+                    if (neox) dst[lane] = __floats2half2_rn(x0, x1), dst[32 + lane] = __floats2half2_rn(y0, y1);
+                    else dst[2 * lane] = __floats2half2_rn(x0, y0), dst[2 * lane + 1] = __floats2half2_rn(x1, y1);
+                }
+            }
+        }
+        if (v && !vq) {
+            __half2 *dst = reinterpret_cast<__half2 *>(v_cache + seq * seq_stride + (int64_t)p * n_kv * 128);
+            for (int i = threadIdx.x; i < n_kv * 32; i += blockDim.x) {
+                const float4 f = *reinterpret_cast<const float4 *>(v + (int64_t)row * n_kv * 128 + 4 * i);
+                dst[2 * i] = __floats2half2_rn(f.x, f.y), dst[2 * i + 1] = __floats2half2_rn(f.z, f.w);
+            }
+        }
+        return;
     }
     const int n_rot = (n_head + (k && !kq ? n_kv : 0)) * half;
     for (int i = threadIdx.x; i < n_rot; i += blockDim.x) {
@@ -481,8 +530,13 @@ b200_status kq_rope_store(float *q, const float *k, const float *v, const int32_
     KQ_REQUIRE(!kvt.quantised() || hd % 32 == 0, "rope: quantised KV rows need head_dim %% 32 == 0");
     RopeTable tab;
     for (int i = 0; i < hd / 2; i++) tab.inv_freq[i] = (float)pow((double)theta, -2.0 * i / (double)hd);
-    kq_launch(rope_store_kernel, n_seq * T, 256, 0, st, q, k, v, pos, pos0_dev, pos0, T, n_head, n_kv, hd, neox, tab,
-                                                 (__half *)k_cache, (__half *)v_cache, seq_stride, kvt);
+    const bool vec = hd == 128 && ((((uintptr_t)q | (uintptr_t)k | (uintptr_t)v) & 15) | (((uintptr_t)k_cache | (uintptr_t)v_cache) & 3)) == 0 && seq_stride % 2 == 0;
+    if (vec)
+        kq_launch(rope_store_kernel<true>, n_seq * T, 256, 0, st, q, k, v, pos, pos0_dev, pos0, T, n_head, n_kv, hd, neox, tab, (__half *)k_cache,
+                  (__half *)v_cache, seq_stride, kvt);
+    else
+        kq_launch(rope_store_kernel<false>, n_seq * T, 256, 0, st, q, k, v, pos, pos0_dev, pos0, T, n_head, n_kv, hd, neox, tab, (__half *)k_cache,
+                  (__half *)v_cache, seq_stride, kvt);
     KQ_COUNT_LAUNCH();
     KQ_LAUNCH_CHECK();
     return B200_OK;
