@@ -44,6 +44,7 @@
 #include <string.h>
 
 #include <algorithm>
+#include <atomic>
 #include <mutex>
 
 namespace {
@@ -873,7 +874,7 @@ b200_status scratch(int dev, size_t img16_bytes, size_t img8_bytes, size_t da_by
     static std::mutex mu;
     static void *buf[MAX_DEVICES][4];
     static size_t cap[MAX_DEVICES][4];
-    static bool captured[MAX_DEVICES][4], attr[MAX_DEVICES];
+    static bool captured[MAX_DEVICES][4];
     static int4 *parts_done[MAX_DEVICES];
     std::lock_guard<std::mutex> lock(mu);
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
@@ -914,22 +915,7 @@ b200_status scratch(int dev, size_t img16_bytes, size_t img8_bytes, size_t da_by
         }
         if (need[i] && capturing) captured[dev][i] = true;
     }
-    if (!attr[dev]) {
-        auto prepare = [](const void *f, int smem, int regs) {
-            cudaFuncAttributes a;
-            KQ_CUDA(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-            KQ_CUDA(cudaFuncGetAttributes(&a, f));
-            // setmaxnreg moves registers of the launch between the warpgroups: more than it was launched with would wait for ever
-            KQ_REQUIRE(4 * a.numRegs >= regs, "gemm: built with %d registers", a.numRegs);
-            return B200_OK;
-        };
-        KQ_TRY(prepare((const void *)gemm_kq_kernel<false, false>, Cfg<false, false>::SMEM, Cfg<false, false>::REG_SUM));
-        KQ_TRY(prepare((const void *)gemm_kq_kernel<false, true>, Cfg<false, true>::SMEM, Cfg<false, true>::REG_SUM));
-        KQ_TRY(prepare((const void *)gemm_kq_kernel<true, false>, Cfg<true, false>::SMEM, Cfg<true, false>::REG_SUM));
-        KQ_TRY(prepare((const void *)gemm_kq_kernel<true, true>, Cfg<true, true>::SMEM, Cfg<true, true>::REG_SUM));
-        KQ_CUDA(cudaGetSymbolAddress((void **)&parts_done[dev], g_parts_done));
-        attr[dev] = true;
-    }
+    if (!parts_done[dev]) KQ_CUDA(cudaGetSymbolAddress((void **)&parts_done[dev], g_parts_done));
     *out = {img16_bytes ? (uint8_t *)buf[dev][0] : nullptr, img8_bytes ? (uint8_t *)buf[dev][1] : nullptr, (float *)buf[dev][2], (float *)buf[dev][3], parts_done[dev]};
     return B200_OK;
 }
@@ -1012,6 +998,24 @@ TokTiles token_tiles_of(uint32_t type, const KqGemvSeg *segs, int nseg, int64_t 
     return row_tiles ? token_tiles(type == B200_TYPE_Q6_K, M, row_tiles, nb) : TokTiles{0, 0, false, 0};
 }
 
+template <bool Q6, bool NARROW>
+b200_status launch(int grid, cudaStream_t st, const Params &p) {
+    using C = Cfg<Q6, NARROW>;
+    static std::atomic<uint32_t> ready; // devices on which this instance may have its shared memory; an instance that nobody uses is not loaded
+    int dev = 0;
+    KQ_CUDA(cudaGetDevice(&dev));
+    if (!(ready.load() >> dev & 1)) {
+        cudaFuncAttributes a;
+        KQ_CUDA(cudaFuncSetAttribute(gemm_kq_kernel<Q6, NARROW>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM));
+        KQ_CUDA(cudaFuncGetAttributes(&a, gemm_kq_kernel<Q6, NARROW>));
+        // setmaxnreg moves registers of the launch between the warpgroups: more than it was launched with would wait for ever
+        KQ_REQUIRE(4 * a.numRegs >= C::REG_SUM, "gemm: built with %d registers", a.numRegs);
+        ready |= 1u << dev;
+    }
+    KQ_CUDA(kq_launch(gemm_kq_kernel<Q6, NARROW>, dim3(grid), dim3(NTHREADS), C::SMEM, st, p));
+    return B200_OK;
+}
+
 // one launch per weight type for the matrices that read the images in sc; dense products cut the tokens by type
 b200_status launch_segs(Params p, bool narrow, const Scratch &sc, const KqGemvSeg *segs, int nseg, int64_t experts, int64_t K, cudaStream_t st) {
     for (const uint32_t type : {(uint32_t)B200_TYPE_Q4_K, (uint32_t)B200_TYPE_Q6_K}) {
@@ -1029,10 +1033,9 @@ b200_status launch_segs(Params p, bool narrow, const Scratch &sc, const KqGemvSe
         KQ_REQUIRE(units < (int64_t)1 << 31, "gemm: bad shape");
         // with experts the number of tiles is known on the device only
         const int grid = p.row_src ? kq_sm_count() : (int)std::min<int64_t>(kq_sm_count(), std::max<int64_t>(1, units / p.min_share));
-        if (type == B200_TYPE_Q4_K && narrow) KQ_CUDA(kq_launch(gemm_kq_kernel<false, true>, dim3(grid), dim3(NTHREADS), Cfg<false, true>::SMEM, st, p));
-        else if (type == B200_TYPE_Q4_K) KQ_CUDA(kq_launch(gemm_kq_kernel<false, false>, dim3(grid), dim3(NTHREADS), Cfg<false, false>::SMEM, st, p));
-        else if (narrow) KQ_CUDA(kq_launch(gemm_kq_kernel<true, true>, dim3(grid), dim3(NTHREADS), Cfg<true, true>::SMEM, st, p));
-        else KQ_CUDA(kq_launch(gemm_kq_kernel<true, false>, dim3(grid), dim3(NTHREADS), Cfg<true, false>::SMEM, st, p));
+        const bool q6 = type == B200_TYPE_Q6_K;
+        if (narrow) KQ_TRY((q6 ? launch<true, true>(grid, st, p) : launch<false, true>(grid, st, p)));
+        else KQ_TRY((q6 ? launch<true, false>(grid, st, p) : launch<false, false>(grid, st, p)));
         KQ_COUNT_LAUNCH();
         KQ_LAUNCH_CHECK();
     }
