@@ -4,8 +4,9 @@
 // Tensor cores: a persistent CTA per SM walks tiles of 128 tokens (TMEM lanes) x 256, 192, 128 or 64 weight rows (columns), token
 // tiles innermost, so that the CTAs at work share the weight rows they read.  K runs in slices of 64 (one
 // 128-byte-swizzled row per operand row); a producer thread brings the slices in by tiled TMA copies through a ring
-// of stages, one thread issues the MMAs into one of two accumulators in TMEM, four warps drain the other one meanwhile,
-// through a transpose in shared memory: stores of one row per lane would run at a fifth of the rate.
+// of stages, one thread issues the MMAs into one of two accumulators in TMEM, eight warps drain the other one meanwhile,
+// through a transpose in shared memory: stores of one row per lane would run at a fifth of the rate.  (Four warps took longer than the MMAs of a tile of
+// 3072 values: 1000 tokens x 2 x 9216 rows 125 us, 98 with eight; 1000 x 3072 x 3072 32 and 29.)
 // A gate / up pair shares a tile half and half, so that the GLU happens where both values are.
 // An f32 operand can come as several bf16 parts (x = hi + mid + lo exactly): the K loop then passes over the
 // same weights once per part.  Block-diagonal products offset the K coordinate of x and the row of W by group.  Products
@@ -22,14 +23,14 @@
 namespace {
 
 constexpr int TM = 128, BK = 64, A_BYTES = TM * BK * 2;
-constexpr int EC = 32, EP = EC + 4, EPI_BYTES = 4 * 32 * EP * 4; // columns an epilogue warp turns round at a time, floats per staged row
+constexpr int EPI_WARPS = 8, EC = 32, EPI_BYTES = EPI_WARPS * 32 * EC * 4; // EC: columns an epilogue warp turns round at a time
 template <int TN>
 struct Tile {
     static constexpr int B_BYTES = TN * BK * 2, STAGE_BYTES = A_BYTES + B_BYTES, STAGES = 192 * 1024 / STAGE_BYTES;
     static constexpr int SMEM_TOTAL = STAGES * STAGE_BYTES + EPI_BYTES + 1024;
     static constexpr uint32_t TMEM_COLS = TN == 192 ? 512 : 2 * TN; // two accumulators, in a power of two of columns
 };
-constexpr int NTHREADS = 192, NEPI = 128; // producer warp, MMA warp, four epilogue warps
+constexpr int NEPI = EPI_WARPS * 32, NTHREADS = 64 + NEPI; // producer warp, MMA warp, epilogue warps
 constexpr uint64_t LIMIT = 5 * KQ_WAIT_LIMIT_NS;
 
 __device__ int g_gemm_bf16_error;
@@ -229,24 +230,29 @@ __global__ void __launch_bounds__(NTHREADS, 1) gemm_bf16_kernel(const __grid_con
         __syncwarp();
     } else {
         const int q = warp & 3; // a warp reaches the TMEM lanes of its quarter
-        float *stage = reinterpret_cast<float *>(sm + S::STAGES * S::STAGE_BYTES) + q * 32 * EP;
+        // a warp's 32 x EC values; the four-float words of row r are exchanged by r % 8, so that neither way round meets a bank conflict
+        float *stage = reinterpret_cast<float *>(sm + S::STAGES * S::STAGE_BYTES) + (warp - 2) * 32 * EC;
+        auto word = [&](int r, int c4) { return stage + r * EC + (((c4 >> 2) ^ (r & 7)) << 2); };
         int t = 0;
         for (int tile = blockIdx.x; tile < n_tiles; tile += gridDim.x, t++) {
             const int buf = t & 1;
-            const bool ok = wait(&acc_full[buf], (uint32_t)((t / 2) & 1), 3);
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            if (!ok) break;
             const Where w = locate(tile);
             const int n0 = w.n0, n_rows = w.n_rows, m0 = w.m0 + q * 32, m_end = std::min(p.c.M, m0 + 32);
             const uint32_t tl = tmem + ((uint32_t)(q * 32) << 16) + buf * TN;
             const KqDenseSeg s = kq_dense_seg(p.c, w.seg);
             // EC columns at a time: a lane takes its row out of TMEM into shared memory, then eight lanes write a row's columns, four
-            // rows per store.  The loops stay loops: unrolled, the four warps would spend their time fetching code.
+            // rows per store.  The loops stay loops: unrolled, the warps would spend their time fetching code.
             const int lim = p.c.groups == 1 ? std::max(n_rows, s.pad_cols) : n_rows; // the padding of a staging row is written too
             const int n_cols = std::min(p.c.glu ? TN / 2 : TN, lim - n0);
             const int r4 = lane >> 3, c4 = (lane & 7) * 4;
+            const bool plain = !p.c.row_mul && !p.c.head_gate && s.act == KQ_ACT_NONE && m_end == m0 + 32; // sums and biases of 32 whole rows
+            const bool ok = wait(&acc_full[buf], (uint32_t)((t / 2) & 1), 3);
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            if (!ok) break;
 #pragma unroll 1
-            for (int j = 0; j < n_cols; j += EC) {
+            for (int j = (warp - 2) / 4 * EC; j < n_cols; j += EPI_WARPS / 4 * EC) {
+                const int n = n0 + j + c4, n_valid = std::max(0, std::min(4, lim - n));
+                const Col4 col(p.c, s, (p.c.experts ? 0 : (int64_t)w.g * n_rows) + n, n_valid); // its biases come in while TMEM is read
 #pragma unroll
                 for (int h = 0; h < EC; h += 16) {
                     uint32_t a[16], b[16];
@@ -260,12 +266,29 @@ __global__ void __launch_bounds__(NTHREADS, 1) gemm_bf16_kernel(const __grid_con
                     }
 #pragma unroll
                     for (int e = 0; e < 16; e += 4)
-                        *reinterpret_cast<uint4 *>(stage + lane * EP + h + e) = make_uint4(a[e], a[e + 1], a[e + 2], a[e + 3]);
+                        *reinterpret_cast<uint4 *>(word(lane, h + e)) = make_uint4(a[e], a[e + 1], a[e + 2], a[e + 3]);
                 }
                 __syncwarp();
-                const int n = n0 + j + c4, n_valid = std::min(4, lim - n);
-                if (n_valid > 0) {
-                    const Col4 col(p.c, s, (p.c.experts ? 0 : (int64_t)w.g * n_rows) + n, n_valid);
+                if (plain && col.vec) { // no tests between the eight stores
+                    const int64_t first = (int64_t)(m0 + r4) * s.ldy + col.col, step = 4 * s.ldy;
+                    float4 v[8];
+#pragma unroll
+                    for (int i = 0; i < 8; i++) {
+                        v[i] = *reinterpret_cast<const float4 *>(word(r4 + 4 * i, c4));
+                        v[i].x += col.bias[0], v[i].y += col.bias[1], v[i].z += col.bias[2], v[i].w += col.bias[3];
+                    }
+                    if (s.out == KQ_OUT_F32) {
+#pragma unroll
+                        for (int i = 0; i < 8; i++) *reinterpret_cast<float4 *>((float *)s.y + first + i * step) = v[i];
+                    } else {
+#pragma unroll
+                        for (int i = 0; i < 8; i++) {
+                            const uint16_t o[4] = {s.out == KQ_OUT_BF16 ? kq_f2bf(v[i].x) : kq_f2h_sat(v[i].x), s.out == KQ_OUT_BF16 ? kq_f2bf(v[i].y) : kq_f2h_sat(v[i].y),
+                                                   s.out == KQ_OUT_BF16 ? kq_f2bf(v[i].z) : kq_f2h_sat(v[i].z), s.out == KQ_OUT_BF16 ? kq_f2bf(v[i].w) : kq_f2h_sat(v[i].w)};
+                            *reinterpret_cast<uint2 *>((uint16_t *)s.y + first + i * step) = make_uint2((uint32_t)o[0] | ((uint32_t)o[1] << 16), (uint32_t)o[2] | ((uint32_t)o[3] << 16));
+                        }
+                    }
+                } else if (n_valid > 0) {
                     if (p.c.row_mul) { // the factors of all of a lane's rows are requested together
                         uint2 f[8];
 #pragma unroll
@@ -273,11 +296,11 @@ __global__ void __launch_bounds__(NTHREADS, 1) gemm_bf16_kernel(const __grid_con
 #pragma unroll
                         for (int i = 0; i < 8; i++)
                             if (m0 + r4 + 4 * i < m_end)
-                                col.store(p.c, s, m0 + r4 + 4 * i, w.g, *reinterpret_cast<const float4 *>(stage + (r4 + 4 * i) * EP + c4), f[i]);
+                                col.store(p.c, s, m0 + r4 + 4 * i, w.g, *reinterpret_cast<const float4 *>(word(r4 + 4 * i, c4)), f[i]);
                     } else {
 #pragma unroll 2
                         for (int r = r4; m0 + r < m_end; r += 4) {
-                            const float4 v = *reinterpret_cast<const float4 *>(stage + r * EP + c4);
+                            const float4 v = *reinterpret_cast<const float4 *>(word(r, c4));
                             col.store(p.c, s, m0 + r, w.g, v);
                         }
                     }
