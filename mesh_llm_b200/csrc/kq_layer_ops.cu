@@ -261,6 +261,7 @@ __device__ __forceinline__ void rec_coeff(float r, float i, float u, float decay
 // Prefill in two passes over chunks of `chunk` positions, a thread per channel.  First: coefficients (over the gates, in
 // place) and each chunk's map of the state, s -> A s + B.  Second: the state in front of a chunk from the maps of the
 // chunks before it, then the recurrence inside the chunk.
+constexpr int AHEAD = 8;
 constexpr int RC = 128, RCHUNK = 16, RCHUNKS = 64; // channels per CTA, positions per chunk at least, chunks at most
 // Positions per chunk.  A thread's walk through its chunk is a chain of dependent steps, and many short chunks hide it; the second pass reads the
 // maps of all chunks in front of its own, so there are not more than 64 of them (a call of 1000 x 3072: 16 chunks of 64 positions
@@ -279,15 +280,25 @@ __global__ void __launch_bounds__(RC) recurrence_chunks_kernel(const __grid_cons
     const int64_t row0 = (int64_t)seq * T;
     const float dsp = w.decay * kq_softplus(w.lam[c]);
     float A = 1.f, B = 0.f;
-#pragma unroll 4
-    for (int t = t0; t < t1; t++) {
-        const int64_t o = (row0 + t) * ldr + c;
-        float a, b;
-        rec_coeff(r[o], ig[o], u[(row0 + t) * ldu + c], dsp, a, b);
-        r[o] = a;
-        ig[o] = b;
-        A *= a;
-        B = fmaf(a, B, b);
+    // AHEAD positions' loads together: behind a store each would be a trip to memory of its own (1000 x 3072: 19 -> 17 us, which its exponentials and roots take; the second pass 19 -> 14)
+    for (int tb = t0; tb < t1; tb += AHEAD) {
+        float rv[AHEAD], iv[AHEAD], uv[AHEAD];
+#pragma unroll
+        for (int j = 0; j < AHEAD; j++) {
+            const int t = min(tb + j, t1 - 1);
+            rv[j] = r[(row0 + t) * ldr + c], iv[j] = ig[(row0 + t) * ldr + c], uv[j] = u[(row0 + t) * ldu + c];
+        }
+#pragma unroll
+        for (int j = 0; j < AHEAD; j++) {
+            if (tb + j >= t1) break;
+            const int64_t o = (row0 + tb + j) * ldr + c;
+            float a, b;
+            rec_coeff(rv[j], iv[j], uv[j], dsp, a, b);
+            r[o] = a;
+            ig[o] = b;
+            A *= a;
+            B = fmaf(a, B, b);
+        }
     }
     float *d = maps + ((int64_t)seq * (gridDim.y + 1) + k + 1) * 2 * w.width + c;
     d[0] = A;
@@ -320,13 +331,21 @@ __global__ void __launch_bounds__(RC) recurrence_scan_kernel(const __grid_consta
     float s = d[0];
 #pragma unroll 8
     for (int j = 1; j <= k; j++) s = fmaf(d[(int64_t)j * 2 * w.width], s, d[((int64_t)j * 2 + 1) * w.width]);
-#pragma unroll 8
-    for (int t = t0; t < t1; t++) {
-        const int64_t o = (row0 + t) * ldr + c;
-        s = fmaf(a[o], s, b[o]);
-        const float v = s * y[(row0 + t) * ldy + c];
-        if (z32) z32[(row0 + t) * ld32 + c] = v;
-        if (z16) z16[(row0 + t) * ld16 + c] = kq_f2bf(v);
+    for (int tb = t0; tb < t1; tb += AHEAD) {
+        float av[AHEAD], bv[AHEAD], yv[AHEAD];
+#pragma unroll
+        for (int j = 0; j < AHEAD; j++) {
+            const int64_t t = row0 + min(tb + j, t1 - 1);
+            av[j] = a[t * ldr + c], bv[j] = b[t * ldr + c], yv[j] = y[t * ldy + c];
+        }
+#pragma unroll
+        for (int j = 0; j < AHEAD; j++) {
+            if (tb + j >= t1) break;
+            s = fmaf(av[j], s, bv[j]);
+            const float v = s * yv[j];
+            if (z32) z32[(row0 + tb + j) * ld32 + c] = v;
+            if (z16) z16[(row0 + tb + j) * ld16 + c] = kq_f2bf(v);
+        }
     }
     if (last) st.s[(int64_t)seq * w.width + c] = s;
 }
