@@ -344,6 +344,7 @@ b200_status kq_launch_gemv_stream(const KqGemvSeg *segs, int nseg, const int8_t 
 bool kq_gemv_batch_parts(uint32_t type, int64_t K); // 5 to 8 tokens of K values take launches over ranges of K
 b200_status kq_rms_norm(const float *x, const float *w, int64_t T, int64_t h, float eps, float *y, int8_t *q,
                         float *d, int16_t *bs, cudaStream_t st, int64_t x_row_stride);
+b200_status kq_rms_norm_heads(float *q, const float *wq, int64_t q_rows, float *k, const float *wk, int64_t k_rows, int64_t h, float eps, cudaStream_t st);
 // Where the tokens of a product may be written by the kernel that makes them, as the product reads them; *im without an image when they go out in the usual form instead
 bool kq_gemm_takes_images();
 b200_status kq_gemm_image(const KqGemvSeg *segs, int nseg, int64_t M, int64_t K, cudaStream_t st, KqTokenImage *im);

@@ -28,7 +28,6 @@ __global__ void __launch_bounds__(256) moe_router_fused_kernel(const float *x, c
     KQ_PDL_TRIGGER();
     extern __shared__ __align__(16) float xn[]; // the normalised row
     __shared__ double part[8];
-    __shared__ float s_scale;
     __shared__ int s_last;
     const int row = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     // The router's weights do not depend on the kernel before: the first 2048 of this warp's first expert
@@ -42,38 +41,63 @@ __global__ void __launch_bounds__(256) moe_router_fused_kernel(const float *x, c
         for (int j = 0; j < PRE; j++)
             if (lane + 32 * j < n4) wpre[j] = __ldg(wr + lane + 32 * j);
     }
-    KQ_PDL_WAIT();
+    // a warp holds up to two blocks of the row, read once, and their norm weights, which do not depend on the kernel before either
+    constexpr int R = 2;
     const float *xr = x + (int64_t)row * h;
+    const int nb = h / 256;
+    float g[R][8], v[R][8];
+    auto load = [&](const float *p, int b, float (&o)[8]) {
+        const float4 f0 = *reinterpret_cast<const float4 *>(p + b * 256 + lane * 8), f1 = *reinterpret_cast<const float4 *>(p + b * 256 + lane * 8 + 4);
+        o[0] = f0.x, o[1] = f0.y, o[2] = f0.z, o[3] = f0.w, o[4] = f1.x, o[5] = f1.y, o[6] = f1.z, o[7] = f1.w;
+    };
+#pragma unroll
+    for (int r = 0; r < R; r++)
+        if (warp + 8 * r < nb) load(norm_w, warp + 8 * r, g[r]);
+    KQ_PDL_WAIT();
     double ss = 0.0; // in double, so that the scale does not depend on the order of the reduction
-    for (int i = tid * 4; i < h; i += 1024) {
-        const float4 v = *reinterpret_cast<const float4 *>(xr + i);
-        ss += (double)v.x * v.x + (double)v.y * v.y + (double)v.z * v.z + (double)v.w * v.w;
+    auto add = [&](const float (&u)[8]) {
+#pragma unroll
+        for (int i = 0; i < 8; i++) ss += (double)u[i] * u[i];
+    };
+#pragma unroll
+    for (int r = 0; r < R; r++)
+        if (warp + 8 * r < nb) load(xr, warp + 8 * r, v[r]);
+#pragma unroll
+    for (int r = 0; r < R; r++)
+        if (warp + 8 * r < nb) add(v[r]);
+    for (int b = warp + 8 * R; b < nb; b += 8) {
+        float u[8];
+        load(xr, b, u);
+        add(u);
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
     if (lane == 0) part[warp] = ss;
     __syncthreads();
-    if (tid == 0) {
-        double t = 0.0;
-        for (int i = 0; i < 8; i++) t += part[i];
-        s_scale = 1.0f / sqrtf((float)(t / (double)h) + eps);
-    }
-    __syncthreads();
-    const float scale = s_scale;
-    const int nb = h / 256;
-    for (int b = warp; b < nb; b += 8) {
-        const int o = b * 256 + lane * 8;
-        const float4 a = *reinterpret_cast<const float4 *>(xr + o);
-        const float4 c = *reinterpret_cast<const float4 *>(xr + o + 4);
-        float v[8] = {a.x, a.y, a.z, a.w, c.x, c.y, c.z, c.w};
+    double t = 0.0;
 #pragma unroll
-        for (int i = 0; i < 8; i++) v[i] = v[i] * scale * norm_w[o + i];
-        *reinterpret_cast<float4 *>(xn + o) = make_float4(v[0], v[1], v[2], v[3]);
-        *reinterpret_cast<float4 *>(xn + o + 4) = make_float4(v[4], v[5], v[6], v[7]);
+    for (int i = 0; i < 8; i++) t += part[i];
+    const float scale = 1.0f / sqrtf((float)(t / (double)h) + eps);
+    auto emit = [&](int b, const float (&u)[8], const float (&f)[8]) {
+        const int o = b * 256 + lane * 8;
+        float n[8];
+#pragma unroll
+        for (int i = 0; i < 8; i++) n[i] = u[i] * scale * f[i];
+        *reinterpret_cast<float4 *>(xn + o) = make_float4(n[0], n[1], n[2], n[3]);
+        *reinterpret_cast<float4 *>(xn + o + 4) = make_float4(n[4], n[5], n[6], n[7]);
         if (blockIdx.x == 0) { // one CTA of the token leaves the Q8 form for the expert matmuls
             const int64_t gb = (int64_t)row * nb + b;
-            kq_quantize_block_warp(v, lane, q + gb * 256, d + gb, bs + gb * 16);
+            kq_quantize_block_warp(n, lane, q + gb * 256, d + gb, bs + gb * 16);
         }
+    };
+#pragma unroll
+    for (int r = 0; r < R; r++)
+        if (warp + 8 * r < nb) emit(warp + 8 * r, v[r], g[r]);
+    for (int b = warp + 8 * R; b < nb; b += 8) {
+        float u[8], f[8];
+        load(xr, b, u);
+        load(norm_w, b, f);
+        emit(b, u, f);
     }
     __syncthreads();
     for (int e = e_first; e < E; e += gridDim.x * 8) { // one warp per expert

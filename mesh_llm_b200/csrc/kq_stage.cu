@@ -323,10 +323,7 @@ b200_status forward_body(b200_stage *st, const int32_t *tokens, const float *hid
             GEMV_(kq_launch_gemm(segs, 3, st->aq, st->ad, st->abs16, rows, h, nullptr, s));
         }
         if (c.qk_norm) {
-            OTHER_(kq_rms_norm(st->q, L.q_norm, (int64_t)rows * c.n_head, hd, c.rms_eps, st->q, nullptr,
-                               nullptr, nullptr, s));
-            OTHER_(kq_rms_norm(st->k, L.k_norm, (int64_t)rows * c.n_head_kv, hd, c.rms_eps, st->k, nullptr,
-                               nullptr, nullptr, s));
+            OTHER_(kq_rms_norm_heads(st->q, L.q_norm, (int64_t)rows * c.n_head, st->k, L.k_norm, (int64_t)rows * c.n_head_kv, hd, c.rms_eps, s));
         }
         if (T == 1) {
             // decode: RoPE, KV store, attention and the split combine are one launch
