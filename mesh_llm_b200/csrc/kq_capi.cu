@@ -224,7 +224,7 @@ b200_status b200_mul_mat_id(uint32_t type, const void *W, int64_t E, const float
     if (n_pairs > 8) { // many pairs: gathered per expert, one grouped launch of the tensor-core kernel
         rc = kq_moe_sort(ids, n_pairs, E, sorted, kq_moe_sort_scratch_bytes(n_pairs, E), st);
         if (rc != B200_OK) return rc;
-        return kq_launch_gemm_grouped(&sg, 1, q, d, bs, act_div, n_pairs, E, K, sorted, st);
+        return kq_launch_gemm_grouped(&sg, 1, {q, d, bs, nullptr, nullptr}, act_div, n_pairs, E, K, sorted, st);
     }
     KqGemvIndirect ind = {ids, (int32_t)n_pairs, (int32_t)act_div};
     return kq_launch_gemv(&sg, 1, q, d, bs, 1, K, nullptr, 0, &ind, st);

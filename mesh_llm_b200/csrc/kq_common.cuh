@@ -350,13 +350,26 @@ bool kq_gemm_takes_images();
 b200_status kq_gemm_image(const KqGemvSeg *segs, int nseg, int64_t M, int64_t K, cudaStream_t st, KqTokenImage *im);
 b200_status kq_launch_gemm_image(const KqGemvSeg *segs, int nseg, const KqTokenImage &im, int64_t K, const float *residual, cudaStream_t st);
 b200_status kq_rms_norm_image(const float *x, const float *w, int64_t h, float eps, const KqTokenImage &im, cudaStream_t st);
+// tokens of a product with experts: tile t of tile_tok tokens (of those that n_tiles counts, the one first_tile further) holds the rows row_src[tile_tok t ..], tile_count[t] of them, and
+// zeros up to a whole number of chunks
+struct KqTileRows {
+    const int32_t *row_src, *tile_count, *n_tiles;
+    int32_t first_tile, tile_tok, narrow;
+};
+b200_status kq_act_image_tiles(const float *x, const float *up, int64_t K, const KqTokenImage &im, const KqTileRows &rows, cudaStream_t st);
 // x, or silu(x) * up, of [im.n_tok][K]; y (may be x): the latter in f32
 b200_status kq_act_image(const float *x, const float *up, float *y, int64_t K, const KqTokenImage &im, cudaStream_t st);
 // MUL_MAT_ID over many tokens: stable expert-major order of the (token, slot) pairs, then one grouped
 // launch of the tensor-core GEMM per expert-packed matrix (y[pair][N] = W[expert(pair)] . x[pair / act_div])
 size_t kq_moe_sort_scratch_bytes(int64_t n_pairs, int64_t E);
 b200_status kq_moe_sort(const int32_t *ids, int64_t n_pairs, int64_t E, int32_t *scratch, size_t scratch_bytes, cudaStream_t st);
-b200_status kq_launch_gemm_grouped(const KqGemvSeg *segs, int nseg, const int8_t *q, const float *d, const int16_t *bs, int act_div,
+struct KqGroupedRows { // source rows: quantised, or those of silu(g) * u (act_div 1), which are quantised on the way into the product's operand
+    const int8_t *q;
+    const float *d;
+    const int16_t *bs;
+    const float *g, *u;
+};
+b200_status kq_launch_gemm_grouped(const KqGemvSeg *segs, int nseg, const KqGroupedRows &rows, int act_div,
                                    int64_t n_pairs, int64_t E, int64_t K, const int32_t *sorted, cudaStream_t st);
 int kq_stream_error_fetch(); // 0 ok; nonzero = a bounded device-side wait gave up since the last call
 int kq_gemm_error_fetch();

@@ -1167,11 +1167,11 @@ b200_status kq_moe_sort(const int32_t *ids, int64_t n_pairs, int64_t E, int32_t 
 
 // y[pair][N] = W[expert of the pair] . x[pair / act_div] for up to three expert-packed matrices: q / d / bs are the quantised
 // activations of the n_pairs / act_div source rows, sorted = the scratch kq_moe_sort left for these pairs.
-b200_status kq_launch_gemm_grouped(const KqGemvSeg *segs, int nseg, const int8_t *q, const float *d, const int16_t *bs, int act_div,
+b200_status kq_launch_gemm_grouped(const KqGemvSeg *segs, int nseg, const KqGroupedRows &rows, int act_div,
                                    int64_t n_pairs, int64_t E, int64_t K, const int32_t *sorted, cudaStream_t st) {
     int dev = 0;
-    KQ_TRY(check_segs(segs, nseg, q, K, &dev));
-    KQ_REQUIRE(n_pairs > 0 && act_div >= 1, "grouped gemm: bad shape");
+    KQ_TRY(check_segs(segs, nseg, rows.q, K, &dev));
+    KQ_REQUIRE(n_pairs > 0 && act_div >= 1 && (!rows.g || act_div == 1), "grouped gemm: bad shape");
     for (int i = 0; i < nseg; i++)
         KQ_REQUIRE(segs[i].expert_stride == kq_device_row_bytes(segs[i].type, K) * segs[i].n_rows && segs[i].expert_stride % 16 == 0,
                    "grouped gemm: expert matrices must be contiguous and 16-byte aligned");
@@ -1193,9 +1193,14 @@ b200_status kq_launch_gemm_grouped(const KqGemvSeg *segs, int nseg, const int8_t
         }
         KQ_TRY(rc);
         p.n_tiles = sorted, p.tile_expert = sorted + 1 + t0, p.row_src = sorted + 1 + mt + t0 * TM, p.tile_count = sorted + 1 + mt + mt * TM + t0;
-        const ImageParams ip = {q, d, bs, sc.img16, sc.img8, sc.da, 0, (int32_t)nb, p.m_pad, act_div, p.row_src, p.tile_count, p.n_tiles, p.first_tile, TM, narrow};
-        KQ_CUDA(kq_launch(act_image_kernel, dim3((unsigned)(p.m_pad / 16), (unsigned)nb), dim3(288), 0, st, ip));
-        KQ_COUNT_LAUNCH();
+        if (rows.g) {
+            const KqTokenImage im = {sc.img16, sc.img8, sc.da, sc.parts_done, 2 * MAX_CTAS * DRAIN_WARPS / 4, p.m_pad, 0};
+            KQ_TRY(kq_act_image_tiles(rows.g, rows.u, K, im, {p.row_src, p.tile_count, p.n_tiles, p.first_tile, TM, narrow}, st));
+        } else {
+            const ImageParams ip = {rows.q, rows.d, rows.bs, sc.img16, sc.img8, sc.da, 0, (int32_t)nb, p.m_pad, act_div, p.row_src, p.tile_count, p.n_tiles, p.first_tile, TM, narrow};
+            KQ_CUDA(kq_launch(act_image_kernel, dim3((unsigned)(p.m_pad / 16), (unsigned)nb), dim3(288), 0, st, ip));
+            KQ_COUNT_LAUNCH();
+        }
         KQ_TRY(launch_segs(p, narrow, sc, segs, nseg, E, K, st));
     }
     return B200_OK;

@@ -43,17 +43,29 @@ __global__ void __launch_bounds__(128) swiglu_quantize_kernel(const float *g, co
 
 // The same for the tensor-core product: eight tokens of a block per CTA, a warp each, gathered in shared memory so that the image is written in full lines.
 // With UP silu(x) * up.  A pass over the codes and a launch less than codes first, image then.
-template <bool UP>
-__global__ void __launch_bounds__(256) act_to_image_kernel(const float *x, const float *up, float *y, int64_t K, const __grid_constant__ KqTokenImage im) {
+// TILES: the rows of a product with experts, gathered; chunks of a tile are one (narrow) or two.
+template <bool UP, bool TILES>
+__global__ void __launch_bounds__(256) act_to_image_kernel(const float *x, const float *up, float *y, int64_t K, const __grid_constant__ KqTokenImage im,
+                                                           const __grid_constant__ KqTileRows rows) {
     KQ_PDL_ENTER();
     constexpr int PITCH = 144; // chunks of 128 bytes, 16 further apart: a warp's stores fall on different banks
     __shared__ __align__(16) uint8_t s16[34 * PITCH], s8[16 * PITCH];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, b = blockIdx.y, t0 = blockIdx.x * 8, t = t0 + warp;
     if (blockIdx.x == 0 && b == 0)
         for (int i = tid; i < im.n_parts; i += 256) im.parts[i] = make_int4(0, 0, 0, 0);
+    int live = im.n_tok;
+    int64_t row = t;
+    if (TILES) {
+        const int tile = t0 / rows.tile_tok, first = tile * rows.tile_tok;
+        row = rows.row_src[t]; // asked for before it is known whether there is one: the table has all of them
+        if (tile >= *rows.n_tiles - rows.first_tile) return;
+        const int n = rows.tile_count[tile], padded = rows.narrow ? (n + 15) & ~15 : 2 * (((n + 1) / 2 + 15) & ~15);
+        if (t0 - first >= padded) return;
+        live = first + n;
+    }
     float v[8] = {};
-    if (t < im.n_tok) {
-        const int64_t at = t * K + b * 256 + lane * 8;
+    if (t < live) {
+        const int64_t at = row * K + b * 256 + lane * 8;
         const float4 x0 = *reinterpret_cast<const float4 *>(x + at), x1 = *reinterpret_cast<const float4 *>(x + at + 4);
         v[0] = x0.x, v[1] = x0.y, v[2] = x0.z, v[3] = x0.w, v[4] = x1.x, v[5] = x1.y, v[6] = x1.z, v[7] = x1.w;
         if (UP) {
@@ -424,8 +436,8 @@ b200_status kq_rms_norm_image(const float *x, const float *w, int64_t h, float e
 b200_status kq_act_image(const float *x, const float *up, float *y, int64_t K, const KqTokenImage &im, cudaStream_t st) {
     KQ_REQUIRE(K > 0 && K % 256 == 0 && im.m_pad % 8 == 0 && ((uintptr_t)x & 15) == 0 && (((uintptr_t)up | (uintptr_t)y) & 15) == 0, "act_image: bad shape");
     const dim3 grid((unsigned)(im.m_pad / 8), (unsigned)(K / 256));
-    if (up) kq_launch(act_to_image_kernel<true>, grid, dim3(256), 0, st, x, up, y, K, im);
-    else kq_launch(act_to_image_kernel<false>, grid, dim3(256), 0, st, x, up, y, K, im);
+    if (up) kq_launch(act_to_image_kernel<true, false>, grid, dim3(256), 0, st, x, up, y, K, im, KqTileRows{});
+    else kq_launch(act_to_image_kernel<false, false>, grid, dim3(256), 0, st, x, up, y, K, im, KqTileRows{});
     KQ_COUNT_LAUNCH();
     KQ_LAUNCH_CHECK();
     return B200_OK;
@@ -445,6 +457,14 @@ b200_status kq_rms_norm(const float *x, const float *w, int64_t T, int64_t h, fl
     }
     if (q) return norm_q8(x, w, T, h, eps, y, q, d, bs, ldx, KqTokenImage{}, st);
     kq_launch(rms_norm_kernel, (unsigned)T, 256, 0, st, x, w, (int)h, eps, y, ldx);
+    KQ_COUNT_LAUNCH();
+    KQ_LAUNCH_CHECK();
+    return B200_OK;
+}
+
+b200_status kq_act_image_tiles(const float *x, const float *up, int64_t K, const KqTokenImage &im, const KqTileRows &rows, cudaStream_t st) {
+    KQ_REQUIRE(up && K > 0 && K % 256 == 0 && im.m_pad % 8 == 0 && rows.tile_tok % 8 == 0 && (((uintptr_t)x | (uintptr_t)up) & 15) == 0, "act_image: bad shape");
+    kq_launch(act_to_image_kernel<true, true>, dim3((unsigned)(im.m_pad / 8), (unsigned)(K / 256)), dim3(256), 0, st, x, up, (float *)nullptr, K, im, rows);
     KQ_COUNT_LAUNCH();
     KQ_LAUNCH_CHECK();
     return B200_OK;

@@ -69,6 +69,9 @@ __global__ void __launch_bounds__(128) router_logits_kernel(const float *W, cons
 // more than one of them per SM: 128 tiles take 12 / 21 / 33 us where a warp per pair takes 10 / 16 / 25 (64 experts at 128 tokens, 8 at 1024), 256 tiles
 // take as long as 128 and the warps per pair 14 / 23 / 37.
 constexpr int ROUTER_TILE = 8, ROUTER_MIN_TILES = 256;
+// Norm, logits and choice in the decode step's one launch up to as many rows (its CTAs, 16 a row, norm the row for themselves): a prompt through four layers of 128
+// experts 653 -> 628 us with 9 rows, 749 -> 731 with 16, 857 -> 850 with 24; 893 and 894 with 32, 1047 and 1072 with 64.
+constexpr int ROUTER_FUSED_ROWS = 24;
 __global__ void __launch_bounds__(128) router_logits_tile_kernel(const float *W, const float *x, int T, int E, int h, float *out) {
     KQ_PDL_ENTER();
     const int lane = threadIdx.x & 31, e_tiles = (E + ROUTER_TILE - 1) / ROUTER_TILE;
@@ -405,14 +408,15 @@ b200_status forward_body(b200_stage *st, const int32_t *tokens, const float *hid
                 moe_fused_on = !(v && v[0] == '0');
             }
             bool fused_small = moe_fused_on && rows <= 8 && classes == CLS_ALL && ku <= 8 && fe % 256 == 0 && h % 256 == 0;
-            if (fused_small) {
+            bool routed = moe_fused_on && classes == CLS_ALL && h % 256 == 0 && rows <= (rows <= 8 ? (fused_small ? 8 : 0) : ROUTER_FUSED_ROWS);
+            if (routed) {
                 const b200_status rs = kq_moe_router_fused(st->x, L.ffn_norm, c.rms_eps, L.router, (int)rows, (int)E, (int)h, (int)ku,
                                                            st->expert_mask, st->rl, st->rid, st->rw, st->aq, st->ad, st->abs16,
                                                            st->moe_counters, s);
-                if (rs == B200_ERR_UNSUPPORTED) fused_small = false;
+                if (rs == B200_ERR_UNSUPPORTED) routed = fused_small = false;
                 else KQ_TRY(rs);
             }
-            if (!fused_small) {
+            if (!routed) {
             OTHER_(kq_rms_norm(st->x, L.ffn_norm, rows, h, c.rms_eps, st->xn, st->aq, st->ad, st->abs16, s));
             if (classes & CLS_OTHER) {
             static bool rb_attr[16]; // the block kernel may have its shared memory, per device
@@ -452,10 +456,9 @@ b200_status forward_body(b200_stage *st, const int32_t *tokens, const float *hid
             if (grouped) {
                 KQ_TRY(kq_moe_sort(st->rid, pairs, E, st->moe_sorted, st->moe_sorted_bytes, s));
                 const KqGemvSeg both[2] = {gu[0], {gu[1].W, gu[1].type, fe, st->hp2, nullptr, fe, kq_device_row_bytes(gu[1].type, h) * fe}};
-                KQ_TRY(kq_launch_gemm_grouped(both, 2, st->aq, st->ad, st->abs16, ku, pairs, E, h, st->moe_sorted, s));
-                KQ_TRY(kq_swiglu_quantize(st->hp, st->hp2, pairs, fe, nullptr, st->aq, st->ad, st->abs16, s));
+                KQ_TRY(kq_launch_gemm_grouped(both, 2, {st->aq, st->ad, st->abs16, nullptr, nullptr}, ku, pairs, E, h, st->moe_sorted, s));
                 const KqGemvSeg down = {(const uint8_t *)L.down_e->dev, L.down_e->type, h, st->yp, nullptr, h, dstride};
-                KQ_TRY(kq_launch_gemm_grouped(&down, 1, st->aq, st->ad, st->abs16, 1, pairs, E, fe, st->moe_sorted, s));
+                KQ_TRY(kq_launch_gemm_grouped(&down, 1, {nullptr, nullptr, nullptr, st->hp, st->hp2}, 1, pairs, E, fe, st->moe_sorted, s));
             } else {
             KqGemvIndirect ind = {st->rid, pairs, ku};
             b200_status rg = B200_ERR_UNSUPPORTED;
