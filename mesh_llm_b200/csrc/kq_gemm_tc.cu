@@ -869,6 +869,7 @@ struct Scratch {
     uint8_t *img16, *img8;
     float *da, *part;
     int4 *parts_done;
+    int dev;
 };
 b200_status scratch(int dev, size_t img16_bytes, size_t img8_bytes, size_t da_bytes, cudaStream_t st, Scratch *out) {
     static std::mutex mu;
@@ -916,7 +917,7 @@ b200_status scratch(int dev, size_t img16_bytes, size_t img8_bytes, size_t da_by
         if (need[i] && capturing) captured[dev][i] = true;
     }
     if (!parts_done[dev]) KQ_CUDA(cudaGetSymbolAddress((void **)&parts_done[dev], g_parts_done));
-    *out = {img16_bytes ? (uint8_t *)buf[dev][0] : nullptr, img8_bytes ? (uint8_t *)buf[dev][1] : nullptr, (float *)buf[dev][2], (float *)buf[dev][3], parts_done[dev]};
+    *out = {img16_bytes ? (uint8_t *)buf[dev][0] : nullptr, img8_bytes ? (uint8_t *)buf[dev][1] : nullptr, (float *)buf[dev][2], (float *)buf[dev][3], parts_done[dev], dev};
     return B200_OK;
 }
 
@@ -972,6 +973,7 @@ struct TokTiles {
     int min_share;
 };
 TokTiles token_tiles(bool q6, int64_t M, int64_t row_tiles, int64_t nb) {
+    const int sms = kq_sm_count();
     TokTiles best = {0, 0, false, 0};
     int64_t best_cost = INT64_MAX;
     for (int chunks = MAX_CHUNKS; chunks >= 1; chunks /= 2) {
@@ -981,8 +983,11 @@ TokTiles token_tiles(bool q6, int64_t M, int64_t row_tiles, int64_t nb) {
         const int64_t tok = c * cw, tiles = kq_div_up(M, tok), pairs = tiles * row_tiles * nb;
         const int64_t per_pair = narrow ? (q6 ? 130 + tok / 4 : 80 + tok / 4) : c == 2 ? (q6 ? 175 : 110) + tok * 3 / 10 : (q6 ? 240 + tok / 7 : 178 + tok * 2 / 7);
         const int64_t groups = narrow ? cw / 16 : c * kq_div_up(std::min(cw, CHUNK / 2), 16); // of 16 tokens that a draining warp has
+        int64_t before = 0;
         for (const int min_share : {2, 3, 4, 6, 8}) {
-            const int64_t ctas = std::max<int64_t>(1, std::min<int64_t>(kq_sm_count(), pairs / min_share)), share = kq_div_up(pairs, ctas);
+            const int64_t ctas = std::max<int64_t>(1, std::min<int64_t>(sms, pairs / min_share)), share = kq_div_up(pairs, ctas);
+            if (ctas == before) continue; // enough pairs for all SMs: nothing to choose
+            before = ctas;
             const int64_t parts = pairs % ctas == 0 && nb % share == 0 ? nb / share : kq_div_up(nb - 1, share) + 1;
             const int64_t cost = share * per_pair + (pairs % ctas == 0 && share % nb == 0 ? 0 : 150 + 50 * groups * kq_div_up(parts, 8) + parts * tok * (narrow ? 50 : 40) / CHUNK);
             if (cost < best_cost) best_cost = cost, best = {(int)tiles, (int)tok, narrow, min_share};
@@ -998,12 +1003,17 @@ TokTiles token_tiles_of(uint32_t type, const KqGemvSeg *segs, int nseg, int64_t 
     return row_tiles ? token_tiles(type == B200_TYPE_Q6_K, M, row_tiles, nb) : TokTiles{0, 0, false, 0};
 }
 
+struct CallTiles {
+    TokTiles q4, q6;
+};
+CallTiles call_tiles(const KqGemvSeg *segs, int nseg, int64_t M, int64_t nb) {
+    return {token_tiles_of(B200_TYPE_Q4_K, segs, nseg, M, nb), token_tiles_of(B200_TYPE_Q6_K, segs, nseg, M, nb)};
+}
+
 template <bool Q6, bool NARROW>
-b200_status launch(int grid, cudaStream_t st, const Params &p) {
+b200_status launch(int dev, int grid, cudaStream_t st, const Params &p) {
     using C = Cfg<Q6, NARROW>;
     static std::atomic<uint32_t> ready; // devices on which this instance may have its shared memory; an instance that nobody uses is not loaded
-    int dev = 0;
-    KQ_CUDA(cudaGetDevice(&dev));
     if (!(ready.load() >> dev & 1)) {
         cudaFuncAttributes a;
         KQ_CUDA(cudaFuncSetAttribute(gemm_kq_kernel<Q6, NARROW>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM));
@@ -1017,12 +1027,12 @@ b200_status launch(int grid, cudaStream_t st, const Params &p) {
 }
 
 // one launch per weight type for the matrices that read the images in sc; dense products cut the tokens by type
-b200_status launch_segs(Params p, bool narrow, const Scratch &sc, const KqGemvSeg *segs, int nseg, int64_t experts, int64_t K, cudaStream_t st) {
+b200_status launch_segs(Params p, bool narrow, const CallTiles *tiles, const Scratch &sc, const KqGemvSeg *segs, int nseg, int64_t experts, int64_t K, cudaStream_t st) {
     for (const uint32_t type : {(uint32_t)B200_TYPE_Q4_K, (uint32_t)B200_TYPE_Q6_K}) {
         int n = 0;
         p.row_tiles = 0;
         if (!p.row_src) {
-            const TokTiles t = token_tiles_of(type, segs, nseg, p.M, p.nb);
+            const TokTiles &t = type == B200_TYPE_Q4_K ? tiles->q4 : tiles->q6;
             p.tok_tiles = t.n, p.tile_tok = t.tok, p.min_share = t.min_share, narrow = t.narrow;
         }
         p.img = type == B200_TYPE_Q4_K ? sc.img16 : sc.img8, p.da = sc.da, p.part = sc.part;
@@ -1034,8 +1044,8 @@ b200_status launch_segs(Params p, bool narrow, const Scratch &sc, const KqGemvSe
         // with experts the number of tiles is known on the device only
         const int grid = p.row_src ? kq_sm_count() : (int)std::min<int64_t>(kq_sm_count(), std::max<int64_t>(1, units / p.min_share));
         const bool q6 = type == B200_TYPE_Q6_K;
-        if (narrow) KQ_TRY((q6 ? launch<true, true>(grid, st, p) : launch<false, true>(grid, st, p)));
-        else KQ_TRY((q6 ? launch<true, false>(grid, st, p) : launch<false, false>(grid, st, p)));
+        if (narrow) KQ_TRY((q6 ? launch<true, true>(sc.dev, grid, st, p) : launch<false, true>(sc.dev, grid, st, p)));
+        else KQ_TRY((q6 ? launch<true, false>(sc.dev, grid, st, p) : launch<false, false>(sc.dev, grid, st, p)));
         KQ_COUNT_LAUNCH();
         KQ_LAUNCH_CHECK();
     }
@@ -1067,14 +1077,8 @@ int kq_gemm_error_fetch() {
 // stream by.  2048 and 4096 tokens x 8192 x 28672 in Q4_K, 125 and 250 MB at once: 1363 and 2788 us; in slabs of 62 MB 1200 and 2406.
 constexpr int64_t SLAB_MIN = MAX_CHUNKS * CHUNK;
 static int64_t slab_tokens(int64_t per_token) { return std::max(SLAB_MIN, SLAB_BYTES / per_token / SLAB_MIN * SLAB_MIN); }
-static int32_t padded_tokens(const KqGemvSeg *segs, int nseg, int64_t M, int64_t nb) {
-    int32_t pad = 0;
-    for (const uint32_t type : {(uint32_t)B200_TYPE_Q4_K, (uint32_t)B200_TYPE_Q6_K}) {
-        const TokTiles t = token_tiles_of(type, segs, nseg, M, nb);
-        pad = std::max(pad, t.n * t.tok);
-    }
-    return pad;
-}
+// the tokens that the images of a call hold, in whole tiles of either type
+static int32_t padded_tokens(const CallTiles &t) { return std::max(t.q4.n * t.q4.tok, t.q6.n * t.q6.tok); }
 
 b200_status kq_gemm_image(const KqGemvSeg *segs, int nseg, int64_t M, int64_t K, cudaStream_t st, KqTokenImage *im) {
     *im = KqTokenImage{};
@@ -1082,7 +1086,7 @@ b200_status kq_gemm_image(const KqGemvSeg *segs, int nseg, int64_t M, int64_t K,
     KQ_TRY(check_segs(segs, nseg, nullptr, K, &dev));
     const int64_t nb = K / 256;
     if (M > slab_tokens(token_bytes(segs, nseg, nb, false) + token_bytes(segs, nseg, nb, true))) return B200_OK; // in slabs
-    const int32_t pad = padded_tokens(segs, nseg, M, nb);
+    const int32_t pad = padded_tokens(call_tiles(segs, nseg, M, nb));
     Scratch sc;
     const b200_status rc = scratch_for(dev, segs, nseg, pad, nb, st, &sc);
     if (rc != B200_OK) return rc == B200_ERR_ALLOC ? B200_OK : rc;
@@ -1099,7 +1103,8 @@ b200_status kq_launch_gemm_image(const KqGemvSeg *segs, int nseg, const KqTokenI
     Scratch sc;
     KQ_TRY(scratch_for(dev, segs, nseg, im.m_pad, p.nb, st, &sc)); // the buffers that kq_gemm_image gave
     KQ_REQUIRE(sc.img16 == im.img16 && sc.img8 == im.img8 && sc.da == im.da, "gemm: another call came between a token image and its product");
-    return launch_segs(p, false, sc, segs, nseg, 1, K, st);
+    const CallTiles tiles = call_tiles(segs, nseg, p.M, p.nb);
+    return launch_segs(p, false, &tiles, sc, segs, nseg, 1, K, st);
 }
 
 b200_status kq_launch_gemm_tc(const KqGemvSeg *segs, int nseg, const int8_t *q, const float *d, const int16_t *bs, int64_t M, int64_t K,
@@ -1115,7 +1120,8 @@ b200_status kq_launch_gemm_tc(const KqGemvSeg *segs, int nseg, const int8_t *q, 
         if (mc < M - m0) mc = kq_div_up(mc, SLAB_MIN) * SLAB_MIN;
         Params p = {};
         p.M = (int32_t)mc, p.nb = (int32_t)nb;
-        p.m_pad = padded_tokens(segs, nseg, mc, nb);
+        const CallTiles tiles = call_tiles(segs, nseg, mc, nb);
+        p.m_pad = padded_tokens(tiles);
         Scratch sc;
         const b200_status rc = scratch_for(dev, segs, nseg, p.m_pad, nb, st, &sc);
         if (rc == B200_ERR_ALLOC && mc > SLAB_MIN) { // no room for these images: fewer at a time
@@ -1133,7 +1139,7 @@ b200_status kq_launch_gemm_tc(const KqGemvSeg *segs, int nseg, const int8_t *q, 
             sg[i].y += m0 * sg[i].n_rows;
         }
         p.residual = residual ? residual + m0 * segs[0].n_rows : nullptr;
-        KQ_TRY(launch_segs(p, false, sc, sg, nseg, 1, K, st));
+        KQ_TRY(launch_segs(p, false, &tiles, sc, sg, nseg, 1, K, st));
     }
     return B200_OK;
 }
@@ -1201,7 +1207,7 @@ b200_status kq_launch_gemm_grouped(const KqGemvSeg *segs, int nseg, const KqGrou
             KQ_CUDA(kq_launch(act_image_kernel, dim3((unsigned)(p.m_pad / 16), (unsigned)nb), dim3(288), 0, st, ip));
             KQ_COUNT_LAUNCH();
         }
-        KQ_TRY(launch_segs(p, narrow, sc, segs, nseg, E, K, st));
+        KQ_TRY(launch_segs(p, narrow, nullptr, sc, segs, nseg, E, K, st));
     }
     return B200_OK;
 }

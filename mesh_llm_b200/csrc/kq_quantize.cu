@@ -92,20 +92,19 @@ __global__ void __launch_bounds__(256) act_to_image_kernel(const float *x, const
             *reinterpret_cast<uint4 *>(im.img8 + group * KQ_TOK8 + i * 16) = *reinterpret_cast<const uint4 *>(s8 + (i >> 3) * PITCH + (i & 7) * 16);
 }
 
-// RMSNorm and Q8 of a row, W warps: a warp holds up to two of the row's blocks in registers, so that the row is read once, the weights before the
-// kernel waits for the one that writes the row.  Outputs: f32 (y), Q8 (q, d, bs), an image; rows past im.n_tok are zeros of the image.  The sum of squares is
+// RMSNorm and Q8 of a row, W warps: a warp holds up to R of the row's blocks in registers, so that the row is read once.  PRE, for few rows: the weights as well, asked for before the
+// kernel waits for the one that writes the row; many rows would rather have the registers (512 rows of 5120 8.9 us with, 7.0 without).  Outputs: f32 (y), Q8 (q, d, bs), an image; rows past im.n_tok are zeros of the image.  The sum of squares is
 // carried in double so that the scale does not depend on the order of the reduction: the normalised values, and with them the Q8 codes, are then
 // reproducible.
-template <int W>
+template <int W, int R, bool PRE>
 __global__ void __launch_bounds__(W * 32) rms_norm_q8_kernel(const float *x, const float *w, int h, float eps, float *y, int8_t *q, float *d, int16_t *bs,
                                                              int64_t x_row_stride, const __grid_constant__ KqTokenImage im) {
-    constexpr int R = 2;
     __shared__ double part[W];
     const int row = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nb = h / 256;
     const bool image = im.img16 || im.img8, live = !image || row < im.n_tok;
     const float *xr = x + (int64_t)row * x_row_stride;
     KQ_PDL_TRIGGER();
-    float g[R][8], v[R][8];
+    float g[PRE ? R : 1][8], v[R][8];
     auto load = [&](const float *p, int b, float (&o)[8]) {
         const float4 a = *reinterpret_cast<const float4 *>(p + b * 256 + lane * 8), c = *reinterpret_cast<const float4 *>(p + b * 256 + lane * 8 + 4);
         o[0] = a.x, o[1] = a.y, o[2] = a.z, o[3] = a.w, o[4] = c.x, o[5] = c.y, o[6] = c.z, o[7] = c.w;
@@ -115,8 +114,10 @@ __global__ void __launch_bounds__(W * 32) rms_norm_q8_kernel(const float *x, con
         for (int i = 0; i < 8; i++) o[i] = 1.0f;
         if (w && b < nb) load(w, b, o);
     };
+    if constexpr (PRE) {
 #pragma unroll
-    for (int r = 0; r < R; r++) weights(warp + r * W, g[r]);
+        for (int r = 0; r < R; r++) weights(warp + r * W, g[r]);
+    }
     KQ_PDL_WAIT();
     if (image && row == 0)
         for (int i = tid; i < im.n_parts; i += W * 32) im.parts[i] = make_int4(0, 0, 0, 0);
@@ -171,7 +172,10 @@ __global__ void __launch_bounds__(W * 32) rms_norm_q8_kernel(const float *x, con
     };
 #pragma unroll
     for (int r = 0; r < R; r++)
-        if (warp + r * W < nb) emit(warp + r * W, v[r], g[r]);
+        if (warp + r * W < nb) {
+            if constexpr (!PRE) weights(warp + r * W, g[0]);
+            emit(warp + r * W, v[r], g[PRE ? r : 0]);
+        }
     for (int b = warp + R * W; b < nb; b += W) {
         float u[8] = {}, f[8];
         if (live) load(xr, b, u);
@@ -420,11 +424,20 @@ b200_status kq_synth_weights(uint32_t type, void *W, int64_t n_rows, int64_t K, 
     return B200_OK;
 }
 
-// 8 warps for rows of up to 4096, 16 for longer ones
+// few rows: 8 warps for up to 4096 values, 16 for more, so that a row is one round of loads; many: 8
 static b200_status norm_q8(const float *x, const float *w, int64_t rows, int64_t h, float eps, float *y, int8_t *q, float *d, int16_t *bs, int64_t ldx,
                            const KqTokenImage &im, cudaStream_t st) {
-    if (h <= 4096) kq_launch(rms_norm_q8_kernel<8>, (unsigned)rows, 256, 0, st, x, w, (int)h, eps, y, q, d, bs, ldx, im);
-    else kq_launch(rms_norm_q8_kernel<16>, (unsigned)rows, 512, 0, st, x, w, (int)h, eps, y, q, d, bs, ldx, im);
+    auto go = [&](auto kernel, int warps) { kq_launch(kernel, (unsigned)rows, warps * 32, 0, st, x, w, (int)h, eps, y, q, d, bs, ldx, im); };
+    if (rows > 2 * kq_sm_count()) { // in registers up to 8192 values
+        if (h <= 2048) go(rms_norm_q8_kernel<8, 1, false>, 8);
+        else if (h <= 4096) go(rms_norm_q8_kernel<8, 2, false>, 8);
+        else if (h <= 6144) go(rms_norm_q8_kernel<8, 3, false>, 8);
+        else go(rms_norm_q8_kernel<8, 4, false>, 8);
+    } else {
+        if (h <= 2048) go(rms_norm_q8_kernel<8, 1, true>, 8);
+        else if (h <= 4096) go(rms_norm_q8_kernel<8, 2, true>, 8);
+        else go(rms_norm_q8_kernel<16, 2, true>, 16);
+    }
     KQ_COUNT_LAUNCH();
     KQ_LAUNCH_CHECK();
     return B200_OK;
