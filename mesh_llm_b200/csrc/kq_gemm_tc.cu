@@ -916,7 +916,13 @@ b200_status scratch(int dev, size_t img16_bytes, size_t img8_bytes, size_t da_by
         }
         if (need[i] && capturing) captured[dev][i] = true;
     }
-    if (!parts_done[dev]) KQ_CUDA(cudaGetSymbolAddress((void **)&parts_done[dev], g_parts_done));
+    if (!parts_done[dev]) {
+        cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed; // no work of a stream that is being captured either
+        KQ_CUDA(cudaThreadExchangeStreamCaptureMode(&mode));
+        const cudaError_t e = cudaGetSymbolAddress((void **)&parts_done[dev], g_parts_done);
+        cudaThreadExchangeStreamCaptureMode(&mode);
+        KQ_CUDA(e);
+    }
     *out = {img16_bytes ? (uint8_t *)buf[dev][0] : nullptr, img8_bytes ? (uint8_t *)buf[dev][1] : nullptr, (float *)buf[dev][2], (float *)buf[dev][3], parts_done[dev], dev};
     return B200_OK;
 }

@@ -11,6 +11,7 @@
 #include <stdlib.h>
 
 #include <algorithm>
+#include <atomic>
 
 b200_status kq_synth_weights(uint32_t type, void *W, int64_t n_rows, int64_t K, uint64_t key, float mean,
                              float sigma, cudaStream_t st);
@@ -185,7 +186,11 @@ __global__ void __launch_bounds__(256) moe_combine_kernel(const float *y, const 
         for (int s = 0; s < 8; s++)
             if (s0 + s < k) acc.x += f[s] * v[s].x, acc.y += f[s] * v[s].y, acc.z += f[s] * v[s].z, acc.w += f[s] * v[s].w;
     }
-    *reinterpret_cast<float4 *>(out + i) = make_float4(r.x + acc.x, r.y + acc.y, r.z + acc.z, r.w + acc.w);
+    if (((uintptr_t)out & 15) == 0) {
+        *reinterpret_cast<float4 *>(out + i) = make_float4(r.x + acc.x, r.y + acc.y, r.z + acc.z, r.w + acc.w);
+    } else { // a caller's rows
+        out[i] = r.x + acc.x, out[i + 1] = r.y + acc.y, out[i + 2] = r.z + acc.z, out[i + 3] = r.w + acc.w;
+    }
 }
 
 __global__ void gather_rows_kernel(const float *x, int64_t row_stride, int64_t first, int n_rows, int h,
@@ -419,13 +424,13 @@ b200_status forward_body(b200_stage *st, const int32_t *tokens, const float *hid
             if (!routed) {
             OTHER_(kq_rms_norm(st->x, L.ffn_norm, rows, h, c.rms_eps, st->xn, st->aq, st->ad, st->abs16, s));
             if (classes & CLS_OTHER) {
-            static bool rb_attr[16]; // the block kernel may have its shared memory, per device
+            static std::atomic<uint32_t> rb_ready; // devices on which the block kernel may have its shared memory
             int dev = 0;
             KQ_CUDA(cudaGetDevice(&dev));
             const int64_t blocks = kq_div_up(rows, RB) * kq_div_up(E, RB);
-            if (blocks >= RB_MIN_BLOCKS && dev < 16) {
-                if (!rb_attr[dev]) KQ_CUDA(cudaFuncSetAttribute(router_logits_block_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, RB_SMEM));
-                rb_attr[dev] = true;
+            if (blocks >= RB_MIN_BLOCKS && dev < 32) {
+                if (!(rb_ready.load() >> dev & 1)) KQ_CUDA(cudaFuncSetAttribute(router_logits_block_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, RB_SMEM));
+                rb_ready |= 1u << dev;
                 kq_launch(router_logits_block_kernel, (unsigned)blocks, 512, RB_SMEM, s, L.router, st->xn, rows, E, h, st->rl);
             } else if (const int64_t tiles = kq_div_up(rows, ROUTER_TILE) * kq_div_up(E, ROUTER_TILE); tiles >= ROUTER_MIN_TILES)
                 kq_launch(router_logits_tile_kernel, (unsigned)kq_div_up(tiles, 4), 128, 0, s,

@@ -428,7 +428,7 @@ def test_down_projection_input_quantised_by_the_gate_up_launch(cfg, n_seq, monke
 
 
 @pytest.mark.parametrize("cfg", [DENSE, LLAMA, MOE], ids=["qwen2-dense", "llama-dense", "qwen3-moe"])
-@pytest.mark.parametrize("T", [9, 16, 23, 255, 257])
+@pytest.mark.parametrize("T", [9, 16, 24, 25, 255, 257])
 def test_rows_written_as_token_images(cfg, T):
     """products of more than 8 rows read an image of their tokens that the norm (up to 256 rows), the quantiser or the SwiGLU writes: rows that fill groups of
     eight and tiles or do not, on both sides of 256, each layer's segments against the oracle from the same input"""
@@ -441,5 +441,21 @@ def test_rows_written_as_token_images(cfg, T):
     x = (np.random.default_rng(T).standard_normal((T, cfg["n_embd"])) * 0.02).astype(np.float32)
     for l in range(2):
         _, st = _load_range(cfg, full, l, l + 1, n_ubatch=288)
+        x, _, _, _ = check_layer("small", f"layer {l}, {T} rows", cfg, LayerOracle(full, cfg, l), st, x, 0)
+        st.close()
+
+
+@pytest.mark.parametrize("T", [4, 5, 8, 9])
+def test_long_rows_of_a_few_tokens(T):
+    """a feed-forward width that 5 to 8 tokens cannot stage at once: those take the tensor-core product, fewer the decode kernel, each segment against the oracle"""
+    from layer_oracle import LayerOracle
+    from test_gpu_real_widths import check_layer
+
+    cfg = dict(DENSE, n_ff=16384, n_layer=2, n_ctx=32)
+    full = orc.Model(**cfg)
+    full.generate(33)
+    x = (np.random.default_rng(T).standard_normal((T, cfg["n_embd"])) * 0.02).astype(np.float32)
+    for l in range(2):  # the down projection is Q4_K in one layer and Q6_K in the other
+        _, st = _load_range(cfg, full, l, l + 1, n_ubatch=16)
         x, _, _, _ = check_layer("small", f"layer {l}, {T} rows", cfg, LayerOracle(full, cfg, l), st, x, 0)
         st.close()
