@@ -185,12 +185,17 @@ __device__ __forceinline__ bool try_wait(uint32_t bar, uint32_t parity, int lane
                  : "memory");
     return __all_sync(0xffffffffu, ok) != 0;
 }
+// What its lanes have waited for is there for every lane behind it, and for whom one of them then arrives for: a vote brings lanes together, but only
+// __syncwarp orders their accesses to memory.
 __device__ __forceinline__ bool wait_on(uint32_t bar, uint32_t parity, int lane, int n, volatile int *give_up, int code) {
     uint64_t t0 = 0;
     while (true) {
 #pragma unroll 1
         for (int i = 0; i < 64; i++)
-            if (try_wait(bar, parity, lane, n)) return true;
+            if (try_wait(bar, parity, lane, n)) {
+                __syncwarp();
+                return true;
+            }
         const uint64_t now = kq_globaltimer_ns();
         if (!t0) t0 = now;
         const bool late = now - t0 > LIMIT;
@@ -200,7 +205,6 @@ __device__ __forceinline__ bool wait_on(uint32_t bar, uint32_t parity, int lane,
             return false;
         }
     }
-    return true;
 }
 
 template <bool Q6, bool NARROW>

@@ -30,6 +30,19 @@ def test_no_barrier_that_a_warp_can_miss_by_giving_up():
     assert drain.index("if (!ok) break;") < drain.index("atomicAdd")
 
 
+def test_a_wait_orders_memory_for_the_whole_warp():
+    """one lane asks for a barrier, all lanes read what it guards, and an elected lane hands it on by an arrival of its own: behind every wait that
+    succeeds the warp meets in a way that orders memory, which a vote does not"""
+    s = source()
+    wait = s[s.index("bool wait_on("):]
+    wait = wait[:wait.index("\n}")]
+    succeeds = list(re.finditer(r"return true;", wait))
+    assert succeeds and all(re.search(r"__syncwarp\(\);\s*$", wait[:m.start()]) for m in succeeds)
+    body = kernel_body()
+    assert "try_wait(" not in body  # every wait goes through wait_on
+    assert body.index("wait_on(bar, par") < body.index("bar_arrive(&acc_full[w])")
+
+
 def constants(q6):
     """the sizes of the rings of one instance"""
     s = source()
