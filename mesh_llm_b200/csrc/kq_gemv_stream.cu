@@ -994,6 +994,7 @@ __device__ __forceinline__ void stream_body(const StreamParams &p, uint8_t *smem
     } else if constexpr (M > 2) {
         // Several tokens: the warps are dealt out to the tokens and a thread has STAGE loads in flight, so that the codes of all tokens come in together.  Token by
         // token, each a round trip to L2 of its own, a launch took 3 us longer with 8 tokens (5120 x 5120 in Q4_K 12.5 -> 9.7 us, 2048 x 2048 9.2 -> 5.9)
+        static_assert(WARPS % M == 0, "a warp past the last token would write behind the tokens, into the ring");
         constexpr int WPT = WARPS / M, NT = WPT * 32, STAGE = 8;
         const int m = warp / WPT, i0 = warp % WPT * 32 + lane, n16 = nb * 16;
         uint8_t *tq = smem + m * act_tok;

@@ -107,3 +107,15 @@ def test_decoded_q4_weights_are_exact_in_f16():
             low, high = fma(h(1024 + q), h(sc), o0), fma(h(1024 + 16 * q), h(h(sc) * h(0.0625)), o1)
             assert float(low) == sc * q - float(k0) and float(high) == sc * q - float(k1)
             assert max(abs(float(low)), abs(float(high))) * 128 * 256 <= 2 ** 24
+
+
+def test_warps_of_the_decode_product_divide_among_the_tokens(tmp_path):
+    """its warps are dealt out to up to 8 tokens; a number that leaves some over, which a build may ask for, would have them write behind the last token: refused"""
+    import shutil
+    import subprocess
+
+    nvcc = shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"
+    src = os.path.join(os.path.dirname(SRC), "kq_gemv_stream.cu")
+    r = subprocess.run([nvcc, "-cuda", "-gencode", "arch=compute_100a,code=sm_100a", "-std=c++17", "--expt-relaxed-constexpr", "-DKQ_GEMV_WARPS=12", "-x", "cu", src,
+                        "-o", str(tmp_path / "x.ii")], capture_output=True, text=True)
+    assert r.returncode != 0 and "a warp past the last token" in r.stderr + r.stdout
