@@ -434,7 +434,8 @@ B200_API b200_status b200_stage_tensor_info(b200_stage *st, int64_t i, char *nam
 B200_API b200_status b200_stage_set_expert_mask(b200_stage *st, const uint8_t *mask, int32_t n_mask);
 /* Diagnostics: copies the first n_floats of one of the stage's activation buffers, as the last forward
  * call (of the stage's last layer) left it, to host memory.  which: "q", "k", "v" (projections; q and
- * k after RoPE when T > 1), "att" (attention output), "g" (SwiGLU output), "x" (residual stream).     */
+ * k after RoPE when T > 1), "att" (attention output), "g" (SwiGLU output), "hp" (the same of the
+ * chosen experts, token by token and slot by slot), "x" (residual stream).                          */
 B200_API b200_status b200_stage_peek(b200_stage *st, const char *which, float *host_out, size_t n_floats);
 B200_API b200_status b200_stage_synchronize(b200_stage *st);
 B200_API int64_t b200_stage_kernel_launches(b200_stage *st); /* launches issued so far        */

@@ -163,6 +163,17 @@ __global__ void __launch_bounds__(512) router_logits_block_kernel(const float *W
     }
 }
 
+// The experts of more than 8 rows: pairs gathered per expert, one grouped launch per matrix type.  Their gate and up products stay apart in hp and hp2, and the
+// SwiGLU goes into the down product's operand alone; otherwise hp holds the SwiGLU.  B200_MOE_GROUPED=0 keeps the second form for every batch size.
+bool experts_grouped(int rows, unsigned classes) {
+    static int on = -1;
+    if (on < 0) {
+        const char *v = getenv("B200_MOE_GROUPED");
+        on = !(v && v[0] == '0');
+    }
+    return on && rows > 8 && classes == CLS_ALL;
+}
+
 // out[t] = res[t] + sum_s w[t][s] * y[t*k+s]   (slot order, deterministic).  A thread has four columns and up to eight slots' loads in flight
 // (1024 tokens, 8 slots of 2048: a column and slot at a time 24 us, now 15); h a multiple of 4
 __global__ void __launch_bounds__(256) moe_combine_kernel(const float *y, const float *w, const float *res, int T, int k, int h,
@@ -451,14 +462,8 @@ b200_status forward_body(b200_stage *st, const int32_t *tokens, const float *hid
             };
             // Many tokens: the pairs are gathered per expert and each expert-packed matrix is one grouped
             // launch of the tensor-core GEMM (build_moe_ffn's MUL_MAT_ID); few tokens: one indirect GEMV
-            // row per pair.  B200_MOE_GROUPED=0 keeps the second form for every batch size.
-            static int grouped_on = -1;
-            if (grouped_on < 0) {
-                const char *v = getenv("B200_MOE_GROUPED");
-                grouped_on = !(v && v[0] == '0');
-            }
-            bool grouped = grouped_on && rows > 8 && classes == CLS_ALL;
-            if (grouped) {
+            // row per pair.
+            if (experts_grouped(rows, classes)) {
                 KQ_TRY(kq_moe_sort(st->rid, pairs, E, st->moe_sorted, st->moe_sorted_bytes, s));
                 const KqGemvSeg both[2] = {gu[0], {gu[1].W, gu[1].type, fe, st->hp2, nullptr, fe, kq_device_row_bytes(gu[1].type, h) * fe}};
                 KQ_TRY(kq_launch_gemm_grouped(both, 2, {st->aq, st->ad, st->abs16, nullptr, nullptr}, ku, pairs, E, h, st->moe_sorted, s));
@@ -945,6 +950,7 @@ b200_status b200_stage_forward(b200_stage *st, const int32_t *tokens, const floa
     KQ_TRY(resolve(st));
     if (st->layers_desc) KQ_TRY(kq_layers_check_pos(st, seq0, n_seq, T, pos0));
     cudaStream_t s = (cudaStream_t)stream;
+    st->gate_up_pairs = experts_grouped(n_seq * T, CLS_ALL) ? (int64_t)n_seq * T * c.n_expert_used : 0;
     const long long before = g_kq_launches;
     if (T == 1 && st->use_graph && !kq_layers_tracing(st)) {
         // decode step: positions come from device memory so one captured graph serves every step
@@ -1024,6 +1030,7 @@ b200_status b200_stage_profile_decode(b200_stage *st, int32_t n_seq, int32_t pos
     int32_t *tok = (int32_t *)st->rid_scratch;
     float *hin = st->xn, *hout = st->att;
     kq_layers_advance(st, 0, n_seq, -1); // the replays move the recurrent states
+    st->gate_up_pairs = experts_grouped(n_seq, classes) ? (int64_t)n_seq * c.n_expert_used : 0;
     cudaStream_t s = st->cap_stream;
     KQ_CUDA(cudaMemsetAsync(tok, 0, 256, s));
     kq_launch(set_pos_kernel, 1, 1, 0, s, st->pos0_dev, pos0);
@@ -1084,10 +1091,14 @@ b200_status b200_stage_peek(b200_stage *st, const char *which, float *host_out, 
     else if (w == "yp") { src = st->yp; cap = R * (size_t)c.n_expert_used * c.n_embd; }
     else if (w == "sorted") { src = (const float *)st->moe_sorted; cap = st->moe_sorted_bytes / 4; }
     else if (w == "rid") { src = (const float *)st->rid; cap = R * (size_t)c.n_expert_used; }
-    KQ_REQUIRE(src, "stage_peek: no buffer named %s (x, q, k, v, att, g)", which);
+    KQ_REQUIRE(src, "stage_peek: no buffer named %s (x, q, k, v, att, g, hp)", which);
     KQ_REQUIRE(n_floats <= cap, "stage_peek: %s holds %zu floats, asked for %zu", which, cap, n_floats);
     KqDevGuard dev_guard(c.device);
     KQ_CUDA(cudaDeviceSynchronize());
+    if (w == "hp" && st->gate_up_pairs) {
+        KQ_TRY(b200_swiglu(st->hp, st->hp2, st->gate_up_pairs * c.n_ff_exp, st->hp, nullptr));
+        st->gate_up_pairs = 0;
+    }
     KQ_CUDA(cudaMemcpy(host_out, src, n_floats * 4, cudaMemcpyDeviceToHost));
     return B200_OK;
 }

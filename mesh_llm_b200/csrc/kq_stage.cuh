@@ -63,6 +63,7 @@ struct b200_stage {
     float *x = nullptr, *xn = nullptr, *q = nullptr, *k = nullptr, *v = nullptr, *att = nullptr, *g = nullptr,
           *u = nullptr, *last = nullptr, *logits_int = nullptr, *att_scratch = nullptr, *rl = nullptr,
           *rw = nullptr, *hp = nullptr, *hp2 = nullptr, *yp = nullptr;
+    int64_t gate_up_pairs = 0; // pairs whose gate and up products the last call left in hp and hp2; 0: it left their SwiGLU in hp
     int32_t *moe_sorted = nullptr; // expert-major order of the routed pairs of a batch
     size_t moe_sorted_bytes = 0;
     uint8_t *expert_mask = nullptr; // one byte per expert, 1 = allowed (all ones when no mask is set)

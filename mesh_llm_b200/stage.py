@@ -152,7 +152,7 @@ class Stage:
         check(lib().b200_stage_set_expert_mask(self.h, m.ctypes.data, m.size))
 
     def peek(self, which, shape):
-        """diagnostics: an internal activation buffer ("q", "k", "v", "att", "g", "x") after the last forward"""
+        """diagnostics: an internal activation buffer ("q", "k", "v", "att", "g", "hp", "x") after the last forward"""
         out = np.empty(shape, np.float32)
         check(lib().b200_stage_peek(self.h, which.encode(), out.ctypes.data, out.size))
         return out

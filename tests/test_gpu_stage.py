@@ -459,3 +459,38 @@ def test_long_rows_of_a_few_tokens(T):
         _, st = _load_range(cfg, full, l, l + 1, n_ubatch=16)
         x, _, _, _ = check_layer("small", f"layer {l}, {T} rows", cfg, LayerOracle(full, cfg, l), st, x, 0)
         st.close()
+
+
+@pytest.mark.parametrize("T", [8, 9, 40, 290])
+def test_peek_at_the_experts_activations(T):
+    """"hp" is the SwiGLU of a token's chosen experts whatever form the batch takes (8 rows: one launch; more: gate and up products of their own, with narrow
+    and with wide tiles), asked for once or twice: against the same tokens eight at a time.  A Q8 code beside a tie that falls on its other side moves a
+    value by about 3e-3 of its block; the bare gate product is off by more than itself.  The second call shows that the first one left the stage as it was"""
+    import torch
+
+    from mesh_llm_b200.stage import Stage
+
+    cfg = dict(MOE, n_layer=1, n_ctx=320)
+    part = dict(layer_begin=0, layer_end=1, has_embd=0, has_output=0)
+    m = orc.Model(**cfg)
+    m.generate(41)
+    st = Stage(**cfg, **part, n_ubatch=300)
+    for n in orc.Model(**cfg, **part).tensor_names():
+        st.set_tensor(n, *m.tensor(n)[:2])
+    x = torch.from_numpy(np.random.default_rng(T).standard_normal((T, cfg["n_embd"])).astype(np.float32)).cuda()
+    ku, fe = cfg["n_expert_used"], cfg["n_ff_exp"]
+    want, ids = [], []
+    for i in range(0, T, 8):
+        n = min(8, T - i)
+        st.forward(hidden_in=x[i:i + n].contiguous(), n_seq=1, T=n, pos0=i)
+        want.append(st.peek("hp", (n * ku, fe)))
+        ids.append(st.peek("rid", (n * ku,)).view(np.int32))
+    want, ids = np.concatenate(want), np.concatenate(ids)
+    outs = []
+    for _ in range(2):
+        outs.append(st.forward(hidden_in=x, n_seq=1, T=T, pos0=0)[0].clone())
+        for _ in range(2):
+            got, same = st.peek("hp", (T * ku, fe)), st.peek("rid", (T * ku,)).view(np.int32) == ids  # two experts beside a tie may change places
+            assert same.mean() >= 0.9 and np.linalg.norm((got - want)[same]) <= 2e-2 * np.linalg.norm(want[same])
+    assert torch.equal(*outs)
+    st.close()
