@@ -341,7 +341,7 @@ b200_status kq_launch_gemv(const KqGemvSeg *segs, int nseg, const int8_t *q, con
 b200_status kq_launch_gemv_stream(const KqGemvSeg *segs, int nseg, const int8_t *q, const float *d,
                                   const int16_t *bs, int M, int64_t K, const float *residual, int swiglu_pairs,
                                   const KqActPrep *prep, cudaStream_t st, KqEmitQ8 *emit = nullptr);
-bool kq_gemv_batch_parts(uint32_t type, int64_t K); // 5 to 8 tokens of K values take launches over ranges of K
+bool kq_batch_takes_product(uint32_t type, int64_t N, int64_t K); // 5 to 8 tokens: the tensor-core product is the faster one
 b200_status kq_rms_norm(const float *x, const float *w, int64_t T, int64_t h, float eps, float *y, int8_t *q,
                         float *d, int16_t *bs, cudaStream_t st, int64_t x_row_stride);
 b200_status kq_rms_norm_heads(float *q, const float *wq, int64_t q_rows, float *k, const float *wk, int64_t k_rows, int64_t h, float eps, cudaStream_t st);

@@ -1533,9 +1533,12 @@ b200_status launch_parts(const KqGemvSeg *segs, int nseg, const int8_t *q, const
 }
 
 } // namespace
-// 5 to 8 tokens of K values take launches over ranges of K
-bool kq_gemv_batch_parts(uint32_t type, int64_t K) {
-    return type == B200_TYPE_Q4_K ? !batch_fits<B200_TYPE_Q4_K, 8>((int)(K / 256)) : !batch_fits<B200_TYPE_Q6_K, 8>((int)(K / 256));
+// Rows that 5 to 8 tokens cannot stage at once (from about 16 k values in Q4_K, 15 k in Q6_K) take launches over ranges of K here, each with its staging; the tensor-core
+// product takes such a matrix as tiles of 16 tokens.  8 tokens, this kernel / the product in us, for 1024, 5120, 8192 and 28672 rows: Q6_K of 16384 values 21 / 17,
+// 42 / 35, 52 / 47, 141 / 131, of 27648 35 / 21, 67 / 49, 87 / 70, 235 / 210: the product for any number of rows.  Q4_K of 16384 values 21 / 14, 28 / 25, 31 / 32, 72 / 83, of
+// 27648 32 / 17, 36 / 34, 46 / 48, 111 / 133: the product up to 5120 rows; with more of them its decoding takes longer than a second staging.  5 tokens alike.
+bool kq_batch_takes_product(uint32_t type, int64_t N, int64_t K) {
+    return type == B200_TYPE_Q4_K ? N <= 5120 && !batch_fits<B200_TYPE_Q4_K, 8>((int)(K / 256)) : !batch_fits<B200_TYPE_Q6_K, 8>((int)(K / 256));
 }
 namespace {
 

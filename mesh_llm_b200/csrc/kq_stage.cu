@@ -271,9 +271,8 @@ StTensor *lt(b200_stage *st, int l, const char *what) {
 // MUL_MAT on quantised activations already sitting in st->aq/ad/abs16
 b200_status mm(b200_stage *st, const StTensor *w, int rows, float *y, const float *bias,
                const float *residual, cudaStream_t s) {
-    // 5 to 8 rows too long for one launch of the decode kernel (27648 and 28672 values; it would stage a third of the row at a time) take the prompts' product, as a tile
-    // of 16 tokens: 5120 x 27648 with 8 tokens 66 -> 50 us in Q6_K, 36 -> 35 in Q4_K.  Without room for its token image: as before
-    if (rows > 4 && rows <= 8 && (w->type == B200_TYPE_Q4_K || w->type == B200_TYPE_Q6_K) && kq_gemv_batch_parts(w->type, w->ne[0])) {
+    // rows too long for one launch of the decode kernel may take the prompts' product; without room for its token image: the decode kernel all the same
+    if (rows > 4 && rows <= 8 && (w->type == B200_TYPE_Q4_K || w->type == B200_TYPE_Q6_K) && kq_batch_takes_product(w->type, w->ne[1], w->ne[0])) {
         const KqGemvSeg sg = {(const uint8_t *)w->dev, w->type, (int32_t)w->ne[1], y, bias, (int32_t)w->ne[1], 0};
         const b200_status rc = kq_launch_gemm(&sg, 1, st->aq, st->ad, st->abs16, rows, w->ne[0], residual, s);
         if (rc != B200_ERR_ALLOC) return rc;

@@ -494,3 +494,23 @@ def test_peek_at_the_experts_activations(T):
             assert same.mean() >= 0.9 and np.linalg.norm((got - want)[same]) <= 2e-2 * np.linalg.norm(want[same])
     assert torch.equal(*outs)
     st.close()
+
+
+def test_route_of_long_rows_by_the_number_of_rows():
+    """Q4_K rows that 8 tokens cannot stage at once: the product (image and product, two launches) for up to 5120 of them, the decode kernel (three ranges
+    of 32768 values) for more; the other launches of the two stages are the same"""
+    import torch
+
+    from mesh_llm_b200.stage import Stage
+
+    launches = []
+    for h in (5120, 5376):
+        cfg = dict(DENSE, n_layer=1, n_embd=h, n_ff=32768, n_ctx=32)
+        st = Stage(**cfg, layer_begin=0, layer_end=1, has_embd=0, has_output=0, n_ubatch=8)
+        st.generate(5)
+        before = st.kernel_launches()
+        out = st.forward(hidden_in=torch.randn((8, h), device="cuda"), n_seq=1, T=8, pos0=0)[0]
+        launches.append(st.kernel_launches() - before)
+        assert bool(torch.isfinite(out).all())
+        st.close()
+    assert launches[1] == launches[0] + 1
