@@ -110,9 +110,16 @@ __global__ void __launch_bounds__(128) router_logits_tile_kernel(const float *W,
 }
 
 // The same for large batches, sum for sum again: 16 warps share 32 tokens x 32 experts, whose rows come into shared memory 128 values at a time, in three
-// stages, so that L2 is read once per 32 rows instead of once per 8.  1024 tokens x 128 experts x 2048: 45 -> 27 us.  From 64 such blocks on; fewer leave SMs idle
-// that the tiles above would use.
-constexpr int RB = 32, RB_STAGES = 3, RB_SMEM = RB_STAGES * 2 * RB * 512, RB_MIN_BLOCKS = 64;
+// stages, so that L2 is read once per 32 rows instead of once per 8.  1024 tokens x 128 experts x 2048: 45 -> 27 us.
+constexpr int RB = 32, RB_STAGES = 3, RB_SMEM = RB_STAGES * 2 * RB * 512;
+// An SM holds one block or three CTAs of four tiles, and a wave of either takes about as long: the blocks where they are fewer waves.  They are so where both sides fill
+// them; a table just past a multiple of 32 experts, or a small one, is padding, and a few blocks leave SMs idle that the tiles use.  Blocks / tiles in us of a layer, width 2048:
+// 1024 x 128 248 / 262 (1 wave, 2), 2048 x 64 320 / 335, 2048 x 128 369 / 380, 4096 x 32 477 / 493, but 2048 x 8 279 / 275 (1, 1), 512 x 128 199 / 197 (1, 1), 2048 x 65 345 / 339 (2, 2),
+// 4096 x 33 496 / 486, 2048 x 160 400 / 394 (3, 3); width 4096 alike, 12 numbers of experts, 512 to 4096 tokens.
+bool router_takes_blocks(int64_t T, int64_t E) {
+    const int64_t sms = kq_sm_count(), blocks = kq_div_up(T, RB) * kq_div_up(E, RB), tiles = kq_div_up(T, ROUTER_TILE) * kq_div_up(E, ROUTER_TILE);
+    return kq_div_up(blocks, sms) < kq_div_up(kq_div_up(tiles, 4), 3 * sms);
+}
 __global__ void __launch_bounds__(512) router_logits_block_kernel(const float *W, const float *x, int T, int E, int h, float *out) {
     KQ_PDL_ENTER();
     extern __shared__ __align__(16) float4 rb[]; // [stage][experts, tokens][row][32]
@@ -437,11 +444,10 @@ b200_status forward_body(b200_stage *st, const int32_t *tokens, const float *hid
             static std::atomic<uint32_t> rb_ready; // devices on which the block kernel may have its shared memory
             int dev = 0;
             KQ_CUDA(cudaGetDevice(&dev));
-            const int64_t blocks = kq_div_up(rows, RB) * kq_div_up(E, RB);
-            if (blocks >= RB_MIN_BLOCKS && dev < 32) {
+            if (router_takes_blocks(rows, E) && dev < 32) {
                 if (!(rb_ready.load() >> dev & 1)) KQ_CUDA(cudaFuncSetAttribute(router_logits_block_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, RB_SMEM));
                 rb_ready |= 1u << dev;
-                kq_launch(router_logits_block_kernel, (unsigned)blocks, 512, RB_SMEM, s, L.router, st->xn, rows, E, h, st->rl);
+                kq_launch(router_logits_block_kernel, (unsigned)(kq_div_up(rows, RB) * kq_div_up(E, RB)), 512, RB_SMEM, s, L.router, st->xn, rows, E, h, st->rl);
             } else if (const int64_t tiles = kq_div_up(rows, ROUTER_TILE) * kq_div_up(E, ROUTER_TILE); tiles >= ROUTER_MIN_TILES)
                 kq_launch(router_logits_tile_kernel, (unsigned)kq_div_up(tiles, 4), 128, 0, s,
                           L.router, st->xn, rows, E, h, st->rl);

@@ -1,4 +1,5 @@
-"""The router of a micro-batch in its two forms: tiles of 8 tokens x 8 experts per warp from 256 tiles on, a warp per pair below."""
+"""The router of a micro-batch in its forms, sum for sum the same: blocks of 32 tokens x 32 experts where those are fewer waves than tiles, tiles of 8 x 8 per warp from 256 tiles
+on, a warp per pair below; and norm, logits and choice in one launch for few rows."""
 import numpy as np
 import pytest
 
@@ -33,15 +34,15 @@ def test_both_forms_route_alike(E, T):
     assert float((whole - parts).norm(dim=1).max() / change.norm(dim=1).mean()) <= 2e-2
 
 
-@pytest.mark.parametrize("E,T,h", [(256, 256, 256), (250, 260, 768), (33, 1025, 512)])
+@pytest.mark.parametrize("E,T,h", [(256, 256, 256), (250, 260, 768), (33, 1025, 512), (250, 520, 768), (62, 1801, 512), (256, 1025, 256)])
 def test_blocks_of_many_tokens(E, T, h):
-    """the router's block form (from 64 blocks of 32 tokens x 32 experts on), its last blocks part empty: the same
-    experts as the other forms take, and the same bound"""
+    """tiles (the first three) and the router's block form (one wave of blocks, full and with its last ones part empty, and two waves): the same
+    experts as a warp per pair or the one launch take, and the same bound"""
     import torch
 
     from mesh_llm_b200.stage import Stage
 
-    cfg = dict(n_layer=1, n_embd=h, n_head=4, n_head_kv=2, head_dim=64, n_ff=0, n_vocab=256, n_ctx=1280, n_expert=E, n_expert_used=2, n_ff_exp=256, qk_norm=1)
+    cfg = dict(n_layer=1, n_embd=h, n_head=4, n_head_kv=2, head_dim=64, n_ff=0, n_vocab=256, n_ctx=2048, n_expert=E, n_expert_used=2, n_ff_exp=256, qk_norm=1)
     part = dict(layer_begin=0, layer_end=1, has_embd=0, has_output=0)
     m = orc.Model(**cfg)
     m.generate(5)
@@ -50,7 +51,7 @@ def test_blocks_of_many_tokens(E, T, h):
         st.set_tensor(n, *m.tensor(n)[:2])
     x = torch.from_numpy(np.random.default_rng(T).standard_normal((T, h)).astype(np.float32)).cuda()
     whole = st.forward(hidden_in=x, n_seq=1, T=T, pos0=0)[0].double().clone()
-    step = 31  # at most 8 blocks: the other forms
+    step = 31  # at most 128 tiles: the other forms
     parts = torch.cat([st.forward(hidden_in=x[i:i + step].contiguous(), n_seq=1, T=min(step, T - i), pos0=i)[0].double().clone() for i in range(0, T, step)])
     st.close()
     change = whole - x.double()
