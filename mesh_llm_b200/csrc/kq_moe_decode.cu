@@ -4,8 +4,8 @@
 //   moe_router_fused_kernel   RMSNorm of the residual row, its Q8 form for the expert matmuls, the router's
 //                             f32 logits (ffn_gate_inp) and, in the last CTA of a token to finish, softmax +
 //                             masked top-k + renormalised weights: llama.cpp's build_moe_ffn up to
-//                             ggml_argsort_top_k (third_party/llama.cpp/patches/0003 lines 82-108); micro-batches of up
-//                             to 24 rows route with it as well
+//                             ggml_argsort_top_k (third_party/llama.cpp/patches/0003 lines 82-108); micro-batches of a
+//                             few more rows route with it as well (router_fused_rows)
 //   moe_down_combine_kernel   quantises the SwiGLU outputs of a token's (token, slot) pairs in its prologue,
 //                             multiplies each by the down matrix of its expert (MUL_MAT_ID) and leaves
 //                             x + sum_s w_s y_s directly: no [pairs x n_embd] intermediate, no combine launch

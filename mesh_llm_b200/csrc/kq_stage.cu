@@ -70,9 +70,11 @@ __global__ void __launch_bounds__(128) router_logits_kernel(const float *W, cons
 // more than one of them per SM: 128 tiles take 12 / 21 / 33 us where a warp per pair takes 10 / 16 / 25 (64 experts at 128 tokens, 8 at 1024), 256 tiles
 // take as long as 128 and the warps per pair 14 / 23 / 37.
 constexpr int ROUTER_TILE = 8, ROUTER_MIN_TILES = 256;
-// Norm, logits and choice in the decode step's one launch up to as many rows (its CTAs, 16 a row, norm the row for themselves): a prompt through four layers of 128
-// experts 653 -> 628 us with 9 rows, 749 -> 731 with 16, 857 -> 850 with 24; 893 and 894 with 32, 1047 and 1072 with 64.
-constexpr int ROUTER_FUSED_ROWS = 24;
+// Norm, logits and choice of more than 8 rows in the decode step's one launch up to as many.  Its CTAs, 16 a row, norm the row for themselves and read the whole table for it, a warp an expert
+// and turn: with more than 128 experts there is a second turn, and a narrow row's three launches are short.  A layer apart / in one launch, us, with 9, 16, 20 and 24 rows: 128 experts x 2048 107 / 99,
+// 121 / 116, 131 / 128, 135 / 132; 128 x 4096 144 / 134, 164 / 157, 181 / 177, 188 / 185; 32 x 1024 79 / 75, 80 / 80, 83 / 82, 83 / 84; 256 x 2048 115 / 109, 131 / 132, 145 / 148, 155 / 158;
+// 256 x 7168 229 / 216, 277 / 277, 312 / 319, 339 / 347; 16 x 512 65 / 67, 66 / 69, 72 / 72, 71 / 73.
+int router_fused_rows(int64_t E, int64_t h) { return h < 1024 ? 8 : E <= 128 ? 24 : 16; }
 __global__ void __launch_bounds__(128) router_logits_tile_kernel(const float *W, const float *x, int T, int E, int h, float *out) {
     KQ_PDL_ENTER();
     const int lane = threadIdx.x & 31, e_tiles = (E + ROUTER_TILE - 1) / ROUTER_TILE;
@@ -430,7 +432,7 @@ b200_status forward_body(b200_stage *st, const int32_t *tokens, const float *hid
                 moe_fused_on = !(v && v[0] == '0');
             }
             bool fused_small = moe_fused_on && rows <= 8 && classes == CLS_ALL && ku <= 8 && fe % 256 == 0 && h % 256 == 0;
-            bool routed = moe_fused_on && classes == CLS_ALL && h % 256 == 0 && rows <= (rows <= 8 ? (fused_small ? 8 : 0) : ROUTER_FUSED_ROWS);
+            bool routed = moe_fused_on && classes == CLS_ALL && h % 256 == 0 && rows <= (rows <= 8 ? (fused_small ? 8 : 0) : router_fused_rows(E, h));
             if (routed) {
                 const b200_status rs = kq_moe_router_fused(st->x, L.ffn_norm, c.rms_eps, L.router, (int)rows, (int)E, (int)h, (int)ku,
                                                            st->expert_mask, st->rl, st->rid, st->rw, st->aq, st->ad, st->abs16,

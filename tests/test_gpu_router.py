@@ -56,3 +56,32 @@ def test_blocks_of_many_tokens(E, T, h):
     st.close()
     change = whole - x.double()
     assert float((whole - parts).norm(dim=1).max() / change.norm(dim=1).mean()) <= 2e-2
+
+
+@pytest.mark.parametrize("E,h,few,many", [(128, 1024, 24, 25), (200, 1024, 16, 17), (16, 512, 8, 9)])
+def test_one_launch_routing_of_a_few_rows(E, h, few, many):
+    """on both sides of the number of rows up to which norm, logits and choice are one launch (three behind it): the same experts as six rows at a time take, and the same bound"""
+    import torch
+
+    from mesh_llm_b200.stage import Stage
+
+    cfg = dict(n_layer=1, n_embd=h, n_head=4, n_head_kv=2, head_dim=64, n_ff=0, n_vocab=256, n_ctx=64, n_expert=E, n_expert_used=4, n_ff_exp=256, qk_norm=1)
+    part = dict(layer_begin=0, layer_end=1, has_embd=0, has_output=0)
+    m = orc.Model(**cfg)
+    m.generate(7)
+    st = Stage(**cfg, **part, n_ubatch=32)
+    for n in orc.Model(**cfg, **part).tensor_names():
+        st.set_tensor(n, *m.tensor(n)[:2])
+    x = torch.from_numpy(np.random.default_rng(E).standard_normal((many, h)).astype(np.float32)).cuda()
+    launches = {}
+    for T in (few, many):
+        before = st.kernel_launches()
+        rows = x[:T].contiguous()
+        whole = st.forward(hidden_in=rows, n_seq=1, T=T, pos0=0)[0].double().clone()
+        launches[T] = st.kernel_launches() - before
+        parts = torch.cat([st.forward(hidden_in=rows[i:i + 6].contiguous(), n_seq=1, T=min(6, T - i), pos0=i)[0].double().clone() for i in range(0, T, 6)])
+        change = whole - rows.double()
+        assert float((whole - parts).norm(dim=1).max() / change.norm(dim=1).mean()) <= 2e-2
+    st.close()
+    if few > 8:
+        assert launches[many] == launches[few] + 2

@@ -22,8 +22,8 @@ def ask(tmp_path_factory):
     with open(os.path.join(CSRC, "kq_stage.cu")) as f:
         s = f.read()
     consts = "".join(re.search(r"^constexpr int " + n + r" = [^;]*;", s, re.M).group(0) + "\n" for n in ("ROUTER_TILE", "RB"))
-    rules = ["router_takes_blocks"]
-    code = PRELUDE + consts + "".join(re.search(r"^\w+ " + n + r"\(.*?^}\n", s, re.M | re.S).group(0) for n in rules)
+    rules = ["router_takes_blocks", "router_fused_rows"]
+    code = PRELUDE + consts + "".join(re.search(r"^\w+ " + n + r"\(.*?}\n(?=\S)", s, re.M | re.S).group(0) for n in rules)
     code += "int main(int, char **v) {\n" + "".join(f'    if (v[1][0] == \'{i}\') printf("%d", (int){n}(atoll(v[2]), atoll(v[3])));\n' for i, n in enumerate(rules)) + "}\n"
     d = tmp_path_factory.mktemp("routes")
     (d / "r.cpp").write_text(code)
@@ -36,3 +36,9 @@ def ask(tmp_path_factory):
 def test_router_logits_by_blocks(ask, T, E, blocks):
     """blocks of 32 tokens x 32 experts only where they were the faster form"""
     assert ask("router_takes_blocks", T, E) == blocks
+
+
+@pytest.mark.parametrize("E,h,rows", [(128, 2048, 24), (8, 2048, 24), (128, 4096, 24), (64, 4096, 24), (32, 1024, 24), (256, 2048, 16), (256, 7168, 16), (256, 8192, 16), (160, 6144, 16), (16, 512, 8)])
+def test_rows_of_the_one_launch_routing(ask, E, h, rows):
+    """as many rows as the one launch was the faster form for; 8 and fewer have a rule of their own"""
+    assert ask("router_fused_rows", E, h) == rows
