@@ -514,3 +514,51 @@ def test_route_of_long_rows_by_the_number_of_rows():
         assert bool(torch.isfinite(out).all())
         st.close()
     assert launches[1] == launches[0] + 1
+
+
+@pytest.mark.parametrize("ku", [4, 9])
+def test_experts_outputs_to_rows_at_any_address(ku):
+    """the combination of the experts' outputs, up to eight slots at a time and more: into rows of a caller that begin four bytes off a 16-byte boundary the same
+    bits as into aligned ones, and the rows that eight tokens at a time give (2e-2: see test_peek_at_the_experts_activations); what stands around them stays"""
+    import torch
+
+    from mesh_llm_b200.stage import Stage
+
+    T, h = 12, MOE["n_embd"]
+    cfg = dict(MOE, n_layer=1, n_expert_used=ku)
+    part = dict(layer_begin=0, layer_end=1, has_embd=0, has_output=0)
+    m = orc.Model(**cfg)
+    m.generate(43)
+    st = Stage(**cfg, **part, n_ubatch=16)
+    for n in orc.Model(**cfg, **part).tensor_names():
+        st.set_tensor(n, *m.tensor(n)[:2])
+    x = torch.from_numpy(np.random.default_rng(ku).standard_normal((T, h)).astype(np.float32)).cuda()
+    aligned = st.forward(hidden_in=x, n_seq=1, T=T, pos0=0)[0].clone()
+    room = torch.full((T * h + 8,), 7.0, device="cuda")
+    st.forward(hidden_in=x, n_seq=1, T=T, pos0=0, hidden_out=room[1:1 + T * h].view(T, h))
+    assert torch.equal(room[1:1 + T * h].view(T, h), aligned) and bool((room[:1] == 7).all()) and bool((room[1 + T * h:] == 7).all())
+    parts = torch.cat([st.forward(hidden_in=x[i:i + 6].contiguous(), n_seq=1, T=6, pos0=i)[0].clone() for i in range(0, T, 6)])
+    assert float((aligned - parts).norm(dim=1).max() / (aligned - x).norm(dim=1).mean()) <= 2e-2
+    st.close()
+
+
+def test_experts_activations_in_slabs():
+    """the down product's operand of more than 256 MB, which the SwiGLU writes: in two launches, the second beginning at a tile of its own.  Every token takes all
+    eight experts, so none can change places; against the same tokens eight at a time, within 2e-2 (see test_peek_at_the_experts_activations)"""
+    import torch
+
+    from mesh_llm_b200 import capi
+    from mesh_llm_b200.stage import Stage
+
+    T, E, h, fe = 512, 8, 256, 97 * 256
+    tiles = T * E // 128 + E  # of 128 pairs, one part empty per expert
+    assert tiles * 128 * (fe // 256) * 544 > 256 << 20
+    st = Stage(n_layer=1, n_embd=h, n_head=4, n_head_kv=2, head_dim=64, n_ff=0, n_vocab=256, n_ctx=T, n_expert=E, n_expert_used=E, n_ff_exp=fe, qk_norm=1,
+               layer_begin=0, layer_end=1, has_embd=0, has_output=0, n_ubatch=T)
+    st.generate(9)
+    x = torch.randn((T, h), generator=torch.Generator(device="cuda").manual_seed(3), device="cuda")
+    whole = st.forward(hidden_in=x, n_seq=1, T=T, pos0=0)[0].clone()
+    parts = torch.cat([st.forward(hidden_in=x[i:i + 8].contiguous(), n_seq=1, T=8, pos0=i)[0].clone() for i in range(0, T, 8)])
+    assert capi.lib().b200_check_device_waits() == 0
+    assert float((whole - parts).norm(dim=1).max() / (whole - x).norm(dim=1).mean()) <= 2e-2
+    st.close()
