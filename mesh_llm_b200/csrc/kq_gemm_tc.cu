@@ -431,53 +431,53 @@ __global__ void __launch_bounds__(NTHREADS, 1) gemm_kq_kernel(const __grid_const
                 }
                 const int s = k % C::RAW_STAGES;
                 if (!NARROW || sa == turn) {
-                if (u >= 2 && !wait(&a_empty[sa], ((u >> 1) - 1) & 1, 7)) break;
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const uint8_t *blk = smem + C::SM_RAW + s * C::RAW_BYTES + row * 32 + (b & 1) * 16; // chunk i of the block 4096 i further
-                const uint4 sc4 = *reinterpret_cast<const uint4 *>(blk + 12 * 4096);
-                const int b8 = b % KQ_Q6_GROUP;
-                const uint32_t dw = b8 < 2 ? dv.x : b8 < 4 ? dv.y : b8 < 6 ? dv.z : dv.w;
-                *reinterpret_cast<uint32_t *>(smem + C::SM_SC + ((u % SC_RING) * ROWS + row) * 4) = (b8 & 1 ? dw >> 16 : dw) & 0xFFFFu;
+                    if (u >= 2 && !wait(&a_empty[sa], ((u >> 1) - 1) & 1, 7)) break;
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                    const uint8_t *blk = smem + C::SM_RAW + s * C::RAW_BYTES + row * 32 + (b & 1) * 16; // chunk i of the block 4096 i further
+                    const uint4 sc4 = *reinterpret_cast<const uint4 *>(blk + 12 * 4096);
+                    const int b8 = b % KQ_Q6_GROUP;
+                    const uint32_t dw = b8 < 2 ? dv.x : b8 < 4 ? dv.y : b8 < 6 ? dv.z : dv.w;
+                    *reinterpret_cast<uint32_t *>(smem + C::SM_SC + ((u % SC_RING) * ROWS + row) * 4) = (b8 & 1 ? dw >> 16 : dw) & 0xFFFFu;
 #pragma unroll (NARROW ? 2 : 1)
-                for (int hh = 0; hh < 2; hh++) { // 128 elements
-                    const uint32_t sc_a = hh ? sc4.z : sc4.x, sc_b = hh ? sc4.w : sc4.y;
-                    uint32_t wide_hi[NARROW ? 32 : 4], wide_lo[NARROW ? 32 : 4]; // NARROW: 128 elements at a time, for more independent work
+                    for (int hh = 0; hh < 2; hh++) { // 128 elements
+                        const uint32_t sc_a = hh ? sc4.z : sc4.x, sc_b = hh ? sc4.w : sc4.y;
+                        uint32_t wide_hi[NARROW ? 32 : 4], wide_lo[NARROW ? 32 : 4]; // NARROW: 128 elements at a time, for more independent work
 #pragma unroll (NARROW ? 2 : 1)
-                    for (int h = 0; h < 2; h++) { // elements 128 hh + 32 q + 16 h + ..
-                        const uint4 a4 = *reinterpret_cast<const uint4 *>(blk + (4 * hh + h) * 4096), c4 = *reinterpret_cast<const uint4 *>(blk + (4 * hh + 2 + h) * 4096),
-                                    q4 = *reinterpret_cast<const uint4 *>(blk + (8 + 2 * hh + h) * 4096);
-                        const uint32_t a[4] = {a4.x, a4.y, a4.z, a4.w}, c[4] = {c4.x, c4.y, c4.z, c4.w}, qh[4] = {q4.x, q4.y, q4.z, q4.w};
+                        for (int h = 0; h < 2; h++) { // elements 128 hh + 32 q + 16 h + ..
+                            const uint4 a4 = *reinterpret_cast<const uint4 *>(blk + (4 * hh + h) * 4096), c4 = *reinterpret_cast<const uint4 *>(blk + (4 * hh + 2 + h) * 4096),
+                                        q4 = *reinterpret_cast<const uint4 *>(blk + (8 + 2 * hh + h) * 4096);
+                            const uint32_t a[4] = {a4.x, a4.y, a4.z, a4.w}, c[4] = {c4.x, c4.y, c4.z, c4.w}, qh[4] = {q4.x, q4.y, q4.z, q4.w};
 #pragma unroll
-                        for (int q = 0; q < 4; q++) { // 16 elements: scale group 8 hh + 2 q + h
-                            // Two codes to a register, 16 bits each: 4 (sc (q - 32) + 8192) is between 16384 and 49152, so neither half reaches into the
-                            // other.  Its upper byte is hi + 128, its lower one 4 lo.
-                            const int sc = (int)((q < 2 ? sc_a : sc_b) << (24 - 8 * ((2 * q) & 3) - 8 * h)) >> 24;
-                            const uint32_t k4 = 4u * (uint32_t)sc, base = 0x80008000u - 0x00800080u * (uint32_t)sc;
-                            uint32_t *hi = wide_hi + (NARROW ? 8 * q + 4 * h : 0), *lo = wide_lo + (NARROW ? 8 * q + 4 * h : 0);
+                            for (int q = 0; q < 4; q++) { // 16 elements: scale group 8 hh + 2 q + h
+                                // Two codes to a register, 16 bits each: 4 (sc (q - 32) + 8192) is between 16384 and 49152, so neither half reaches into the
+                                // other.  Its upper byte is hi + 128, its lower one 4 lo.
+                                const int sc = (int)((q < 2 ? sc_a : sc_b) << (24 - 8 * ((2 * q) & 3) - 8 * h)) >> 24;
+                                const uint32_t k4 = 4u * (uint32_t)sc, base = 0x80008000u - 0x00800080u * (uint32_t)sc;
+                                uint32_t *hi = wide_hi + (NARROW ? 8 * q + 4 * h : 0), *lo = wide_lo + (NARROW ? 8 * q + 4 * h : 0);
 #pragma unroll
-                            for (int i = 0; i < 4; i++) {
-                                const uint32_t n = q & 1 ? c[i] : a[i], top = q == 0 ? qh[i] << 4 : q == 1 ? qh[i] << 2 : q == 2 ? qh[i] : qh[i] >> 2;
-                                const uint32_t code = ((q & 2 ? n >> 4 : n) & 0x0F0F0F0Fu) | (top & 0x30303030u);
-                                const uint32_t even = (code & 0x00FF00FFu) * k4 + base, odd = ((code >> 8) & 0x00FF00FFu) * k4 + base;
-                                hi[i] = __byte_perm(even, odd, 0x7351) ^ 0x80808080u;
-                                lo[i] = __byte_perm(even, odd, 0x6240);
-                            }
-                            const uint32_t at = tl + sa * 128 + 32 * hh + 8 * q + 4 * h;
-                            if (!NARROW) {
-                                TMEM_ST4(at, hi);
-                                TMEM_ST4(at + 64, lo);
+                                for (int i = 0; i < 4; i++) {
+                                    const uint32_t n = q & 1 ? c[i] : a[i], top = q == 0 ? qh[i] << 4 : q == 1 ? qh[i] << 2 : q == 2 ? qh[i] : qh[i] >> 2;
+                                    const uint32_t code = ((q & 2 ? n >> 4 : n) & 0x0F0F0F0Fu) | (top & 0x30303030u);
+                                    const uint32_t even = (code & 0x00FF00FFu) * k4 + base, odd = ((code >> 8) & 0x00FF00FFu) * k4 + base;
+                                    hi[i] = __byte_perm(even, odd, 0x7351) ^ 0x80808080u;
+                                    lo[i] = __byte_perm(even, odd, 0x6240);
+                                }
+                                const uint32_t at = tl + sa * 128 + 32 * hh + 8 * q + 4 * h;
+                                if (!NARROW) {
+                                    TMEM_ST4(at, hi);
+                                    TMEM_ST4(at + 64, lo);
+                                }
                             }
                         }
+                        if constexpr (NARROW) {
+                            TMEM_ST32(tl + sa * 128 + 32 * hh, wide_hi);
+                            TMEM_ST32(tl + sa * 128 + 32 * hh + 64, wide_lo);
+                        }
                     }
-                    if constexpr (NARROW) {
-                        TMEM_ST32(tl + sa * 128 + 32 * hh, wide_hi);
-                        TMEM_ST32(tl + sa * 128 + 32 * hh + 64, wide_lo);
-                    }
-                }
-                asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-                asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-                __syncwarp();
-                if (lane == 0) bar_arrive(&a_full[sa]);
+                    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+                    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                    __syncwarp();
+                    if (lane == 0) bar_arrive(&a_full[sa]);
                 }
                 if (lane == 0 && (b % 2 == 1 || b == nb - 1)) bar_arrive(&raw_empty[s]);
                 if (++b == nb) b = 0, tile++;
@@ -1156,10 +1156,12 @@ b200_status kq_launch_gemm_tc(const KqGemvSeg *segs, int nseg, const int8_t *q, 
 
 // ---- MUL_MAT_ID over many tokens: pairs gathered per expert, one grouped launch of the tensor-core kernel ----
 // Scratch of the sort, in int32 words: [0] number of live tiles, [1 .. 1 + max_tiles) expert per tile,
-// [1 + max_tiles ..) pair per tile row, then pairs per tile; max_tiles = ceil(n_pairs / 128) + n_expert bounds sum_e ceil(c_e / 128).
-// Pairs of a tile: with few pairs an expert narrow tiles (128 experts, one pair each: a layer's step of 16 users 754 us in four layers, as tiles of two chunks 930); from about
-// as many as fill one, wide ones, where most experts are one tile (64 pairs each: two layers 1246 us, 1308 as narrow tiles).  Narrow tiles need no more
-// room for the sort than wide ones: at most 48 E / 64 + E tiles of 64 rows against E of 128.
+// [1 + max_tiles ..) pair per tile row, then pairs per tile; with t = moe_tile(n_pairs, n_expert) pairs a tile, max_tiles = ceil(n_pairs / t) + n_expert bounds sum_e ceil(c_e / t).
+// So the places in it depend on both numbers: sort and products are given the same.
+// Pairs of a tile: with few pairs an expert narrow tiles, whose blocks two warpgroups decode; from about as many as fill one, wide ones, where most experts are one
+// tile.  Narrow / wide, us, with 8, 48, 64 and 96 pairs an expert: 128 experts 768 x 2048 in Q4_K 63 / 87, 113 / 133, 151 / 148, 208 / 183; 2048 x 768 in Q6_K 87 / 103, 143 / 161, 202 / 170, 272 / 197;
+// 8 experts 14336 x 4096 in Q4_K 94 / 135, 128 / 165, 179 / 170, 231 / 178; 256 experts 2048 x 2048 in Q6_K 301 / 429, 463 / 576, 659 / 617, 874 / 689; fourteen such tables alike.  Narrow tiles
+// need no more room for the sort than wide ones: at most 48 E / 64 + E tiles of 64 rows against E of 128.
 static inline int moe_tile(int64_t n_pairs, int64_t E) { return n_pairs <= 48 * E ? CHUNK : 2 * CHUNK; }
 static inline int64_t moe_max_tiles(int64_t n_pairs, int64_t E) { return kq_div_up(n_pairs, moe_tile(n_pairs, E)) + E; }
 
