@@ -13,7 +13,7 @@
 // A tile is 128 weight rows x up to 256 tokens.  Weight rows are the M of the MMA (TMEM lanes), tokens its N in chunks of
 // up to 64.  Packed blocks arrive by TMA; a warpgroup (a thread per row) decodes them into TMEM, two bytes per weight in both types, from where
 // the MMAs take them as their A operand, so that decoded weights never pass through shared memory.  The token operand is an image that
-// act_image_kernel writes (f16 codes and sums of 16 for Q4_K, the codes themselves for Q6_K): one bulk copy per chunk and block.  Two warps issue MMAs in turn, each with an accumulator of its own;
+// act_image_kernel, or the kernel that makes the tokens, writes (f16 codes and sums of 16 for Q4_K, the codes themselves for Q6_K): one bulk copy per chunk and block.  Two warps issue MMAs in turn, each with an accumulator of its own;
 // the draining warps add the accumulators to the running f32 result, which stays in registers for the whole tile.  Lanes of a
 // warp hold neighbouring rows of W, so results leave in full lines.
 // With tiles of two or four chunks one warpgroup decodes and two drain, half of every chunk each.  Narrow tiles are one chunk: their blocks take the decoding longer
